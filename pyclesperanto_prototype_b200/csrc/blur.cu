@@ -6,9 +6,19 @@
 // float32 intermediates; a pass with sigma <= 0 is a copy.  Inside a pass
 // the output is acc = fma(w_i, v_i, acc) for i = -r..r ascending from 0.
 //
-// Layout: the row pass stages a run of one x-row (+halo) in shared memory;
-// the column passes (y and z) stage a (rows + 2r) x 32-column tile, so every
-// global access is a coalesced 128-byte segment.
+// Each thread makes 8 consecutive outputs along the pass axis of two lines at
+// once (two rows in the x pass, two adjacent columns in the y and z passes), the
+// two lines packed (fma.rn.f32x2: two independent round-to-nearest FMAs, the
+// rounding of fmaf).  Lines are staged in shared memory as float32; a block of
+// 8 taps takes the 8 values of the window already held and the next 8, so 64
+// packed FMAs share 8 packed loads.  Taps lie in shared memory as pairs
+// (w, w).  Nothing is padded with zero taps: 0 x infinity would be NaN.
+// What bounds it: the FMA pipe (sigma 10, 64 x 1024 x 1024: 81 taps x 3 are 0.44 ms
+// at 128 FMAs per SM and cycle, three reads and writes 0.25 ms); measured
+// 0.85 ms (2.02 with one output per thread and a shared load per FMA), the pipe
+// 60% busy, the rest in staging and at the one barrier of each CTA.  Staging
+// with all of a thread's loads in flight at once (asynchronous 16-byte copies
+// in the y and z passes, batches of 128-bit loads in x) took it from 1.07 ms.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -16,65 +26,269 @@ namespace cle {
 
 namespace {
 
-constexpr int kRowTile = 1024;   // outputs per CTA along x
-constexpr int kRowThreads = 256;
-constexpr int kColW = 32;        // columns per CTA in the column pass
-constexpr int kColRows = 64;     // outputs per CTA along the pass axis
-constexpr int kColThreadsY = 8;
+constexpr int kK = 8;             // outputs per thread along the pass axis, taps per block
+constexpr int kSepThreads = 256;
+constexpr int kRowMax = 256;      // x pass: most outputs of a row per CTA
+constexpr int kBlk = kK + 2;      // x pass: pitch of 8 staged pairs (16-byte lanes on odd granules)
 
+// acc[k] += w * win[k + t] for the 8 outputs; win = lo (8 values) then hi
+__device__ __forceinline__ void add_tap(float2 w, int t, const float2 (&lo)[kK], const float2 (&hi)[kK],
+                                        float2 (&acc)[kK]) {
+#pragma unroll
+    for (int k = 0; k < kK; ++k) acc[k] = __ffma2_rn(w, k + t < kK ? lo[(k + t) % kK] : hi[(k + t) % kK], acc[k]);
+}
+
+// The taps' chain over a staged line: block(j) loads the window's 8 packed
+// values 8j .. 8j + 7 of the thread (values past the last tap's are loaded but
+// not used).
+template <typename Block>
+__device__ __forceinline__ void tap_chain(const float2 *sw, int n, float2 (&acc)[kK], Block block) {
+    float2 a[kK], b[kK];
+    block(0, a);
+    int i = 0;
+    // two blocks of taps per round, the window's halves changing places
+    for (; i + 2 * kK <= n; i += 2 * kK) {
+        block(i / kK + 1, b);
+#pragma unroll
+        for (int t = 0; t < kK; ++t) add_tap(sw[i + t], t, a, b, acc);
+        block(i / kK + 2, a);
+#pragma unroll
+        for (int t = 0; t < kK; ++t) add_tap(sw[i + kK + t], t, b, a, acc);
+    }
+    if (i + kK <= n) {
+        block(i / kK + 1, b);
+#pragma unroll
+        for (int t = 0; t < kK; ++t) add_tap(sw[i + t], t, a, b, acc);
+        i += kK;
+#pragma unroll
+        for (int t = 0; t < kK; ++t) a[t] = b[t];
+    }
+    if (i < n) {
+        block(i / kK + 1, b);
+#pragma unroll
+        for (int t = 0; t < kK - 1; ++t)
+            if (i + t < n) add_tap(sw[i + t], t, a, b, acc);
+    }
+}
+
+__host__ __device__ constexpr int tap_slots(int n) { return (n + 1) & ~1; }   // float2 slots of the taps, 16-byte multiple
+// 8-value blocks of a line that tap_chain may load for `out` outputs
+__host__ __device__ constexpr int line_blocks(int out, int n) { return out / kK + n / kK + 1; }
+
+// four consecutive aligned source values as float32
+__device__ __forceinline__ void load4(const float *p, float (&v)[4]) {
+    const float4 f = __ldg(reinterpret_cast<const float4 *>(p));
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+}
+__device__ __forceinline__ void load4(const uint16_t *p, float (&v)[4]) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
+    v[0] = (float)(u.x & 0xFFFFu); v[1] = (float)(u.x >> 16);
+    v[2] = (float)(u.y & 0xFFFFu); v[3] = (float)(u.y >> 16);
+}
+__device__ __forceinline__ void load4(const uint8_t *p, float (&v)[4]) {
+    const uint32_t u = __ldg(reinterpret_cast<const uint32_t *>(p));
+    v[0] = (float)(u & 0xFFu); v[1] = (float)((u >> 8) & 0xFFu);
+    v[2] = (float)((u >> 16) & 0xFFu); v[3] = (float)(u >> 24);
+}
+
+__device__ __forceinline__ void copy_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// x pass: a CTA takes np row pairs and an x tile of `tile` outputs (a
+// multiple of 8) of each.
 template <typename Tin>
-__global__ void __launch_bounds__(kRowThreads)
-blur_row_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t rows, int W,
-                const __grid_constant__ Taps taps) {
-    extern __shared__ float s[];
-    const int r = (taps.n - 1) / 2;
-    const int64_t row = blockIdx.y + (int64_t)blockIdx.z * gridDim.y;
-    if (row >= rows) return;
-    const int x0 = blockIdx.x * kRowTile;
-    const Tin *in = src + row * (int64_t)W;
-    const int span = kRowTile + 2 * r;
-    for (int i = threadIdx.x; i < span; i += kRowThreads) {
-        int x = clampi(x0 - r + i, 0, W - 1);
-        s[i] = to_f32(in[x]);
+__global__ void __launch_bounds__(kSepThreads)
+blur_row_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t rows, int W, int tile, int np,
+                FastDiv fc, int vec, const __grid_constant__ Taps taps) {
+    extern __shared__ __align__(16) float2 sm[];
+    const int n = taps.n, r = (n - 1) / 2;
+    float2 *sw = sm, *line = sm + tap_slots(n);
+    const int pitch = kBlk * line_blocks(tile, n);
+    const int x0 = blockIdx.x * tile;
+    const int64_t row0 = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * (2 * np);
+    if (row0 >= rows) return;
+    for (int i = threadIdx.x; i < n; i += kSepThreads) sw[i] = make_float2(taps.w[i], taps.w[i]);
+    // staging, a warp per row pair: column c of the line is x = x0 - r + c
+    const int span = tile + 2 * r, lane = threadIdx.x & 31;
+    auto put = [&](float2 *ln, int c, float2 v) { ln[c + 2 * (c / kK)] = v; };
+    for (int q = threadIdx.x >> 5; q < np; q += kSepThreads / 32) {
+        const Tin *ra = src + min(row0 + 2 * q, rows - 1) * W, *rb = src + min(row0 + 2 * q + 1, rows - 1) * W;
+        float2 *ln = line + q * pitch;
+        if (vec) {
+            // 4 columns per lane from aligned groups (W and x0 are multiples of 4)
+            const int xa = x0 - ((r + 3) & ~3), d = x0 - r - xa;
+            for (int c0 = 4 * lane; c0 < span + d; c0 += 3 * 128) {
+                float va[3][4], vb[3][4];
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    const int c = c0 + 128 * u, x = xa + c;
+                    if (c < span + d) {
+                        if (x >= 0 && x + 4 <= W) {
+                            load4(ra + x, va[u]);
+                            load4(rb + x, vb[u]);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                va[u][k] = to_f32(ra[clampi(x + k, 0, W - 1)]);
+                                vb[u][k] = to_f32(rb[clampi(x + k, 0, W - 1)]);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int c = c0 + 128 * u + k - d;
+                        if (c >= 0 && c < span) put(ln, c, make_float2(va[u][k], vb[u][k]));
+                    }
+            }
+        } else {
+#pragma unroll 4
+            for (int c = lane; c < span; c += 32) {
+                const int x = clampi(x0 - r + c, 0, W - 1);
+                put(ln, c, make_float2(to_f32(ra[x]), to_f32(rb[x])));
+            }
+        }
     }
     __syncthreads();
-    float *out = dst + row * (int64_t)W;
-#pragma unroll 4
-    for (int k = 0; k < kRowTile / kRowThreads; ++k) {
-        int xo = threadIdx.x + k * kRowThreads;
-        if (x0 + xo >= W) break;
-        float acc = 0.0f;
-        for (int i = 0; i < taps.n; ++i) acc = __fmaf_rn(taps.w[i], s[xo + i], acc);
-        out[x0 + xo] = acc;
+    const int per = tile / kK;   // items per row pair
+    for (int e = threadIdx.x; e < np * per; e += kSepThreads) {
+        const int q = (int)fc.div((uint32_t)e), c = e - q * per;
+        const int64_t ra = row0 + 2 * q;
+        const int x = x0 + c * kK;
+        if (ra >= rows || x >= W) continue;
+        const float2 *base = line + q * pitch + c * kBlk;
+        float2 acc[kK];
+#pragma unroll
+        for (int k = 0; k < kK; ++k) acc[k] = make_float2(0.f, 0.f);
+        tap_chain(sw, n, acc, [&](int j, float2 (&v)[kK]) {
+            const float4 *p = reinterpret_cast<const float4 *>(base + j * kBlk);
+#pragma unroll
+            for (int k = 0; k < kK / 2; ++k) {
+                const float4 f = p[k];
+                v[2 * k] = make_float2(f.x, f.y);
+                v[2 * k + 1] = make_float2(f.z, f.w);
+            }
+        });
+        float *o = dst + ra * W + x;
+        const bool two = ra + 1 < rows;
+        if ((W & 3) == 0 && x + kK <= W && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+            for (int k = 0; k < kK; k += 4) {
+                *reinterpret_cast<float4 *>(o + k) = make_float4(acc[k].x, acc[k + 1].x, acc[k + 2].x, acc[k + 3].x);
+                if (two) *reinterpret_cast<float4 *>(o + W + k) = make_float4(acc[k].y, acc[k + 1].y, acc[k + 2].y, acc[k + 3].y);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kK; ++k)
+                if (x + k < W) {
+                    o[k] = acc[k].x;
+                    if (two) o[W + k] = acc[k].y;
+                }
+        }
     }
 }
 
 // Pass along an axis of length L with element stride `inner`, for a volume
-// viewed as [outer][L][inner].
-template <typename Tin>
-__global__ void __launch_bounds__(kColW *kColThreadsY)
-blur_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t inner, int L,
-                int64_t outer, const __grid_constant__ Taps taps) {
-    extern __shared__ float s[];
-    const int r = (taps.n - 1) / 2;
-    const int64_t c = (int64_t)blockIdx.x * kColW + threadIdx.x;
-    const int l0 = blockIdx.y * kColRows;
-    const int64_t o = blockIdx.z;
-    if (o >= outer) return;
-    const int span = kColRows + 2 * r;
-    const int64_t base = o * (int64_t)L * inner;
-    for (int j = threadIdx.y; j < span; j += kColThreadsY) {
-        int l = clampi(l0 - r + j, 0, L - 1);
-        s[j * kColW + threadIdx.x] = (c < inner) ? to_f32(src[base + (int64_t)l * inner + c]) : 0.0f;
+// viewed as [outer][L][inner]: a CTA takes NG x 8 outputs along the axis and
+// 2 x NC columns (NG x NC = 256 threads).
+template <typename Tin, int NG>
+__global__ void __launch_bounds__(kSepThreads)
+blur_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t inner, int L, int vec,
+                const __grid_constant__ Taps taps, float *__restrict__ mm) {
+    constexpr int NC = kSepThreads / NG, COLS = 2 * NC, ROWS = NG * kK;
+    extern __shared__ __align__(16) float2 sm[];
+    const int n = taps.n, r = (n - 1) / 2;
+    float2 *sw = sm;
+    float *s = reinterpret_cast<float *>(sm + tap_slots(n));   // [8 * line_blocks][COLS]
+    const int64_t c0 = (int64_t)blockIdx.x * COLS;
+    const int l0 = blockIdx.y * ROWS;
+    const int64_t base = (int64_t)blockIdx.z * L * inner;
+    for (int i = threadIdx.x; i < n; i += kSepThreads) sw[i] = make_float2(taps.w[i], taps.w[i]);
+    const int span = min(ROWS, L - l0) + 2 * r;
+    if (vec) {
+        // 4 columns per thread (inner a multiple of 4); most tiles need no clamp
+        constexpr int QPR = COLS / 4, STEP = kSepThreads / QPR;
+        const int c = 4 * (threadIdx.x % QPR), j0 = threadIdx.x / QPR;
+        const Tin *p = src + base + min(c0 + c, inner - 4);
+        const bool inside = l0 >= r && l0 - r + span <= L;
+        if constexpr (sizeof(Tin) == 4) {
+            // float32: asynchronous copies, all in flight at once
+            const Tin *q = p + (int64_t)(inside ? l0 - r + j0 : 0) * inner;
+            for (int j = j0; j < span; j += STEP, q += (int64_t)STEP * inner)
+                copy_async16(s + j * COLS + c, inside ? q : p + (int64_t)clampi(l0 - r + j, 0, L - 1) * inner);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        } else {
+            for (int j = j0; j < span; j += 4 * STEP) {
+                float v[4][4];
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (j + b * STEP < span) load4(p + (int64_t)clampi(l0 - r + j + b * STEP, 0, L - 1) * inner, v[b]);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (j + b * STEP < span)
+                        *reinterpret_cast<float4 *>(s + (j + b * STEP) * COLS + c) = make_float4(v[b][0], v[b][1], v[b][2], v[b][3]);
+            }
+        }
+    } else {
+        constexpr int STEP = kSepThreads / COLS;
+        const int c = threadIdx.x % COLS, j0 = threadIdx.x / COLS;
+        const Tin *p = src + base + min(c0 + c, inner - 1);
+#pragma unroll 8
+        for (int j = j0; j < span; j += STEP) s[j * COLS + c] = to_f32(p[(int64_t)clampi(l0 - r + j, 0, L - 1) * inner]);
     }
     __syncthreads();
-    if (c >= inner) return;
-    for (int lo = threadIdx.y; lo < kColRows; lo += kColThreadsY) {
-        int l = l0 + lo;
-        if (l >= L) break;
-        float acc = 0.0f;
-        for (int i = 0; i < taps.n; ++i) acc = __fmaf_rn(taps.w[i], s[(lo + i) * kColW + threadIdx.x], acc);
-        dst[base + (int64_t)l * inner + c] = acc;
+    const int cp = threadIdx.x % NC, g = threadIdx.x / NC;
+    const int64_t c = c0 + 2 * cp;
+    float vmin = INFINITY, vmax = -INFINITY;   // of the stored values (when mm)
+    if (c < inner && l0 + g * kK < L) {
+        const float *col = s + g * kK * COLS + 2 * cp;
+        float2 acc[kK];
+#pragma unroll
+        for (int k = 0; k < kK; ++k) acc[k] = make_float2(0.f, 0.f);
+        tap_chain(sw, n, acc, [&](int j, float2 (&v)[kK]) {
+#pragma unroll
+            for (int k = 0; k < kK; ++k) v[k] = *reinterpret_cast<const float2 *>(col + (j * kK + k) * COLS);
+        });
+        float *o = dst + base + (int64_t)(l0 + g * kK) * inner + c;
+        const int left = L - (l0 + g * kK);
+        const bool two = c + 1 < inner;
+        const bool pair = (inner & 1) == 0 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0;
+#pragma unroll
+        for (int k = 0; k < kK; ++k) {
+            if (k < left) {
+                float *q = o + (int64_t)k * inner;
+                if (pair) *reinterpret_cast<float2 *>(q) = acc[k];
+                else {
+                    q[0] = acc[k].x;
+                    if (two) q[1] = acc[k].y;
+                }
+                if (mm) {
+                    vmin = fminf(vmin, acc[k].x);
+                    vmax = fmaxf(vmax, acc[k].x);
+                    if (two) { vmin = fminf(vmin, acc[k].y); vmax = fmaxf(vmax, acc[k].y); }
+                }
+            }
+        }
+    }
+    if (mm) {
+        __shared__ float s_mn[kSepThreads / 32], s_mx[kSepThreads / 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
+            vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+        }
+        if ((threadIdx.x & 31) == 0) { s_mn[threadIdx.x >> 5] = vmin; s_mx[threadIdx.x >> 5] = vmax; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kSepThreads / 32; ++w) { vmin = fminf(vmin, s_mn[w]); vmax = fmaxf(vmax, s_mx[w]); }
+            const int64_t cta = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+            mm[2 * cta] = vmin;
+            mm[2 * cta + 1] = vmax;
+        }
     }
 }
 
@@ -85,30 +299,62 @@ __global__ void convert_kernel(const Tin *__restrict__ src, float *__restrict__ 
         dst[i] = to_f32(src[i]);
 }
 
+// Thread groups along the axis of a col pass: short axes take fewer outputs and
+// more columns per CTA, as far as the staged lines of a long window fit shared
+// memory.
+int col_groups(int64_t L, int n) { return L <= 32 && n <= 129 ? 4 : L <= 64 && n <= 321 ? 8 : 16; }
+
+// CTAs of the last pass of an image (y in 2D, z in 3D) with n taps
+int64_t last_pass_ctas(const Img &im, int n) {
+    const bool vol = im.ndim == 3;
+    const int64_t L = vol ? im.D : im.H, inner = vol ? im.H * im.W : im.W;
+    const int ng = col_groups(L, n);
+    const int64_t cols = 2 * (kSepThreads / ng), rows = ng * kK;
+    return ((inner + cols - 1) / cols) * ((L + rows - 1) / rows);
+}
+
+template <typename Tin, int NG>
+int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, const Taps &t, float *mm,
+               cudaStream_t st) {
+    constexpr int COLS = 2 * (kSepThreads / NG), ROWS = NG * kK;
+    const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((L + ROWS - 1) / ROWS), (unsigned)outer);
+    const size_t smem = sizeof(float2) * tap_slots(t.n) + sizeof(float) * COLS * kK * line_blocks(ROWS, t.n);
+    if (smem > 48 * 1024)
+        CLE_CUDA(cudaFuncSetAttribute(blur_col_kernel<Tin, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int vec = inner % 4 == 0 && reinterpret_cast<uintptr_t>(src) % (4 * sizeof(Tin)) == 0;
+    blur_col_kernel<Tin, NG><<<grid, kSepThreads, smem, st>>>(src, dst, inner, L, vec, t, mm);
+    return CLE_OK;
+}
+
 template <typename Tin>
-int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps &t,
+int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps &t, float *mm,
                 cudaStream_t st) {
-    const int r = (t.n - 1) / 2;
     if (axis == 2) {
+        // the row split evenly into tiles of at most kRowMax outputs, row pairs
+        // to fill the CTA's threads
         const int64_t rows = im.D * im.H;
-        dim3 grid((unsigned)((im.W + kRowTile - 1) / kRowTile), (unsigned)std::min<int64_t>(rows, 65535),
-                  (unsigned)((rows + 65534) / 65535));
-        size_t smem = sizeof(float) * (kRowTile + 2 * r);
+        const int tiles = (int)((im.W + kRowMax - 1) / kRowMax);
+        const int tile = (int)(((im.W + tiles - 1) / tiles + kK - 1) / kK * kK);
+        const int np = std::max(1, std::min(kSepThreads / (tile / kK), 16));
+        const int64_t ctas = (rows + 2 * np - 1) / (2 * np);
+        const dim3 grid((unsigned)((im.W + tile - 1) / tile), (unsigned)std::min<int64_t>(ctas, 65535),
+                        (unsigned)((ctas + 65534) / 65535));
+        const size_t smem = sizeof(float2) * (tap_slots(t.n) + (size_t)np * kBlk * line_blocks(tile, t.n));
         if (smem > 48 * 1024)
             CLE_CUDA(cudaFuncSetAttribute(blur_row_kernel<Tin>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        blur_row_kernel<Tin><<<grid, kRowThreads, smem, st>>>(src, dst, rows, (int)im.W, t);
+        const int vec = im.W % 4 == 0 && reinterpret_cast<uintptr_t>(src) % (4 * sizeof(Tin)) == 0;
+        blur_row_kernel<Tin><<<grid, kSepThreads, smem, st>>>(src, dst, rows, (int)im.W, tile, np,
+                                                              FastDiv((uint32_t)(tile / kK)), vec, t);
     } else {
         int64_t inner, outer;
         int L;
         if (axis == 1) { inner = im.W; L = (int)im.H; outer = im.D; }
         else { inner = im.W * im.H; L = (int)im.D; outer = 1; }
-        dim3 grid((unsigned)((inner + kColW - 1) / kColW), (unsigned)((L + kColRows - 1) / kColRows),
-                  (unsigned)outer);
-        dim3 block(kColW, kColThreadsY);
-        size_t smem = sizeof(float) * kColW * (kColRows + 2 * r);
-        if (smem > 48 * 1024)
-            CLE_CUDA(cudaFuncSetAttribute(blur_col_kernel<Tin>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        blur_col_kernel<Tin><<<grid, block, smem, st>>>(src, dst, inner, L, outer, t);
+        switch (col_groups(L, t.n)) {
+            case 4: CLE_TRY((launch_col<Tin, 4>(src, dst, inner, L, outer, t, mm, st))); break;
+            case 8: CLE_TRY((launch_col<Tin, 8>(src, dst, inner, L, outer, t, mm, st))); break;
+            default: CLE_TRY((launch_col<Tin, 16>(src, dst, inner, L, outer, t, mm, st))); break;
+        }
     }
     CLE_LAUNCH_CHECK("blur pass");
     return CLE_OK;
@@ -122,7 +368,7 @@ int launch_convert(const Tin *src, float *dst, int64_t n, cudaStream_t st) {
 }
 
 template <typename Tin>
-int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, float *t2,
+int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, float *t2, float *mm,
                     cudaStream_t st) {
     // pass order x (axis 2), y (axis 1), z (axis 0, 3D only)
     const int passes = (src.ndim == 3) ? 3 : 2;
@@ -135,10 +381,10 @@ int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, 
         float *o = (p == passes - 1) ? dst : bufs[which];
         const Taps *t = taps[p];
         if (cur_is_src) {
-            if (t) CLE_TRY(launch_pass<Tin>((const Tin *)cur, o, src, 2 - p, *t, st));
+            if (t) CLE_TRY(launch_pass<Tin>((const Tin *)cur, o, src, 2 - p, *t, p == passes - 1 ? mm : nullptr, st));
             else CLE_TRY(launch_convert<Tin>((const Tin *)cur, o, n, st));
         } else {
-            if (t) CLE_TRY(launch_pass<float>((const float *)cur, o, src, 2 - p, *t, st));
+            if (t) CLE_TRY(launch_pass<float>((const float *)cur, o, src, 2 - p, *t, p == passes - 1 ? mm : nullptr, st));
             else if (o != cur) CLE_CUDA(cudaMemcpyAsync(o, cur, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
         }
         cur = o;
@@ -158,7 +404,7 @@ size_t separable_workspace_bytes(const Img &im) {
 }
 
 int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty, const Taps *tz,
-                     Arena &ws, cudaStream_t st) {
+                     Arena &ws, cudaStream_t st, float *mm) {
     float *t1 = ws.take<float>(src.n());
     float *t2 = ws.take<float>(src.n());
     if (!ws.ok()) {
@@ -167,9 +413,9 @@ int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty,
     }
     const Taps *taps[3] = {tx, ty, tz};
     switch (src.dtype) {
-        case CLE_F32: return separable_typed<float>(src, dst, taps, t1, t2, st);
-        case CLE_U16: return separable_typed<uint16_t>(src, dst, taps, t1, t2, st);
-        case CLE_U8: return separable_typed<uint8_t>(src, dst, taps, t1, t2, st);
+        case CLE_F32: return separable_typed<float>(src, dst, taps, t1, t2, mm, st);
+        case CLE_U16: return separable_typed<uint16_t>(src, dst, taps, t1, t2, mm, st);
+        case CLE_U8: return separable_typed<uint8_t>(src, dst, taps, t1, t2, mm, st);
         default:
             set_error("gaussian_blur: source dtype %d not supported (u8/u16/f32)", src.dtype);
             return CLE_ERR_DTYPE;
@@ -186,6 +432,23 @@ int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, A
     if (sy > 0) { CLE_TRY(make_gauss_taps(sy, ty)); py = &ty; }
     if (src.ndim == 3 && sz > 0) { CLE_TRY(make_gauss_taps(sz, tz)); pz = &tz; }
     return separable_filter(src, dst, px, py, pz, ws, st);
+}
+
+int separable_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st) {
+    Taps t;
+    CLE_TRY(make_gauss_taps(sigma, t));
+    const int64_t ctas = last_pass_ctas(src, t.n);
+    float *partial = ws.take<float>(2 * (size_t)ctas);
+    if (!ws.ok()) { set_error("gaussian_blur: workspace too small"); return CLE_ERR_WORKSPACE; }
+    CLE_TRY(separable_filter(src, dst, &t, &t, src.ndim == 3 ? &t : nullptr, ws, st, partial));
+    return minmax_finish(partial, (int)ctas, d_minmax, st);
+}
+
+size_t separable_minmax_workspace_bytes(const Img &src) {
+    // the most CTAs the last pass takes for any window
+    Arena a(nullptr, 0);
+    a.take<float>(2 * (size_t)std::max(last_pass_ctas(src, 1), last_pass_ctas(src, kMaxTaps)));
+    return a.off + separable_workspace_bytes(src);
 }
 
 }  // namespace cle

@@ -26,7 +26,12 @@
 //     slot per plane (the plane loop is not unrolled, which keeps the kernel's
 //     code small enough for the instruction caches).
 // Radius R (= sigma_to_kernel_size(sigma)/2) is a template parameter; radii
-// above kMaxFusedR or anisotropic sigmas use the three-pass path.  Given a
+// above the line and anisotropic sigmas use the three-pass path.  In 3D the
+// line is R = 8: above it the partial sums leave one CTA per SM and the halos of
+// tile and chunk (60 rows for 32, 28 planes) cost more than three passes over
+// memory do: R = 14 on 61 x 479 x 347 0.255 against 0.152 ms, 64 x 256 x 256
+// 0.095 / 0.062, 128 x 512 x 512 0.370 / 0.283, 128 x 1024 x 1024 1.295 / 0.974; R = 8
+// on the last two 0.179 / 0.238 and 0.517 / 0.866.  Given a
 // partial buffer, each CTA also reduces the exact min / max of the values it
 // stores (the global min / max of the result in a one-CTA finish), which
 // saves threshold_otsu's separate pass over the blurred image.
@@ -527,7 +532,7 @@ int launch_fused_r(const Img &src, float *dst, const Taps &t, float *mm, int *st
 
 template <typename Tin, bool Z, int R = 1>
 int dispatch_r(const Img &src, float *dst, const Taps &t, int r, float *mm, int *status, cudaStream_t st) {
-    if constexpr (R > kMaxFusedR) {
+    if constexpr (R > (Z ? kMaxFusedR3 : kMaxFusedR)) {
         set_error("internal: fused radius out of range");
         return CLE_ERR_ARG;
     } else {
@@ -543,7 +548,7 @@ bool fused_blur_applies(const Img &src, double sx, double sy, double sz) {
     if (src.ndim == 3 && sz != sx) return false;
     if (src.dtype != CLE_F32 && src.dtype != CLE_U16 && src.dtype != CLE_U8) return false;
     const int r = (sigma_to_kernel_size(sx) - 1) / 2;
-    return r >= 1 && r <= kMaxFusedR && src.W < (1 << 30) && src.H < (1 << 30);
+    return r >= 1 && r <= (src.ndim == 3 ? kMaxFusedR3 : kMaxFusedR) && src.W < (1 << 30) && src.H < (1 << 30);
 }
 
 int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, float *mm, int *status) {
@@ -560,19 +565,21 @@ int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, float 
 }
 
 size_t blur_minmax_workspace_bytes(const Img &src) {
-    // any sigma: the three-pass path with the separate min / max, or the
-    // fused partials (at most fused_chunk_cap z chunks per tile)
+    // any sigma: the three-pass path with its min / max, or the fused partials
+    // (at most fused_chunk_cap z chunks per tile)
     int dev = 0;
     cudaGetDevice(&dev);
     const int64_t tiles = ((src.W + kTX - 1) / kTX) * ((src.H + kTY - 1) / kTY);
     const int64_t chunks = fused_chunk_cap(tiles, std::max<int64_t>(src.D, 1), num_sms(dev));
     const size_t fused = sizeof(float) * 2 * (size_t)(tiles * chunks) + 256;
-    return std::max(fused, separable_workspace_bytes(src) + minmax_workspace_bytes(src));
+    return std::max(fused, std::max(separable_minmax_workspace_bytes(src),
+                                    separable_workspace_bytes(src) + minmax_workspace_bytes(src)));
 }
 
 int blur_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st,
                 int *status) {
     if (!fused_blur_applies(src, sigma, sigma, sigma)) {
+        if (sigma > 0) return separable_minmax(src, dst, sigma, d_minmax, ws, st);
         CLE_TRY(gaussian_blur(src, dst, sigma, sigma, sigma, ws, st, status));
         Img T = src;
         T.data = dst;

@@ -8,15 +8,20 @@ namespace cle {
 // blur.cu
 size_t separable_workspace_bytes(const Img &im);
 int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty, const Taps *tz,
-                     Arena &ws, cudaStream_t st);
+                     Arena &ws, cudaStream_t st, float *mm = nullptr);
+// Three-pass isotropic blur (sigma > 0) whose {min, max} lands in d_minmax,
+// reduced in the last pass (mm above: 2 floats per CTA of it).
+size_t separable_minmax_workspace_bytes(const Img &src);
+int separable_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st);
 // status (optional): a device status word; given it, the fused path of a
 // volume may stage planes with TMA copies and reports a stage wait that ran
 // out there (CLE_ERR_ITER_LIMIT)
 int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, Arena &ws,
                   cudaStream_t st, int *status = nullptr);
 
-// blur_fused.cu (isotropic sigma, radius <= kMaxFusedR, one launch)
-constexpr int kMaxFusedR = 14;
+// blur_fused.cu (isotropic sigma, one launch): radius up to kMaxFusedR in 2D,
+// kMaxFusedR3 in 3D
+constexpr int kMaxFusedR = 14, kMaxFusedR3 = 8;
 bool fused_blur_applies(const Img &src, double sx, double sy, double sz);
 // mm (optional): 2 floats per CTA, the CTA's min / max of the result
 int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, float *mm = nullptr,

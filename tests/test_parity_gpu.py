@@ -82,6 +82,31 @@ def test_gaussian_blur_tma_staging_bit_exact(cle, oracle, dtype, shape, sigma):
     assert np.array_equal(dst.cpu().numpy(), oracle.gaussian_blur(a.astype(np.float32), sigma, sigma, sigma))
 
 
+# three passes: tile widths and heights with remainders (8 outputs per thread,
+# 128 / 64 / 32 outputs per CTA along y and z by the axis length and the window),
+# odd row counts, every remainder of taps modulo 8, windows longer than the axis,
+# vector and scalar staging (bit exact: the same chain of fused multiply-adds)
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 9, 40), (33, 65, 36), (130, 7, 261), (66, 129, 4), (131, 263), (40, 516)])
+@pytest.mark.parametrize("sig", [(4.2, 0.3, 0.6), (1.1, 4.3, 1.3), (0.4, 6.0, 41.0), (64.0, 0.2, 2.7), (0.0, 3.7, 5.0)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_gaussian_blur_three_pass_bit_exact(cle, oracle, shape, sig, dtype):
+    r = rng(33)
+    a = (r.integers(0, np.iinfo(dtype).max, size=shape) if dtype != np.float32
+         else r.uniform(-1000, 1000, size=shape)).astype(dtype)
+    got = cle.pull(cle.gaussian_blur(a, None, *sig))
+    assert np.array_equal(got, oracle.gaussian_blur(a.astype(np.float32), *sig))
+
+
+def test_gaussian_blur_three_pass_keeps_infinities_local(cle):
+    # a value at infinity reaches the outputs whose window holds it and no others
+    a = np.ones((5, 40, 300), np.float32)
+    a[2, 20, 150] = np.inf
+    got = cle.pull(cle.gaussian_blur(a, None, 4, 1, 4))
+    bad = ~np.isfinite(got)
+    zz, yy, xx = np.nonzero(bad)
+    assert (yy.min(), yy.max(), xx.min(), xx.max()) == (16, 24, 134, 166)
+
+
 def test_gaussian_blur_reference_test(cle):
     # tests/test_gaussian_blur.py:4-22 of the reference
     t = np.zeros((5, 5))
