@@ -6,32 +6,44 @@
 // once:
 //   * a CTA owns a kTX x kTY output tile in (x, y) and marches along z over a
 //     chunk of planes (plus R halo planes at each end, clamped);
-//   * per input plane it stages the clamped (kTY+2R) x (kTX+2R) tile in
-//     shared memory as float32.  On volumes whose rows are a multiple of 16
-//     bytes and whose grid fills two waves of resident CTAs (and when the
-//     caller gives a status word) one thread fetches
-//     each plane's raw tile with a TMA copy (cp.async.bulk.tensor) into a ring
-//     of kStages shared-memory stages, kStages-1 planes ahead, completion
-//     counted by an mbarrier per stage; the CTA converts the landed tile to
-//     float32 with 64/128-bit shared loads.  Otherwise the next plane's raw
-//     values are loaded into registers while the current one is computed
-//     and converted when stored;
-//   * x pass: each item produces 8 consecutive x outputs of one row as four
-//     packed pairs (fma.rn.f32x2: two independent round-to-nearest FMAs, the
-//     same rounding as fmaf) from 128-bit shared loads; the operand pair of an
-//     odd offset is formed from the loaded registers;
-//   * y pass: each thread produces kRY rows of a pair of adjacent columns,
-//     the pair packed, from a register window of 64-bit shared loads;
-//   * z pass: a register ring of 2R+1 planes per owned column pair, shifted by one
-//     slot per plane (the plane loop is not unrolled, which keeps the kernel's
-//     code small enough for the instruction caches).
-// Radius R (= sigma_to_kernel_size(sigma)/2) is a template parameter; radii
-// above the line and anisotropic sigmas use the three-pass path.  In 3D the
-// line is R = 8: above it the partial sums leave one CTA per SM and the halos of
-// tile and chunk (60 rows for 32, 28 planes) cost more than three passes over
-// memory do: R = 14 on 61 x 479 x 347 0.255 against 0.152 ms, 64 x 256 x 256
-// 0.095 / 0.062, 128 x 512 x 512 0.370 / 0.283, 128 x 1024 x 1024 1.295 / 0.974; R = 8
-// on the last two 0.179 / 0.238 and 0.517 / 0.866.  Given a
+//   * planes go in groups of P (4, or 2 or 1 where shared memory is short).  The
+//     raw (kTY+2R) x (kTX+2R) tiles of a group are staged in shared memory in
+//     the source's own type, two groups deep.  On volumes whose rows are a
+//     multiple of 16 bytes (when the caller gives a status word) one thread
+//     fetches a group with TMA copies (cp.async.bulk.tensor) an interval
+//     ahead, completion counted by an mbarrier per stage; otherwise each
+//     thread loads its share of a plane into registers through a table of
+//     clamped offsets and stores it into the stage;
+//   * x pass: an item is 8 x outputs of two rows, the two rows packed
+//     (fma.rn.f32x2: two independent round-to-nearest FMAs, the same rounding
+//     as fmaf), from 128-bit shared loads of the raw rows, converted in
+//     registers (8/16-bit values by a byte permute into 2^23 + v and an exact
+//     subtraction).  Column pairs would need an operand pair per odd offset,
+//     which the compiler forms again at every use (66 moves an item: 1.92 ms
+//     against 1.73 for 512 x 1024 x 1024 at R = 8).  Rows are an odd number of
+//     16-byte granules apart, so the eight lanes of a load phase fall on
+//     different banks;
+//   * every pass runs in transposed form: a value is added to each output it
+//     contributes to, output o taking tap i at its i-th step, which is the
+//     same ascending chain per output.  So the x and y passes need no window
+//     of values, and the z pass keeps 2R partial sums per column; it takes a
+//     group's P planes at once, each partial sum moving P slots on;
+//   * group g + 1's x pass and group g's y and z passes share one interval
+//     between two CTA barriers (the x results are double-buffered).  One
+//     barrier per plane instead of one per group left 18% of the warp time in
+//     barriers (2.67 against 1.99 ms at that point).
+// What bounds it: at R = 8 a voxel takes 59.5 FMAs (x on 48 rows for 32), 0.93 ms
+// for 512 x 1024 x 1024 at 128 per SM and cycle; measured 1.73 ms (3.04 with three
+// barriers per plane, a float32 tile and a shifted z ring), the FMA pipe 65%
+// busy with 4 warps per scheduler, which the 2R partial sums allow (124
+// registers).
+// Radius R (= sigma_to_kernel_size(sigma)/2) is a template parameter; anisotropic
+// sigmas and larger radii use the three-pass path.  In 3D the line is R = 8:
+// above it the partial sums leave one CTA per SM and the halos of tile and chunk
+// (60 rows for 32, 28 planes) cost more than three passes over memory do: R = 14
+// on 61 x 479 x 347 0.251 against 0.152 ms, 64 x 256 x 256 0.106 / 0.062,
+// 128 x 512 x 512 0.370 / 0.283, 128 x 1024 x 1024 1.295 / 0.974; R = 8 on the last two
+// 0.179 / 0.238 and 0.517 / 0.866.  Given a
 // partial buffer, each CTA also reduces the exact min / max of the values it
 // stores (the global min / max of the result in a one-CTA finish), which
 // saves threshold_otsu's separate pass over the blurred image.
@@ -49,56 +61,65 @@ namespace {
 
 constexpr int kTX = 32;          // output columns per CTA
 constexpr int kTY = 32;          // output rows per CTA
-constexpr int kRY = 2;           // output rows per thread (y and z passes)
 constexpr int kCP = kTX / 2;     // column pairs per tile (y and z passes own a pair)
-constexpr int kXO = 8;           // x outputs per x-pass item
+constexpr int kRY = 2;           // output rows per thread (y and z passes)
 constexpr int kThreads = kCP * (kTY / kRY);   // 256
 constexpr int kWarps = kThreads / 32;
+constexpr int kXS = kTX + 4;     // row stride of the x results (an odd number of 16-byte granules)
+constexpr uint64_t kStageWaitNs = 2000000000ull;   // bound of one stage wait
 
+// Resident CTAs per SM the registers allow (2R partial sums per owned column).
 template <int R>
+constexpr int min_ctas() { return R <= 4 ? 3 : 2; }
+
+template <typename Tin, int R, bool Z>
 struct Geom {
-    static constexpr int ROWS = kTY + 2 * R;                     // staged rows
-    static constexpr int COLS = kTX + 2 * R;                     // staged columns
-    static constexpr int QUADS = (kXO + 2 * R + 3) / 4;          // float4 per x-pass item
-    static constexpr int STRIDE = ((COLS + 3) / 4) * 4 + 4;      // In row stride (floats)
-    static constexpr int ROWS_PER_WARP = (ROWS + kWarps - 1) / kWarps;
-    static constexpr int COL_LOADS = (COLS + 31) / 32;
-    static constexpr int LOADS = ROWS_PER_WARP * COL_LOADS;
-    static constexpr size_t SMEM = sizeof(float) * (ROWS * STRIDE + ROWS * kTX);
-    static_assert(ROWS * (kTX / kXO) <= kThreads, "x pass: at most one item per thread");
+    static constexpr int ES = (int)sizeof(Tin);
+    // x outputs per x-pass item; a single image has no other plane's work to
+    // fill the threads with, so smaller items
+    static constexpr int XO = Z ? 8 : 4;
+    static constexpr int A = 16 / ES;                             // elements per 16-byte granule
+    // the staged row starts at x0 - R - OFF, a multiple of 16 bytes from the row's start
+    static constexpr int OFF = (R + A - 1) / A * A - R;
+    static constexpr int ROWS = kTY + 2 * R;
+    static constexpr int COLS = kTX + 2 * R;
+    static constexpr int GR = (OFF + COLS + A - 1) / A;           // granules a row needs
+    static constexpr int BX = (GR | 1) * A;                       // row stride (odd granules)
+    static constexpr int VB = std::min(16, XO * ES);              // bytes per load of an x item
+    static constexpr int VA = VB / ES;                            // elements of one
+    static constexpr int NV = (OFF + XO + 2 * R + VA - 1) / VA;  // loads per x item
+    static constexpr int ITEMS = ROWS / 2 * (kTX / XO);          // x items per plane (two rows each)
+    static constexpr uint32_t BYTES = (uint32_t)(BX * ROWS * ES); // one plane's copy
+    static constexpr int STAGE = (int)((BYTES + 127) / 128 * 128);
+    static constexpr int LOADS = (ROWS * BX + kThreads - 1) / kThreads;
+    static constexpr int XBUF = ROWS * kXS;                       // floats of one plane's x results
+    static constexpr size_t TAB = Z ? sizeof(int) * ROWS * BX : 0;   // offset table of the register staging
+    static constexpr size_t smem_of(int p) {
+        return 128 + (size_t)(Z ? 2 * p : 1) * (STAGE + sizeof(float) * XBUF) + TAB;
+    }
+    // planes per group: as many as leave room for min_ctas CTAs per SM
+    static constexpr int fit(int p) { return p == 1 || (size_t)min_ctas<R>() * (smem_of(p) + 2048) <= 227 * 1024 ? p : fit(p / 2); }
+    static constexpr int P = Z ? fit(4) : 1;
+    static constexpr size_t SMEM = smem_of(P);
+    static_assert((kTX / XO - 1) * XO + NV * VA <= BX, "x item reads inside the staged row");
+    static_assert((BX * ES / 16) % 2 == 1 && XO * ES % VB == 0, "aligned x items on odd row strides");
+    static_assert(BX <= 256 && ROWS <= 256, "TMA box dimension above 256");
 };
 
-// Two CTAs per SM (<= 128 registers, no spills) while the z ring is small.
+// Taps -R..0 (a Gaussian's taps are symmetric: tap i and tap -i come from the
+// same i * i), a kernel parameter.
 template <int R>
-constexpr int min_ctas() { return R <= 8 ? 2 : 1; }
+struct HalfTaps {
+    float w[R + 1];
+};
 
 // ---- TMA staging ------------------------------------------------------------
 // The box of a plane starts at x = x0 - R - OFF (OFF rounds it down so that
 // x * sizeof(Tin) is a multiple of 16 bytes, the tiled copy's rule for the
 // innermost coordinate), y = y0 - R and z = the clamped plane.  Box parts
-// outside the image arrive zero-filled and are never read: the conversion
-// gathers every staged element from its clamped coordinate, which lies inside
-// both the image and the box.
-constexpr int kStages = 3;
-constexpr uint64_t kStageWaitNs = 2000000000ull;   // bound of one stage wait
-
-template <typename Tin, int R>
-struct TmaGeom {
-    static constexpr int ES = (int)sizeof(Tin);
-    static constexpr int A = 16 / ES;                                   // x alignment (elements)
-    static constexpr int OFF = (R + A - 1) / A * A - R;
-    static constexpr int BX = (Geom<R>::COLS + OFF + A - 1) / A * A;    // box columns
-    static constexpr int BY = Geom<R>::ROWS;                            // box rows
-    static constexpr uint32_t BYTES = (uint32_t)(BX * BY * ES);         // one plane's copy
-    static constexpr int STAGE = (int)((BYTES + 127) / 128 * 128);
-    static constexpr bool VEC = OFF % 4 == 0;                           // quads start 4-aligned
-    static constexpr int QC = (Geom<R>::COLS + 3) / 4;                  // quads per staged row
-    static constexpr int QPT = (BY * QC + kThreads - 1) / kThreads;     // quads per thread
-    static constexpr size_t SMEM = 128 + (size_t)kStages * STAGE + Geom<R>::SMEM;
-    static_assert(BX <= 256 && BY <= 256, "TMA box dimension above 256");
-    static_assert(!VEC || 4 * QC + OFF <= BX, "quad conversion reads inside the box row");
-};
-
+// outside the image arrive zero-filled; a CTA whose tile reaches over the
+// image's x or y edge then overwrites them in the stage with their clamped
+// elements, which lie inside both the image and the box.
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -131,6 +152,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
         if (global_ns() - t0 > kStageWaitNs) return false;
     return true;
 }
+// The same inside a CTA: a wait that runs out raises *fail, and a raised *fail
+// ends every wait.
+__device__ __forceinline__ void mbar_wait_or_fail(uint64_t *bar, uint32_t parity, int *fail) {
+    if (mbar_try_wait(bar, parity)) return;
+    const uint64_t t0 = global_ns();
+    while (!mbar_try_wait(bar, parity)) {
+        if (*(volatile int *)fail != 0) return;
+        if (global_ns() - t0 > kStageWaitNs) { *(volatile int *)fail = 1; return; }
+    }
+}
 // Orders this thread's earlier shared-memory accesses before its next
 // async-proxy (TMA) write into the same memory.
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -145,76 +176,187 @@ __device__ __forceinline__ void tma_load_plane(void *dst, const CUtensorMap *map
         : "memory");
 }
 
-// four consecutive staged source values as float32 (the same values as to_f32)
-__device__ __forceinline__ float4 quad_f32(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ float4 quad_f32(const uint16_t *p) {
-    const uint2 u = *reinterpret_cast<const uint2 *>(p);
-    return make_float4((float)(u.x & 0xFFFFu), (float)(u.x >> 16), (float)(u.y & 0xFFFFu), (float)(u.y >> 16));
+// Staged source values as float32 (the same values as to_f32), one of two rows
+// each, as a packed pair: element k of the 32-bit words u and v.  An unsigned
+// value below 2^23: its bits under the exponent of 2^23 are 2^23 + value
+// exactly, and subtracting 2^23 is exact.
+__device__ __forceinline__ float2 word_pair(uint32_t u, uint32_t v, int, float) {
+    return make_float2(__uint_as_float(u), __uint_as_float(v));
 }
-__device__ __forceinline__ float4 quad_f32(const uint8_t *p) {
-    const uint32_t u = *reinterpret_cast<const uint32_t *>(p);
-    return make_float4((float)(u & 0xFFu), (float)((u >> 8) & 0xFFu), (float)((u >> 16) & 0xFFu), (float)(u >> 24));
+__device__ __forceinline__ float2 word_pair(uint32_t u, uint32_t v, int k, uint16_t) {
+    const uint32_t sel = k ? 0x7432u : 0x7410u;
+    return __fadd2_rn(make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, sel)), __uint_as_float(__byte_perm(v, 0x4B000000u, sel))),
+                      make_float2(-8388608.0f, -8388608.0f));
+}
+__device__ __forceinline__ float2 word_pair(uint32_t u, uint32_t v, int k, uint8_t) {
+    const uint32_t sel = 0x7440u + (uint32_t)k;
+    return __fadd2_rn(make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, sel)), __uint_as_float(__byte_perm(v, 0x4B000000u, sel))),
+                      make_float2(-8388608.0f, -8388608.0f));
+}
+// VB (16, 8 or 4) bytes from shared memory
+template <int VB>
+__device__ __forceinline__ void load_words(const uint8_t *p, uint32_t *w) {
+    if constexpr (VB == 16) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(p);
+        w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+    } else if constexpr (VB == 8) {
+        const uint2 u = *reinterpret_cast<const uint2 *>(p);
+        w[0] = u.x; w[1] = u.y;
+    } else {
+        w[0] = *reinterpret_cast<const uint32_t *>(p);
+    }
 }
 
-// TMA: stage planes with the tensor map `tmap` (3D only); a stage wait that
-// runs out sets *status and ends the CTA after its copies have landed.
+// TMA: stage planes with the tensor map `tmap` (3D only).  A stage wait that
+// runs out raises s_fail: no later wait blocks, no more copies are issued, the
+// copies in flight are waited for and *status is set.
 template <typename Tin, int R, bool Z, bool TMA>
-__global__ void __launch_bounds__(kThreads, min_ctas<R>())
+__global__ void __launch_bounds__(kThreads, (min_ctas<R>()))
 blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorMap tmap,
                   float *__restrict__ dst, int D, int H, int W, int zchunk,
-                  const __grid_constant__ Taps taps, float *__restrict__ mm, int *__restrict__ status) {
+                  const __grid_constant__ HalfTaps<R> taps, float *__restrict__ mm, int *__restrict__ status) {
     static_assert(!TMA || Z, "TMA staging is for volumes");
-    using G = Geom<R>;
-    using TG = TmaGeom<Tin, R>;
-    constexpr int WIN = 2 * R + 1;
-    extern __shared__ __align__(16) float smem[];
-    // TMA: kStages raw stages first (128-byte aligned), then In and Xo
-    uint8_t *raw = reinterpret_cast<uint8_t *>(smem);
-    if constexpr (TMA) raw += (128u - (smem_addr(smem) & 127u)) & 127u;
-    float *In = TMA ? reinterpret_cast<float *>(raw + kStages * TG::STAGE) : smem;   // [ROWS][STRIDE]
-    float *Xo = In + G::ROWS * G::STRIDE;                                             // [ROWS][kTX]
+    using G = Geom<Tin, R, Z>;
+    constexpr int WIN = 2 * R + 1, BX = G::BX, P = G::P;
+    constexpr bool kRegStage = Z && !TMA;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    // raw stages [1 or 2][P][STAGE], x results [1 or 2][P][ROWS][kXS], offsets
+    uint8_t *raw = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
+    float *Xo = reinterpret_cast<float *>(raw + (Z ? 2 * P : 1) * G::STAGE);
+    int *tab = reinterpret_cast<int *>(Xo + (Z ? 2 * P : 1) * G::XBUF);
+
+    // in 3D the taps stay in registers as packed pairs (w, w), read once
+    // through shared memory: taken from the parameter they are fetched for
+    // every use, two register moves each
+    float2 wr[R + 1];
+    if constexpr (Z) {
+        __shared__ float s_taps[R + 1];
+        if (threadIdx.x <= R) s_taps[threadIdx.x] = taps.w[threadIdx.x];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i <= R; ++i) {
+            wr[i].x = *(volatile float *)&s_taps[i];
+            wr[i].y = *(volatile float *)&s_taps[i];
+        }
+    }
+    auto tap = [&](int i) {
+        const int k = i <= R ? i : 2 * R - i;
+        if constexpr (Z) return wr[k];
+        else return make_float2(taps.w[k], taps.w[k]);
+    };
 
     const int tid = threadIdx.x;
     const int x0 = blockIdx.x * kTX;
     const int y0 = blockIdx.y * kTY;
     const int z0 = Z ? (int)blockIdx.z * zchunk : 0;
     const int z1 = Z ? min(D, z0 + zchunk) : 1;
-    // virtual planes z0-R .. z1-1+R (clamped); 2D: the single plane
+    // virtual planes z0-R .. z1-1+R (clamped), in groups of P; 2D: the single plane
     const int nvirt = Z ? (z1 - z0) + 2 * R : 1;
+    const int ngroups = (nvirt + P - 1) / P;
     const int zbase = Z ? z0 - R : 0;
     const int64_t plane = (int64_t)H * W;
+    const int xs = x0 - R - G::OFF, ys = y0 - R;   // image coordinates of the staged tile's first element
+    // plane p of group g
+    auto stage = [&](int g, int p) { return reinterpret_cast<Tin *>(raw + ((Z ? (g & 1) * P : 0) + p) * G::STAGE); };
+    auto xres = [&](int g, int p) { return Xo + ((Z ? (g & 1) * P : 0) + p) * G::XBUF; };
 
-    // staging: warp w loads rows w, w+kWarps, ...; lane loads columns
-    // lane, lane+32, ... (clamped to the image)
-    const int lane = tid & 31, warp = tid >> 5;
-    int gx[G::COL_LOADS];
-#pragma unroll
-    for (int c = 0; c < G::COL_LOADS; ++c) gx[c] = clampi(x0 - R + lane + 32 * c, 0, W - 1);
-    // raw source values; converted when stored, so the loads of the next
-    // plane stay in flight while the current plane is computed
+    // register staging: element s of the stage comes from image offset tab[s]
+    // (clamped); raw values, so the loads stay in flight until stored
     Tin pre[TMA ? 1 : G::LOADS];
+    auto offset_of = [&](int s) {
+        const int r = s / BX, c = s - r * BX;
+        return clampi(ys + r, 0, H - 1) * W + clampi(xs + c, 0, W - 1);
+    };
     auto load_plane = [&](int v) {
-        const int zi = Z ? clampi(zbase + v, 0, D - 1) : 0;
-        const Tin *p = src + (int64_t)zi * plane;
+        const Tin *p = src + (int64_t)(Z ? clampi(zbase + v, 0, D - 1) : 0) * plane;
 #pragma unroll
-        for (int rr = 0; rr < G::ROWS_PER_WARP; ++rr) {
-            const int r = warp + rr * kWarps;
-            const Tin *row = p + (int64_t)clampi(y0 - R + r, 0, H - 1) * W;
-#pragma unroll
-            for (int c = 0; c < G::COL_LOADS; ++c) {
-                const bool ok = r < G::ROWS && lane + 32 * c < G::COLS;
-                if constexpr (!TMA) pre[rr * G::COL_LOADS + c] = ok ? __ldg(row + gx[c]) : Tin(0);
-            }
+        for (int k = 0; k < G::LOADS; ++k) {
+            const int s = tid + k * kThreads;
+            if constexpr (!TMA) pre[k] = s < G::ROWS * BX ? __ldg(p + (Z ? tab[s] : offset_of(s))) : Tin(0);
         }
     };
-    auto store_plane = [&]() {
+    auto store_plane = [&](Tin *d) {
 #pragma unroll
-        for (int rr = 0; rr < G::ROWS_PER_WARP; ++rr) {
-            const int r = warp + rr * kWarps;
+        for (int k = 0; k < G::LOADS; ++k) {
+            const int s = tid + k * kThreads;
+            if constexpr (!TMA)
+                if (s < G::ROWS * BX) d[s] = pre[k];
+        }
+    };
+
+    // TMA staging: one barrier per stage; a tile over the image's edge is patched
+    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ int s_fail;
+    const bool patch = xs + G::OFF < 0 || ys < 0 || x0 + kTX + R > W || y0 + kTY + R > H;
+    auto issue = [&](int g) {   // one thread: group g into its stage
+        const int n = min(P, nvirt - g * P);
+        fence_proxy_async_smem();
+        mbar_expect_tx(&bars[g & 1], (uint32_t)n * G::BYTES);
+        for (int p = 0; p < n; ++p)
+            tma_load_plane(stage(g, p), &tmap, xs, ys, clampi(zbase + g * P + p, 0, D - 1), &bars[g & 1]);
+    };
+    auto patch_plane = [&](Tin *d) {
+        // columns left / right of the image, then rows above / below it; an
+        // element inside the image is a source only, so the order is free
+        const int nl = max(0, -(xs + G::OFF)), nc = nl + max(0, x0 + kTX + R - W);
+        for (int e = tid; e < nc * G::ROWS; e += kThreads) {
+            const int k = e / G::ROWS, r = e - k * G::ROWS;
+            const int c = G::OFF + (k < nl ? k : G::COLS - nc + k);
+            d[r * BX + c] = d[(clampi(ys + r, 0, H - 1) - ys) * BX + clampi(xs + c, 0, W - 1) - xs];
+        }
+        const int nt = max(0, -ys), nr = nt + max(0, y0 + kTY + R - H);
+        for (int e = tid; e < nr * G::COLS; e += kThreads) {
+            const int k = e / G::COLS, c = G::OFF + e - k * G::COLS;
+            const int r = k < nt ? k : G::ROWS - nr + k;
+            d[r * BX + c] = d[(clampi(ys + r, 0, H - 1) - ys) * BX + clampi(xs + c, 0, W - 1) - xs];
+        }
+        fence_proxy_async_smem();
+    };
+    // TMA: group g has landed (and is patched); its barrier's phase is g / 2
+    auto arrive_group = [&](int g) {
+        mbar_wait_or_fail(&bars[g & 1], (uint32_t)(g >> 1) & 1u, &s_fail);
+        if (patch) {                       // uniform per CTA
+            for (int p = 0; p < P; ++p) patch_plane(stage(g, p));
+            __syncthreads();
+        }
+    };
+
+    // x pass of group g: an item is XO outputs of rows r and r + ROWS / 2 of a
+    // plane, the two rows packed; column c of the item adds tap c - k to
+    // output k
+    auto x_pass = [&](int g) {
+        constexpr int HR = G::ROWS / 2, EW = 4 / G::ES;     // EW: elements per 32-bit word
+        const int n = min(P, nvirt - g * P) * G::ITEMS;
+#pragma unroll 1
+        for (int e = tid; e < n; e += kThreads) {
+            const int p = P == 1 ? 0 : e / G::ITEMS, q0 = e - p * G::ITEMS;
+            const int part = q0 / HR, r = q0 - part * HR;
+            const uint8_t *pa = reinterpret_cast<const uint8_t *>(stage(g, p) + r * BX + part * G::XO);
+            float2 acc[G::XO];
 #pragma unroll
-            for (int c = 0; c < G::COL_LOADS; ++c)
-                if constexpr (!TMA)
-                    if (r < G::ROWS && lane + 32 * c < G::COLS) In[r * G::STRIDE + lane + 32 * c] = to_f32(pre[rr * G::COL_LOADS + c]);
+            for (int k = 0; k < G::XO; ++k) acc[k] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < G::NV; ++q) {
+                uint32_t u[G::VB / 4], w[G::VB / 4];
+                load_words<G::VB>(pa + q * G::VB, u);
+                load_words<G::VB>(pa + q * G::VB + HR * BX * G::ES, w);
+#pragma unroll
+                for (int t = 0; t < G::VA; ++t) {
+                    const int c = q * G::VA + t - G::OFF;
+                    if (c >= 0 && c < G::XO + 2 * R) {
+                        const float2 f = word_pair(u[t / EW], w[t / EW], t % EW, Tin());
+#pragma unroll
+                        for (int k = 0; k < G::XO; ++k)
+                            if (c - k >= 0 && c - k <= 2 * R) acc[k] = __ffma2_rn(tap(c - k), f, acc[k]);
+                    }
+                }
+            }
+            float *xo = xres(g, p) + r * kXS + part * G::XO;
+#pragma unroll
+            for (int k = 0; k < G::XO; k += 4) {
+                *reinterpret_cast<float4 *>(xo + k) = make_float4(acc[k].x, acc[k + 1].x, acc[k + 2].x, acc[k + 3].x);
+                *reinterpret_cast<float4 *>(xo + HR * kXS + k) = make_float4(acc[k].y, acc[k + 1].y, acc[k + 2].y, acc[k + 3].y);
+            }
         }
     };
 
@@ -224,11 +366,11 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
     const bool c0_ok = (x0 + tx) < W, c1_ok = (x0 + tx + 1) < W;
     const bool pair_store = c1_ok && (W & 1) == 0;     // 8-byte aligned float2 store
     float vmin = INFINITY, vmax = -INFINITY;   // of the stored values (when mm)
-    auto store2 = [&](int64_t off, float2 v) {
-        if (pair_store) *reinterpret_cast<float2 *>(dst + off) = v;
+    auto store2 = [&](float *o, float2 v) {
+        if (pair_store) *reinterpret_cast<float2 *>(o) = v;
         else {
-            if (c0_ok) dst[off] = v.x;
-            if (c1_ok) dst[off + 1] = v.y;
+            if (c0_ok) o[0] = v.x;
+            if (c1_ok) o[1] = v.y;
         }
         if (mm) {
             vmin = fminf(vmin, v.x);
@@ -236,154 +378,126 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
             if (c1_ok) { vmin = fminf(vmin, v.y); vmax = fmaxf(vmax, v.y); }
         }
     };
+    // rows this thread stores, and the output place that plane 0 of the group would finish
+    const int nrow = c0_ok ? min(kRY, H - (y0 + ry0)) : 0;
+    float *op = dst + (int64_t)(z0 - (Z ? 2 * R : 0)) * plane + (int64_t)(y0 + ry0) * W + x0 + tx;
 
-    float2 ring[kRY][WIN];
+    // z partial sums: ring[j][i] of row j belongs to the output plane that has
+    // taken taps 0..i (2R of them under way)
+    float2 ring[kRY][2 * R];
 #pragma unroll
     for (int j = 0; j < kRY; ++j)
 #pragma unroll
-        for (int i = 0; i < WIN; ++i) ring[j][i] = make_float2(0.0f, 0.0f);
+        for (int i = 0; i < 2 * R; ++i) ring[j][i] = make_float2(0.0f, 0.0f);
 
-    // TMA staging state: per-stage barriers, box origin, and for tiles that
-    // need no x clamp the quads this thread converts (raw offset in elements,
-    // In offset in floats; -1 = none)
-    __shared__ __align__(8) uint64_t bars[kStages];
-    const int xs = x0 - R - TG::OFF, ys = y0 - R;
-    const bool quads = TG::VEC && x0 - R >= 0 && x0 - R + G::COLS <= W;
-    int qsrc[TG::QPT], qdst[TG::QPT];
-    auto issue = [&](int v) {   // one thread: plane v into stage v % kStages
-        uint64_t *bar = &bars[v % kStages];
-        fence_proxy_async_smem();
-        mbar_expect_tx(bar, TG::BYTES);
-        tma_load_plane(raw + (v % kStages) * TG::STAGE, &tmap, xs, ys, clampi(zbase + v, 0, D - 1), bar);
-    };
-    auto convert = [&](const Tin *rs) {
-        if (quads) {
-#pragma unroll
-            for (int k = 0; k < TG::QPT; ++k)
-                if (qsrc[k] >= 0) *reinterpret_cast<float4 *>(In + qdst[k]) = quad_f32(rs + qsrc[k]);
-        } else {
-            for (int e = tid; e < G::ROWS * G::COLS; e += kThreads) {
-                const int r = e / G::COLS, c = e - r * G::COLS;
-                const int sr = clampi(ys + r, 0, H - 1) - ys;
-                const int sc = clampi(x0 - R + c, 0, W - 1) - xs;
-                In[r * G::STRIDE + c] = to_f32(rs[sr * TG::BX + sc]);
-            }
-        }
-    };
+    // groups 0 and 1 on their way, group 0 through its x pass
+    int issued = 0;   // TMA, thread 0: groups issued
     if constexpr (TMA) {
-#pragma unroll
-        for (int k = 0; k < TG::QPT; ++k) {
-            const int e = tid + k * kThreads;
-            const int r = e / TG::QC, q = e - r * TG::QC;
-            const bool ok = e < TG::BY * TG::QC;
-            qsrc[k] = ok ? (clampi(ys + r, 0, H - 1) - ys) * TG::BX + 4 * q + TG::OFF : -1;
-            qdst[k] = r * G::STRIDE + 4 * q;
-        }
         if (tid == 0) {
-            for (int s = 0; s < kStages; ++s) mbar_init(&bars[s], 1);
+            s_fail = 0;
+            mbar_init(&bars[0], 1);
+            mbar_init(&bars[1], 1);
             mbar_init_fence();
         }
         __syncthreads();
         if (tid == 0)
-            for (int v = 0; v < kStages - 1 && v < nvirt; ++v) issue(v);
+            for (; issued < 2 && issued < ngroups; ++issued) issue(issued);
+        arrive_group(0);
     } else {
-        load_plane(0);
-    }
-    int failed_at = -1;   // TMA: plane whose stage wait ran out
-    // one plane per iteration, not unrolled (the loop body stays small enough
-    // for the instruction caches); the ring shifts by one slot per plane, so
-    // ring[j][i] holds plane v - 2R + i
-#pragma unroll 1
-    for (int v = 0; v < nvirt; ++v) {
-        __syncthreads();   // previous plane fully consumed (In, Xo, its stage)
-        if constexpr (TMA) {
-            if (tid == 0 && v + kStages - 1 < nvirt) issue(v + kStages - 1);
-            const bool ok = mbar_wait(&bars[v % kStages], (uint32_t)(v / kStages) & 1u);
-            if (ok) convert(reinterpret_cast<const Tin *>(raw + (v % kStages) * TG::STAGE));
-            if (__syncthreads_or(!ok)) { failed_at = v; break; }
-        } else {
-            store_plane();
-            if (v + 1 < nvirt) load_plane(v + 1);
+        if constexpr (Z) {
+            for (int s = tid; s < G::ROWS * BX; s += kThreads) tab[s] = offset_of(s);
             __syncthreads();
         }
-        // x pass: rows 0..ROWS-1, kXO outputs per item as packed pairs; the
-        // operand pair of an odd offset is formed from the loaded registers
-        if (tid < G::ROWS * (kTX / kXO)) {
-            const int r = tid / (kTX / kXO);
-            const int xq = (tid - r * (kTX / kXO)) * kXO;
-            float2 A[2 * G::QUADS];                    // A[k] = (v[xq+2k], v[xq+2k+1])
-            const float4 *pa = reinterpret_cast<const float4 *>(In + r * G::STRIDE + xq);
-#pragma unroll
-            for (int q = 0; q < G::QUADS; ++q) {
-                const float4 f = pa[q];
-                A[2 * q] = make_float2(f.x, f.y);
-                A[2 * q + 1] = make_float2(f.z, f.w);
-            }
-            float2 acc[kXO / 2];
-#pragma unroll
-            for (int p = 0; p < kXO / 2; ++p) acc[p] = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < WIN; ++i) {
-                const float2 w = make_float2(taps.w[i], taps.w[i]);
-#pragma unroll
-                for (int p = 0; p < kXO / 2; ++p) {
-                    const int o = 2 * p + i;               // operand (v[xq+o], v[xq+o+1])
-                    const float2 opnd = (o % 2 == 0) ? A[o / 2] : make_float2(A[o / 2].y, A[o / 2 + 1].x);
-                    acc[p] = __ffma2_rn(w, opnd, acc[p]);
-                }
-            }
-            float4 *xo = reinterpret_cast<float4 *>(Xo + r * kTX + xq);
-#pragma unroll
-            for (int p = 0; p < kXO / 4; ++p)
-                xo[p] = make_float4(acc[2 * p].x, acc[2 * p].y, acc[2 * p + 1].x, acc[2 * p + 1].y);
+        for (int v = 0; v < nvirt && v < 2 * P; ++v) {
+            load_plane(v);
+            store_plane(stage(v / P, v % P));
         }
         __syncthreads();
-        // y pass: kRY rows of the column pair
-        float2 col[kRY + 2 * R];
+    }
+    x_pass(0);
+    __syncthreads();
+    if constexpr (TMA) {
+        if (tid == 0 && issued < ngroups && *(volatile int *)&s_fail == 0) issue(issued++);
+    }
+    // one group per interval between two barriers: group g + 1's x pass (its
+    // stage has landed) and group g's y and z passes; the plane loop is not
+    // unrolled (its body stays small enough for the instruction caches)
+#pragma unroll 1
+    for (int g = 0; g < ngroups; ++g) {
+        if (Z && g + 1 < ngroups) {
+            if constexpr (TMA) arrive_group(g + 1);
+            x_pass(g + 1);
+        }
+        // y pass: kRY rows of the column pair; row j of the window adds tap
+        // j - o to output row o.  Planes past the last one give values that
+        // only reach outputs past the last one.
+        float2 yv[P][kRY];
 #pragma unroll
-        for (int j = 0; j < kRY + 2 * R; ++j) col[j] = *reinterpret_cast<const float2 *>(Xo + (ry0 + j) * kTX + tx);
-        float2 yv[kRY];
+        for (int p = 0; p < P; ++p) {
+            if constexpr (kRegStage) {
+                if (g * P + p + 2 * P < nvirt) load_plane(g * P + p + 2 * P);
+            }
+            const float *xr = xres(g, p) + ry0 * kXS + tx;
 #pragma unroll
-        for (int j = 0; j < kRY; ++j) {
-            float2 a = make_float2(0.f, 0.f);
+            for (int o = 0; o < kRY; ++o) yv[p][o] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < WIN; ++i) a = __ffma2_rn(make_float2(taps.w[i], taps.w[i]), col[j + i], a);
-            yv[j] = a;
+            for (int j = 0; j < kRY + 2 * R; ++j) {
+                const float2 c = *reinterpret_cast<const float2 *>(xr + j * kXS);
+#pragma unroll
+                for (int o = 0; o < kRY; ++o)
+                    if (j - o >= 0 && j - o <= 2 * R) yv[p][o] = __ffma2_rn(tap(j - o), c, yv[p][o]);
+            }
+            // the stage of group g was consumed an interval ago
+            if constexpr (kRegStage) {
+                if (g * P + p + 2 * P < nvirt) store_plane(stage(g, p));
+            }
         }
         if constexpr (Z) {
+            // z pass, P planes at a time: the partial sum with taps 0..a takes
+            // taps a + 1.. from the group's planes in order; the one that takes
+            // tap 2R is finished by that plane, the others move on P slots
+            // (descending a: slot a + P has been read before it is written)
 #pragma unroll
             for (int j = 0; j < kRY; ++j) {
+                float2 out[P];
 #pragma unroll
-                for (int i = 0; i < WIN - 1; ++i) ring[j][i] = ring[j][i + 1];
-                ring[j][WIN - 1] = yv[j];
-            }
-            // z pass: output plane z0 + v - 2R once 2R+1 planes are held
-            if (v >= 2 * R) {
-                const int zo = z0 + v - 2 * R;
+                for (int a = 2 * R - 1; a >= -P; --a) {
+                    float2 t = a >= 0 ? ring[j][a >= 0 ? a : 0] : make_float2(0.f, 0.f);
 #pragma unroll
-                for (int j = 0; j < kRY; ++j) {
-                    float2 a = make_float2(0.f, 0.f);
+                    for (int p = 0; p < P; ++p) {
+                        const int i = a + 1 + p;
+                        if (i >= 0 && i <= 2 * R) {
+                            t = __ffma2_rn(tap(i), yv[p][j], t);
+                            if (i == 2 * R) out[p] = t;
+                        }
+                    }
+                    if (a + P < 2 * R) ring[j][a + P < 2 * R ? a + P : 0] = t;
+                }
 #pragma unroll
-                    for (int i = 0; i < WIN; ++i) a = __ffma2_rn(make_float2(taps.w[i], taps.w[i]), ring[j][i], a);
-                    const int y = y0 + ry0 + j;
-                    if (c0_ok && y < H) store2((int64_t)zo * plane + (int64_t)y * W + x0 + tx, a);
+                for (int p = 0; p < P; ++p) {
+                    const int v = g * P + p;
+                    if (v >= 2 * R && v < nvirt && j < nrow) store2(op + (int64_t)p * plane + j * W, out[p]);
                 }
             }
+            op += P * plane;
         } else {
 #pragma unroll
-            for (int j = 0; j < kRY; ++j) {
-                const int y = y0 + ry0 + j;
-                if (c0_ok && y < H) store2((int64_t)y * W + x0 + tx, yv[j]);
-            }
+            for (int j = 0; j < kRY; ++j)
+                if (j < nrow) store2(op + j * W, yv[0][j]);
+        }
+        if constexpr (Z) __syncthreads();
+        if constexpr (TMA) {
+            // group g + 1's stage is consumed: group g + 3 into it
+            if (tid == 0 && issued < ngroups && *(volatile int *)&s_fail == 0) issue(issued++);
         }
     }
     if constexpr (TMA) {
-        if (failed_at >= 0) {
-            // the copies still in flight (planes failed_at .. issued-1) land
-            // before the CTA's shared memory is released
+        // (the barrier above ordered every s_fail write)
+        if (*(volatile int *)&s_fail != 0) {
+            // the copies still in flight land before the CTA's shared memory is
+            // released: the last group of each stage
             if (tid == 0) {
-                const int issued = min(nvirt, failed_at + kStages);
-                for (int p = failed_at; p < issued; ++p) mbar_wait(&bars[p % kStages], (uint32_t)(p / kStages) & 1u);
+                for (int q = max(0, issued - 2); q < issued; ++q) mbar_wait(&bars[q & 1], (uint32_t)(q >> 1) & 1u);
                 atomicCAS(status, 0, (int)CLE_ERR_ITER_LIMIT);
             }
             return;
@@ -391,6 +505,7 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
     }
     if (mm) {
         __shared__ float s_mn[kWarps], s_mx[kWarps];
+        const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
@@ -407,11 +522,13 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
     }
 }
 
-// Upper bound on the z chunks of the fused launch: four waves of two CTAs per
-// SM (the most a tile count could use), at most one chunk per plane.
+// Upper bound on the z chunks of the fused launch: four waves of four CTAs per
+// SM (above what any radius has resident; the most a tile count could use), at most one chunk per plane.
 int64_t fused_chunk_cap(int64_t tiles, int64_t D, int sms) {
-    return std::max<int64_t>(1, std::min<int64_t>(D, (8 * (int64_t)sms + tiles - 1) / tiles));
+    return std::max<int64_t>(1, std::min<int64_t>(D, (16 * (int64_t)sms + tiles - 1) / tiles));
 }
+
+int resident_ctas(int R) { return R <= 4 ? min_ctas<4>() : min_ctas<8>(); }
 
 // Grid of the fused launch: (x tiles, y tiles, z chunks).  A CTA's time is
 // about its planes (chunk + 2R halo), and CTAs run in waves of the resident
@@ -427,7 +544,7 @@ dim3 fused_grid(const Img &src, int R, int &zchunk) {
         int dev = 0;
         cudaGetDevice(&dev);
         const int sms = num_sms(dev);
-        const int64_t slots = (int64_t)sms * (R <= 8 ? 2 : 1);
+        const int64_t slots = (int64_t)sms * resident_ctas(R);
         const int64_t tiles = (int64_t)gx * gy;
         const int64_t cap = fused_chunk_cap(tiles, src.D, sms);
         int64_t best = -1;
@@ -447,7 +564,7 @@ dim3 fused_grid(const Img &src, int R, int &zchunk) {
 }
 
 // The source as a 3D tiled tensor map (x = W innermost) with the box of
-// TmaGeom<Tin, R>; false when the layout does not allow one (row pitch or base
+// Geom<Tin, R, true>; false when the layout does not allow one (row pitch or base
 // address not a multiple of 16 bytes) or the driver lacks the encoder.
 // The driver's tensor-map encoder, looked up once outside any stream capture
 // (an immutable function pointer; until then, and if the driver lacks it,
@@ -475,14 +592,14 @@ void *tensor_map_encoder(cudaStream_t st) {
 
 template <typename Tin, int R>
 bool encode_source_map(const Img &src, CUtensorMap &map, cudaStream_t st) {
-    using TG = TmaGeom<Tin, R>;
+    using TG = Geom<Tin, R, true>;
     const uint64_t pitch = (uint64_t)src.W * sizeof(Tin);
     if (pitch % 16 != 0 || (reinterpret_cast<uintptr_t>(src.data) & 15) != 0) return false;
     void *const fn = tensor_map_encoder(st);
     if (fn == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)src.W, (cuuint64_t)src.H, (cuuint64_t)src.D};
     const cuuint64_t strides[2] = {(cuuint64_t)pitch, (cuuint64_t)(pitch * (uint64_t)src.H)};
-    const cuuint32_t box[3] = {(cuuint32_t)TG::BX, (cuuint32_t)TG::BY, 1u};
+    const cuuint32_t box[3] = {(cuuint32_t)TG::BX, (cuuint32_t)TG::ROWS, 1u};
     const cuuint32_t estride[3] = {1u, 1u, 1u};
     const CUtensorMapDataType dt = sizeof(Tin) == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                  : sizeof(Tin) == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16
@@ -495,29 +612,21 @@ bool encode_source_map(const Img &src, CUtensorMap &map, cudaStream_t st) {
 
 template <typename Tin, int R, bool Z>
 int launch_fused_r(const Img &src, float *dst, const Taps &t, float *mm, int *status, cudaStream_t st) {
-    using G = Geom<R>;
-    static_assert(min_ctas<R>() == (R <= 8 ? 2 : 1), "fused_grid's occupancy rule");
+    using G = Geom<Tin, R, Z>;
     int zchunk = 1;
     const dim3 grid = fused_grid(src, R, zchunk);
     if (grid.y > 65535 || grid.z > 65535) { set_error("gaussian_blur: image too large for the fused path"); return CLE_ERR_TOO_LARGE; }
+    HalfTaps<R> pt;
+    for (int i = 0; i <= R; ++i) pt.w[i] = t.w[i];
     alignas(64) CUtensorMap map;
     std::memset(&map, 0, sizeof(map));
     if constexpr (Z) {
-        // TMA staging once the grid fills two waves of resident CTAs: with
-        // fewer CTAs (one wave, one or two per SM) the register-staged path
-        // measured faster (128 x 512 x 512 at R = 8: 0.265 vs 0.305 ms;
-        // 512 x 1024 x 1024: 3.19 vs 3.12 ms the other way)
-        int dev = 0;
-        cudaGetDevice(&dev);
-        const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
-        const bool waves2 = ctas >= 2 * (int64_t)num_sms(dev) * min_ctas<R>();
-        if (status != nullptr && waves2 && encode_source_map<Tin, R>(src, map, st)) {
+        if (status != nullptr && encode_source_map<Tin, R>(src, map, st)) {
             auto kern = blur_fused_kernel<Tin, R, true, true>;
-            const size_t smem = TmaGeom<Tin, R>::SMEM;
             // set on every call: the attribute belongs to the current device's context
-            CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            kern<<<grid, kThreads, smem, st>>>((const Tin *)src.data, map, dst, (int)src.D, (int)src.H,
-                                               (int)src.W, zchunk, t, mm, status);
+            CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
+            kern<<<grid, kThreads, G::SMEM, st>>>((const Tin *)src.data, map, dst, (int)src.D, (int)src.H,
+                                                        (int)src.W, zchunk, pt, mm, status);
             CLE_LAUNCH_CHECK("gaussian_blur fused (TMA)");
             return CLE_OK;
         }
@@ -525,7 +634,7 @@ int launch_fused_r(const Img &src, float *dst, const Taps &t, float *mm, int *st
     auto kern = blur_fused_kernel<Tin, R, Z, false>;
     CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
     kern<<<grid, kThreads, G::SMEM, st>>>((const Tin *)src.data, map, dst, (int)src.D, (int)src.H, (int)src.W,
-                                          zchunk, t, mm, status);
+                                                zchunk, pt, mm, status);
     CLE_LAUNCH_CHECK("gaussian_blur fused");
     return CLE_OK;
 }

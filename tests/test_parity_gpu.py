@@ -82,6 +82,22 @@ def test_gaussian_blur_tma_staging_bit_exact(cle, oracle, dtype, shape, sigma):
     assert np.array_equal(dst.cpu().numpy(), oracle.gaussian_blur(a.astype(np.float32), sigma, sigma, sigma))
 
 
+# TMA staging works in groups of planes: fewer planes than a group, a last group
+# that is not full, images smaller than a tile (every edge clamped), rows of one
+# 16-byte granule, and every way the rounded-down box origin can lie (bit exact:
+# the same chain of fused multiply-adds)
+@pytest.mark.parametrize("dtype,width", [(np.uint8, 16), (np.uint8, 80), (np.uint16, 8), (np.uint16, 72),
+                                         (np.float32, 4), (np.float32, 100)])
+@pytest.mark.parametrize("depth,height", [(1, 1), (2, 33), (5, 31), (19, 70)])
+@pytest.mark.parametrize("sigma", [0.3, 1.0, 1.3, 2.0, 2.3, 3.5])
+def test_gaussian_blur_tma_small_bit_exact(cle, oracle, dtype, width, depth, height, sigma):
+    r = rng(31)
+    a = (r.integers(0, np.iinfo(dtype).max, size=(depth, height, width)) if dtype != np.float32
+         else r.uniform(-5000, 5000, size=(depth, height, width))).astype(dtype)
+    got = cle.pull(cle.gaussian_blur(a, None, sigma, sigma, sigma))
+    assert np.array_equal(got, oracle.gaussian_blur(a.astype(np.float32), sigma, sigma, sigma))
+
+
 # three passes: tile widths and heights with remainders (8 outputs per thread,
 # 128 / 64 / 32 outputs per CTA along y and z by the axis length and the window),
 # odd row counts, every remainder of taps modulo 8, windows longer than the axis,
