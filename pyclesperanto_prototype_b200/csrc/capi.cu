@@ -419,7 +419,7 @@ int cle_masked_voronoi_labeling(const cle_tensor *bin, const cle_tensor *msk, co
 size_t cle_connected_components_labeling_diamond_workspace_bytes(const cle_tensor *bin) {
     Img im;
     if (to_img(bin, im, "binary_input")) return 0;
-    return ccl_workspace_bytes(im);
+    return ccl_workspace_bytes(im, true);
 }
 
 int cle_connected_components_labeling_diamond(const cle_tensor *bin, const cle_tensor *dst, void *ws,
@@ -429,7 +429,7 @@ int cle_connected_components_labeling_diamond(const cle_tensor *bin, const cle_t
     CLE_TRY(to_img(dst, d, "labeling_destination"));
     CLE_TRY(same_shape(a, d, "binary_input", "labeling_destination"));
     if (d.dtype != CLE_U32 && d.dtype != CLE_F32) { set_error("connected_components_labeling_diamond: destination must be uint32 or float32"); return CLE_ERR_DTYPE; }
-    CLE_TRY(ws_check(ws, ws_bytes, ccl_workspace_bytes(a), "connected_components_labeling_diamond"));
+    CLE_TRY(ws_check(ws, ws_bytes, ccl_workspace_bytes(a, true), "connected_components_labeling_diamond"));
     CLE_TRY(set_device_of(a, bin));
     Arena ar(ws, ws_bytes);
     uint32_t *lab = ar.take<uint32_t>(a.n());

@@ -83,7 +83,7 @@ int maxima_seeds(const Img &T, const float *d_thr32, uint8_t *seg, uint32_t *lab
                  uint32_t *d_count, cudaStream_t st);
 
 // ccl.cu
-size_t ccl_workspace_bytes(const Img &im);
+size_t ccl_workspace_bytes(const Img &im, bool diamond = false);
 // Dense CCL of (binary != 0) into u32 labels (x-major float32 key ranks).
 // diamond: face connectivity (4 in 2D, 6 in 3D) instead of the 3^d box
 int ccl_dense(const Img &binary, uint32_t *labels, Arena &ws, cudaStream_t st, bool diamond = false);

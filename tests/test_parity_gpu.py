@@ -251,6 +251,39 @@ def test_ccl_exact(cle, oracle, shape, density):
     assert np.array_equal(got, oracle.connected_components_labeling_box(b))
 
 
+# tiles of 32 x 16 x 8 voxels (32 x 64 in images): one tile, exact tiles, one voxel
+# more in each direction; masks whose components cross many tiles, touch only
+# diagonally across tile faces, edges and corners, or fill a tile to its most
+# components
+CCL_TILE_SHAPES = [(1, 1), (64, 32), (65, 33), (129, 97), (1, 70, 40), (8, 16, 32), (9, 17, 33), (17, 40, 65), (16, 33, 64)]
+
+
+def _ccl_masks(shape):
+    r = rng(41)
+    idx = np.indices(shape)
+    yield "sparse", r.uniform(size=shape) < 0.03
+    yield "percolating", r.uniform(size=shape) < (0.4 if len(shape) == 2 else 0.15)
+    yield "dense", r.uniform(size=shape) < 0.9
+    yield "full", np.ones(shape, bool)
+    yield "checkerboard", idx.sum(0) % 2 == 0              # diagonal contacts only
+    yield "isolated", np.all(idx % 2 == 0, axis=0)         # the most components with the box
+    yield "lines", (idx[-1] + 2 * idx[-2]) % 5 == 0
+    snake = (idx[-2] % 2 == 0)
+    snake |= (idx[-2] % 4 == 1) & (idx[-1] == shape[-1] - 1) | (idx[-2] % 4 == 3) & (idx[-1] == 0)
+    yield "snake", snake if len(shape) == 2 else snake & (idx[0] % 2 == 0) | (idx[0] % 2 == 1) & (idx[1] == 0) & (idx[2] == 0)
+
+
+@pytest.mark.parametrize("shape", CCL_TILE_SHAPES)
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32])
+def test_ccl_tiles_exact(cle, oracle, shape, dtype):
+    for name, m in _ccl_masks(shape):
+        b = m.astype(dtype)
+        got = cle.pull(cle.connected_components_labeling_box(b))
+        assert np.array_equal(got, oracle.connected_components_labeling_box(b)), name
+        got = cle.pull(cle.connected_components_labeling_diamond(b))
+        assert np.array_equal(got, oracle.connected_components_labeling_diamond(b)), name
+
+
 def test_ccl_reference_test(cle):
     a = np.array([[[1, 0, 1], [1, 0, 0], [0, 0, 1]]])
     assert np.array_equal(cle.pull(cle.connected_components_labeling_box(a)),
