@@ -415,18 +415,48 @@ __global__ void mask_kernel(const Ts *__restrict__ s, const Tm *__restrict__ m, 
 }
 
 template <typename T>
-__global__ void label_max_partial(const T *__restrict__ s, int64_t n, uint32_t *__restrict__ out) {
+__device__ __forceinline__ uint32_t label_of(T v) {
+    if constexpr (std::is_floating_point<T>::value) return v > (T)0 ? (uint32_t)(int64_t)v : 0u;
+    else return (uint32_t)v;
+}
+
+// Largest label: four 128-bit loads per thread in flight (4-byte labels on a
+// 16-byte boundary), one atomic per CTA.  512 x 1024 x 1024 uint32: 0.54 ms with
+// scalar loads and an atomic per warp.
+constexpr int kMaxThreads = 512;
+template <typename T>
+__global__ void __launch_bounds__(kMaxThreads)
+label_max_partial(const T *__restrict__ s, int64_t n, uint32_t *__restrict__ out) {
     uint32_t m = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t v;
-        if constexpr (std::is_floating_point<T>::value) v = s[i] > (T)0 ? (uint32_t)(int64_t)s[i] : 0u;
-        else v = (uint32_t)s[i];
-        m = max(m, v);
-    }
+    const int64_t stride = (int64_t)gridDim.x * kMaxThreads, i0 = blockIdx.x * (int64_t)kMaxThreads + threadIdx.x;
+    int64_t done = 0;
+    if constexpr (sizeof(T) == 4) {
+        if ((reinterpret_cast<uintptr_t>(s) & 15) == 0) {
+            const int64_t n4 = n / 4;
+            const uint4 *s4 = reinterpret_cast<const uint4 *>(s);
+            for (int64_t j = i0; j < n4; j += 4 * stride) {
+                uint4 u[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+                for (int k = 0; k < 4; ++k) u[k] = j + k * stride < n4 ? __ldcs(s4 + j + k * stride) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    T v[4];
+                    memcpy(v, &u[k], 16);
+                    m = max(max(m, max(label_of(v[0]), label_of(v[1]))), max(label_of(v[2]), label_of(v[3])));
+                }
+            }
+            done = n4 * 4;
+        }
+    }
+    for (int64_t i = done + i0; i < n; i += stride) m = max(m, label_of(s[i]));
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ uint32_t s_m[kMaxThreads / 32];
+    if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = __reduce_max_sync(0xffffffffu, threadIdx.x < kMaxThreads / 32 ? s_m[threadIdx.x] : 0u);
+        if (threadIdx.x == 0 && m) atomicMax(out, m);
+    }
 }
 
 }  // namespace
@@ -614,12 +644,12 @@ size_t label_max_workspace_bytes(const Img &) { return 0; }
 int label_max(const Img &labels, uint32_t *d_max, Arena &, cudaStream_t st) {
     CLE_CUDA(cudaMemsetAsync(d_max, 0, sizeof(uint32_t), st));
     const int64_t n = labels.n();
-    const int blocks = launch_blocks(n, 256, 4);
+    const int blocks = launch_blocks(n / 4 + 1, kMaxThreads, 4);
     switch (labels.dtype) {
-        case CLE_U32: label_max_partial<uint32_t><<<blocks, 256, 0, st>>>((const uint32_t *)labels.data, n, d_max); break;
-        case CLE_F32: label_max_partial<float><<<blocks, 256, 0, st>>>((const float *)labels.data, n, d_max); break;
-        case CLE_U16: label_max_partial<uint16_t><<<blocks, 256, 0, st>>>((const uint16_t *)labels.data, n, d_max); break;
-        case CLE_U8: label_max_partial<uint8_t><<<blocks, 256, 0, st>>>((const uint8_t *)labels.data, n, d_max); break;
+        case CLE_U32: label_max_partial<uint32_t><<<blocks, kMaxThreads, 0, st>>>((const uint32_t *)labels.data, n, d_max); break;
+        case CLE_F32: label_max_partial<float><<<blocks, kMaxThreads, 0, st>>>((const float *)labels.data, n, d_max); break;
+        case CLE_U16: label_max_partial<uint16_t><<<blocks, kMaxThreads, 0, st>>>((const uint16_t *)labels.data, n, d_max); break;
+        case CLE_U8: label_max_partial<uint8_t><<<blocks, kMaxThreads, 0, st>>>((const uint8_t *)labels.data, n, d_max); break;
         default: set_error("label_maximum: unsupported dtype %d", labels.dtype); return CLE_ERR_DTYPE;
     }
     CLE_LAUNCH_CHECK("label_maximum");

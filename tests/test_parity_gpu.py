@@ -475,6 +475,54 @@ def test_statistics_row_segments(cle, oracle, shape, pattern, on_device):
                   oracle.statistics_of_labelled_pixels(inten.astype(np.float32), lab))
 
 
+# bricks of 32 x 8 x 4 voxels (32 x 32 in images): one voxel, exact bricks, one voxel
+# more in each direction, images thinner than a brick (fewer labels kept of each);
+# a label that fills many bricks, more labels in a brick than are kept, stripes
+# along each axis, absent labels
+def _stat_labels(shape):
+    r = rng(51)
+    idx = np.indices(shape)
+    yield "one", np.ones(shape)
+    yield "own", np.arange(1, np.prod(shape) + 1).reshape(shape)           # every voxel its own
+    yield "few", r.integers(0, 4, size=shape) * 3                          # labels 3, 6, 9
+    yield "many", r.integers(0, 200, size=shape)
+    yield "x", idx[-1] // 3
+    yield "y", idx[-2] + 1
+    yield "first", idx[0] // 2
+    yield "background", np.where(r.uniform(size=shape) < 0.02, r.integers(2, 30, size=shape), 1)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (32, 32), (33, 65), (70, 3), (8, 16, 64), (9, 33, 65), (4, 8, 32), (2, 50, 1),
+                                   (37, 2, 5)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_statistics_bricks(cle, oracle, shape, dtype):
+    r = rng(52)
+    inten = (r.integers(0, np.iinfo(dtype).max, size=shape) if dtype != np.float32
+             else r.uniform(-100, 5000, size=shape)).astype(dtype)
+    for name, lab in _stat_labels(shape):
+        lab = lab.astype(np.uint32)
+        if lab.max() == 0:
+            continue
+        ref = oracle.statistics_of_labelled_pixels(inten.astype(np.float32), lab)
+        src = cle.push_native(inten)
+        import torch
+        dev = cle.B200Array(torch.from_numpy(lab.astype(np.int32)).cuda().view(torch.uint32))
+        _assert_stats(cle.statistics_of_labelled_pixels(src, dev), ref)
+        _assert_stats(cle.statistics_of_labelled_pixels(src, lab), ref)     # float32 labels
+
+
+def test_statistics_infinite_intensity_stays_in_its_label(cle):
+    lab = np.zeros((6, 40, 70), np.uint32)
+    lab[1:5, 2:20, 1:30] = 1
+    lab[1:5, 20:38, 31:69] = 2
+    inten = np.ones(lab.shape, np.float32)
+    inten[2, 5, 7] = np.inf
+    s = cle.statistics_of_labelled_pixels(inten, lab)
+    for k in ("sum_intensity", "sum_intensity_times_x", "sum_intensity_times_y", "sum_intensity_times_z", "max_intensity"):
+        assert s[k][0] == np.inf and np.isfinite(s[k][1]), k
+    assert s["mean_intensity"][1] == 1 and s["min_intensity"][0] == 1
+
+
 def test_statistics_reference_tables(cle, oracle):
     inten = np.array([[0, 1, 2], [1, 2, 3], [2, 3, 4]])
     lab = np.array([[1, 1, 2], [1, 2, 2], [3, 3, 3]])
