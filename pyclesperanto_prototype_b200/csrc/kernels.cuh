@@ -113,12 +113,14 @@ int voronoi_frontier(const Img &shape, uint32_t *labels, const uint8_t *seg,
 // largest seed label on the device) and up to 120 steps; otherwise the labels
 // are left as given and the frontier kernel above grows them.  seg: mask
 // bytes as the seed passes write them (kMaskByte); the growth keeps each
-// labelled voxel's arrival step in them.  Workspace includes the frontier
-// kernel's.
+// labelled voxel's arrival step in them.  segments: the mask is the whole
+// image, the list holds one labelled voxel per 8-voxel row segment and the
+// mask bytes of labelled voxels are 0x80 already.  Workspace includes the
+// frontier kernel's.
 size_t voronoi_grow_workspace_bytes(const Img &im);
 int voronoi_grow(const Img &shape, uint32_t *labels, uint8_t *seg, const uint32_t *seeds,
                  const uint32_t *d_seed_count, const uint32_t *d_max_label, int *d_status, Arena &ws,
-                 cudaStream_t st, const Limits &lim);
+                 cudaStream_t st, const Limits &lim, int segments = 0);
 size_t voronoi_dense_workspace_bytes(const Img &im);
 int masked_voronoi_dense(const Img &binary, const Img &mask, const Img &dst, int *d_status,
                          Arena &ws, cudaStream_t st, const Limits &lim);

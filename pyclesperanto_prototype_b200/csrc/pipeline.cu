@@ -199,8 +199,10 @@ int masked_voronoi_binary(const Img &bin, const Img &mask, const Img &dst, Arena
 // ---- extend_labeling_via_voronoi / voronoi_labeling -------------------------
 // _tier4/_extend_labeling_via_voronoi.py:13-60: the labels (uint32, any values)
 // grow into every zero voxel with the onlyzero_overwrite_maximum box/diamond
-// Jacobi steps until a step changes nothing -- the brick growth kernel with a
-// mask that covers the whole image.  voronoi_labeling (_tier5/_voronoi_labeling.py:
+// Jacobi steps until a step changes nothing -- the key growth with a mask that
+// covers the whole image (labels above 2^24 - 1 and paths above its step range
+// take the brick growth behind it).  1024 x 1024 with a spot per 33 x 33 pixels:
+// 0.80 ms with the brick growth (two grid barriers a step), 0.27 now.  voronoi_labeling (_tier5/_voronoi_labeling.py:
 // 8-40) is connected_components_labeling_box followed by that growth.
 namespace {
 
@@ -225,10 +227,11 @@ constexpr int kSeedWarps = 8;
 // One seed voxel per 8-voxel row segment (x aligned to 8) that holds a label;
 // the segment lies in one growth brick (8 x by 4 y), so the 3x3x3 brick
 // neighbourhood of the seed's brick covers every voxel next to a label of the
-// segment.  A warp reads 32 x of one row.  One global atomic per CTA.
+// segment.  A warp reads 32 x of one row.  One global atomic per CTA.  Also
+// the mask bytes: arrival step 0 on labels, not yet known elsewhere.
 __global__ void __launch_bounds__(kSeedWarps * 32)
-brick_seeds_kernel(const uint32_t *__restrict__ lab, uint32_t W, uint32_t WB, FastDiv fWB, uint32_t nb,
-                   uint32_t *__restrict__ seeds, uint32_t *__restrict__ d_count) {
+brick_seeds_kernel(const uint32_t *__restrict__ lab, uint8_t *__restrict__ seg, uint32_t W, uint32_t WB, FastDiv fWB,
+                   uint32_t nb, uint32_t *__restrict__ seeds, uint32_t *__restrict__ d_count) {
     __shared__ uint32_t s_n, s_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t base = blockIdx.x * kSeedWarps; base < nb; base += gridDim.x * kSeedWarps) {
@@ -239,7 +242,9 @@ brick_seeds_kernel(const uint32_t *__restrict__ lab, uint32_t W, uint32_t WB, Fa
         bool has = false;
         if (b < nb) {
             const uint32_t r = fWB.div(b), xb = b - r * WB, x = xb * 32u + (uint32_t)lane;
-            const unsigned bal = __ballot_sync(0xffffffffu, x < W && lab[r * W + x] != 0u);
+            const bool on = x < W && lab[r * W + x] != 0u;
+            if (x < W) seg[r * W + x] = on ? (uint8_t)0x80 : kMaskByte;
+            const unsigned bal = __ballot_sync(0xffffffffu, on);
             const unsigned seg8 = (bal >> (lane & 24)) & 0xFFu;   // this lane's 8-voxel segment
             has = (lane & 7) == 0 && seg8 != 0u;
             if (has) {
@@ -273,13 +278,16 @@ ExtLayout take_ext_layout(Arena &a, const Img &im) {
 // Grows `lab` in place over the whole image; status in l.sc.
 int grow_everywhere(const Img &im, uint32_t *lab, ExtLayout &l, Arena &tail, cudaStream_t st,
                     const Limits &lim) {
-    CLE_CUDA(cudaMemsetAsync(l.seg, 1, (size_t)im.n(), st));
     const uint32_t WB = (uint32_t)((im.W + 31) / 32);
     const uint32_t nb = (uint32_t)(im.D * im.H) * WB;
     brick_seeds_kernel<<<launch_blocks((int64_t)nb * 32, kSeedWarps * 32), kSeedWarps * 32, 0, st>>>(
-        lab, (uint32_t)im.W, WB, FastDiv(WB), nb, l.seeds, &l.sc->seed_count);
+        lab, l.seg, (uint32_t)im.W, WB, FastDiv(WB), nb, l.seeds, &l.sc->seed_count);
     CLE_LAUNCH_CHECK("brick seeds");
-    return voronoi_frontier(im, lab, l.seg, l.seeds, &l.sc->seed_count, &l.sc->status, tail, st, lim);
+    Img L = im;
+    L.data = lab;
+    L.dtype = CLE_U32;
+    CLE_TRY(label_max(L, &l.sc->nlabels, tail, st));
+    return voronoi_grow(im, lab, l.seg, l.seeds, &l.sc->seed_count, &l.sc->nlabels, &l.sc->status, tail, st, lim, 1);
 }
 
 }  // namespace
@@ -287,7 +295,7 @@ int grow_everywhere(const Img &im, uint32_t *lab, ExtLayout &l, Arena &tail, cud
 size_t extend_voronoi_workspace_bytes(const Img &im) {
     Arena a(nullptr, 0);
     take_ext_layout(a, im);
-    const size_t tail = std::max(ccl_workspace_bytes(im), voronoi_frontier_workspace_bytes(im));
+    const size_t tail = std::max(ccl_workspace_bytes(im), voronoi_grow_workspace_bytes(im));
     return a.off + tail;
 }
 

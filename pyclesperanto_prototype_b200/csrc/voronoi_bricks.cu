@@ -579,7 +579,7 @@ voronoi_keys_kernel(uint32_t *lab, uint8_t *seg, BGeo G, const uint32_t *seeds,
                     const uint32_t *d_seed_count, const uint32_t *d_max_label, uint32_t *B0, uint32_t *B1,
                     uint32_t *bstep, KState *S, int *d_status, uint32_t max_steps,
                     uint64_t loop_ns, uint64_t barrier_ns, const volatile int *cancel,
-                    unsigned long long *trace, BQueue Qb, int use_bitmap) {
+                    unsigned long long *trace, BQueue Qb, int use_bitmap, int segments) {
     constexpr int NW = KBT / 32;
     constexpr int ZR = IS3D ? 1 : 0;
     constexpr int K = BZ + 2 * ZR;
@@ -592,8 +592,12 @@ voronoi_keys_kernel(uint32_t *lab, uint8_t *seg, BGeo G, const uint32_t *seeds,
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
     WarpAppender ap{&S->err, 0u};
     const uint64_t t_entry = global_ns();
-    // labels that do not fit 24 bits: the brick kernel takes over (uniform)
-    if (__ldcg(d_max_label) > 0x00FFFFFFu) {
+    // labels that do not fit 24 bits, or a whole image (segments) in which
+    // kKeyMaxS steps from every seed segment cannot reach all voxels: the brick
+    // kernel takes over (uniform)
+    const uint32_t ns = __ldcg(d_seed_count);
+    const uint64_t reach = (uint64_t)ns * (2u * kKeyMaxS + 8u) * (2u * kKeyMaxS + 1u) * (IS3D ? 2u * kKeyMaxS + 1u : 1u);
+    if (__ldcg(d_max_label) > 0x00FFFFFFu || (segments && reach < (uint64_t)g.D * g.H * g.W)) {
         if (gtid == 0) S->gate = 1;
         return;
     }
@@ -601,18 +605,19 @@ voronoi_keys_kernel(uint32_t *lab, uint8_t *seg, BGeo G, const uint32_t *seeds,
 
     // round 0: each seed's brick and the neighbouring bricks the seed touches
     // (a seed on a brick's face, edge or corner); the growth reaches every
-    // other brick through a changed voxel next to it
-    const uint32_t ns = __ldcg(d_seed_count);
+    // other brick through a changed voxel next to it.  With `segments` a listed
+    // voxel stands for the labelled voxels of its 8-voxel row segment (the
+    // brick's width), whose mask bytes are set already.
     for (uint32_t base = blockIdx.x * NW; base < ns; base += gridDim.x * NW) {
         const uint32_t i = base + warp;
         if (i < ns) {
             const uint32_t m = __ldcg(seeds + i);
-            if (lane == 0) seg[m] = 0x80u;   // in the mask, arrival step 0
+            if (lane == 0 && !segments) seg[m] = 0x80u;   // in the mask, arrival step 0
             uint32_t x, y, z;
             m2xyz(g, m, x, y, z);
             const int dz = lane / 9 - 1, dyb = (lane / 3) % 3 - 1, dxb = lane % 3 - 1;
             const uint32_t xr = x % kBX, yr = y % kBY, zr = z % BZ;
-            const bool touch = (dxb == 0 || (dxb < 0 ? xr == 0 : xr == kBX - 1)) &&
+            const bool touch = (segments || dxb == 0 || (dxb < 0 ? xr == 0 : xr == kBX - 1)) &&
                                (dyb == 0 || (dyb < 0 ? yr == 0 : yr == kBY - 1)) &&
                                (dz == 0 || (dz < 0 ? zr == 0 : zr == (uint32_t)BZ - 1));
             const bool want = lane < 27 && (IS3D || dz == 0) && touch;
@@ -1081,7 +1086,7 @@ size_t voronoi_grow_workspace_bytes(const Img &im) {
 
 int voronoi_grow(const Img &im, uint32_t *lab, uint8_t *seg, const uint32_t *seeds,
                  const uint32_t *d_seed_count, const uint32_t *d_max_label, int *d_status, Arena &ws,
-                 cudaStream_t st, const Limits &lim) {
+                 cudaStream_t st, const Limits &lim, int segments) {
     // the key kernel's state sits behind the brick kernel's workspace, so the
     // gate word survives that kernel's set-up
     const size_t off0 = ws.off;
@@ -1128,7 +1133,7 @@ int voronoi_grow(const Img &im, uint32_t *lab, uint8_t *seg, const uint32_t *see
     int use_bitmap = im.n() > kWideVoxels ? 1 : 0;
     void *args[] = {&lab, (void *)&seg, &G, (void *)&seeds, (void *)&d_seed_count, (void *)&d_max_label,
                     &B0, &B1, &bstep, &S, &d_status, &max_steps, &loop_ns, &barrier_ns,
-                    (void *)&cancel, &trace, &Qb, &use_bitmap};
+                    (void *)&cancel, &trace, &Qb, &use_bitmap, &segments};
     CLE_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kKeyBT), args, smem, st));
     count_launches(1);
     // the brick kernel, which returns at once unless the gate was raised

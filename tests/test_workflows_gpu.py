@@ -172,6 +172,28 @@ def test_extend_labeling_via_voronoi_any_label_values(cle, oracle, shape):
     assert np.array_equal(got, oracle.extend_labeling_via_voronoi(lab))
 
 
+# whole-image growth: one label in a corner or the middle whose farthest voxel
+# lies below, at and above the key growth's 120 steps, the largest labels it takes
+# and the first it does not, labels that fill whole row segments, none at all
+@pytest.mark.parametrize("shape", [(1, 119), (3, 121), (5, 125), (118, 122), (130, 300), (6, 40, 121), (30, 9, 260)])
+@pytest.mark.parametrize("where", ["corner", "middle", "rows", "none"])
+@pytest.mark.parametrize("top", [7, 2 ** 24 - 1, 2 ** 24])
+def test_extend_labeling_via_voronoi_key_range(cle, oracle, shape, where, top):
+    import torch
+    lab = np.zeros(shape, np.uint32)
+    if where == "corner":
+        lab[(0,) * len(shape)] = top
+    elif where == "middle":
+        lab[tuple(s // 2 for s in shape)] = top
+        lab[(-1,) * len(shape)] = 3
+    elif where == "rows":
+        lab[..., shape[-1] // 3:shape[-1] // 3 + 40] = np.arange(shape[-2], dtype=np.uint32)[:, None] % 5 + 1
+        lab[..., 0, 0] = top
+    src = cle.B200Array(torch.from_numpy(lab.astype(np.int64).astype(np.int32)).cuda().view(torch.uint32))
+    got = cle.pull(cle.extend_labeling_via_voronoi(src, cle.create_labels_like(src)))
+    assert np.array_equal(got, oracle.extend_labeling_via_voronoi(lab))
+
+
 # ---------------------------------- minimum / maximum box, top-hat -------
 def test_box_reference_tests(cle):
     # tests/test_minimum_box.py, test_maximum_box.py, test_top_hat_box.py of the reference
