@@ -198,7 +198,7 @@ blur_row_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t ro
 template <typename Tin, int NG>
 __global__ void __launch_bounds__(kSepThreads)
 blur_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t inner, int L, int vec,
-                const __grid_constant__ Taps taps, float *__restrict__ mm) {
+                const __grid_constant__ Taps taps, MinMaxState *__restrict__ mm) {
     constexpr int NC = kSepThreads / NG, COLS = 2 * NC, ROWS = NG * kK;
     extern __shared__ __align__(16) float2 sm[];
     const int n = taps.n, r = (n - 1) / 2;
@@ -285,9 +285,7 @@ blur_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t in
         __syncthreads();
         if (threadIdx.x == 0) {
             for (int w = 1; w < kSepThreads / 32; ++w) { vmin = fminf(vmin, s_mn[w]); vmax = fmaxf(vmax, s_mx[w]); }
-            const int64_t cta = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-            mm[2 * cta] = vmin;
-            mm[2 * cta + 1] = vmax;
+            add_minmax(mm, vmin, vmax, gridDim.x * gridDim.y * gridDim.z);
         }
     }
 }
@@ -304,17 +302,8 @@ __global__ void convert_kernel(const Tin *__restrict__ src, float *__restrict__ 
 // memory.
 int col_groups(int64_t L, int n) { return L <= 32 && n <= 129 ? 4 : L <= 64 && n <= 321 ? 8 : 16; }
 
-// CTAs of the last pass of an image (y in 2D, z in 3D) with n taps
-int64_t last_pass_ctas(const Img &im, int n) {
-    const bool vol = im.ndim == 3;
-    const int64_t L = vol ? im.D : im.H, inner = vol ? im.H * im.W : im.W;
-    const int ng = col_groups(L, n);
-    const int64_t cols = 2 * (kSepThreads / ng), rows = ng * kK;
-    return ((inner + cols - 1) / cols) * ((L + rows - 1) / rows);
-}
-
 template <typename Tin, int NG>
-int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, const Taps &t, float *mm,
+int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, const Taps &t, MinMaxState *mm,
                cudaStream_t st) {
     constexpr int COLS = 2 * (kSepThreads / NG), ROWS = NG * kK;
     const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((L + ROWS - 1) / ROWS), (unsigned)outer);
@@ -327,7 +316,7 @@ int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, 
 }
 
 template <typename Tin>
-int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps &t, float *mm,
+int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps &t, MinMaxState *mm,
                 cudaStream_t st) {
     if (axis == 2) {
         // the row split evenly into tiles of at most kRowMax outputs, row pairs
@@ -368,7 +357,7 @@ int launch_convert(const Tin *src, float *dst, int64_t n, cudaStream_t st) {
 }
 
 template <typename Tin>
-int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, float *t2, float *mm,
+int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, float *t2, MinMaxState *mm,
                     cudaStream_t st) {
     // pass order x (axis 2), y (axis 1), z (axis 0, 3D only)
     const int passes = (src.ndim == 3) ? 3 : 2;
@@ -404,7 +393,7 @@ size_t separable_workspace_bytes(const Img &im) {
 }
 
 int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty, const Taps *tz,
-                     Arena &ws, cudaStream_t st, float *mm) {
+                     Arena &ws, cudaStream_t st, MinMaxState *mm) {
     float *t1 = ws.take<float>(src.n());
     float *t2 = ws.take<float>(src.n());
     if (!ws.ok()) {
@@ -434,21 +423,10 @@ int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, A
     return separable_filter(src, dst, px, py, pz, ws, st);
 }
 
-int separable_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st) {
+int separable_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st) {
     Taps t;
     CLE_TRY(make_gauss_taps(sigma, t));
-    const int64_t ctas = last_pass_ctas(src, t.n);
-    float *partial = ws.take<float>(2 * (size_t)ctas);
-    if (!ws.ok()) { set_error("gaussian_blur: workspace too small"); return CLE_ERR_WORKSPACE; }
-    CLE_TRY(separable_filter(src, dst, &t, &t, src.ndim == 3 ? &t : nullptr, ws, st, partial));
-    return minmax_finish(partial, (int)ctas, d_minmax, st);
-}
-
-size_t separable_minmax_workspace_bytes(const Img &src) {
-    // the most CTAs the last pass takes for any window
-    Arena a(nullptr, 0);
-    a.take<float>(2 * (size_t)std::max(last_pass_ctas(src, 1), last_pass_ctas(src, kMaxTaps)));
-    return a.off + separable_workspace_bytes(src);
+    return separable_filter(src, dst, &t, &t, src.ndim == 3 ? &t : nullptr, ws, st, mm);
 }
 
 }  // namespace cle

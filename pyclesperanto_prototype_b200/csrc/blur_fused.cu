@@ -44,9 +44,8 @@
 // on 61 x 479 x 347 0.251 against 0.152 ms, 64 x 256 x 256 0.106 / 0.062,
 // 128 x 512 x 512 0.370 / 0.283, 128 x 1024 x 1024 1.295 / 0.974; R = 8 on the last two
 // 0.179 / 0.238 and 0.517 / 0.866.  Given a
-// partial buffer, each CTA also reduces the exact min / max of the values it
-// stores (the global min / max of the result in a one-CTA finish), which
-// saves threshold_otsu's separate pass over the blurred image.
+// min / max state, each CTA also adds the exact min / max of the values it
+// stores and the last CTA writes the result's, which saves threshold_otsu's separate pass over the blurred image.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <atomic>
@@ -214,10 +213,10 @@ template <typename Tin, int R, bool Z, bool TMA>
 __global__ void __launch_bounds__(kThreads, (min_ctas<R>()))
 blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorMap tmap,
                   float *__restrict__ dst, int D, int H, int W, int zchunk,
-                  const __grid_constant__ HalfTaps<R> taps, float *__restrict__ mm, int *__restrict__ status) {
+                  const __grid_constant__ HalfTaps<R> taps, MinMaxState *__restrict__ mm, int *__restrict__ status) {
     static_assert(!TMA || Z, "TMA staging is for volumes");
     using G = Geom<Tin, R, Z>;
-    constexpr int WIN = 2 * R + 1, BX = G::BX, P = G::P;
+    constexpr int BX = G::BX, P = G::P;
     constexpr bool kRegStage = Z && !TMA;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     // raw stages [1 or 2][P][STAGE], x results [1 or 2][P][ROWS][kXS], offsets
@@ -515,9 +514,7 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
         __syncthreads();
         if (tid == 0) {
             for (int w = 1; w < kWarps; ++w) { vmin = fminf(vmin, s_mn[w]); vmax = fmaxf(vmax, s_mx[w]); }
-            const int64_t cta = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-            mm[2 * cta] = vmin;
-            mm[2 * cta + 1] = vmax;
+            add_minmax(mm, vmin, vmax, gridDim.x * gridDim.y * gridDim.z);
         }
     }
 }
@@ -611,7 +608,7 @@ bool encode_source_map(const Img &src, CUtensorMap &map, cudaStream_t st) {
 }
 
 template <typename Tin, int R, bool Z>
-int launch_fused_r(const Img &src, float *dst, const Taps &t, float *mm, int *status, cudaStream_t st) {
+int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, int *status, cudaStream_t st) {
     using G = Geom<Tin, R, Z>;
     int zchunk = 1;
     const dim3 grid = fused_grid(src, R, zchunk);
@@ -640,7 +637,7 @@ int launch_fused_r(const Img &src, float *dst, const Taps &t, float *mm, int *st
 }
 
 template <typename Tin, bool Z, int R = 1>
-int dispatch_r(const Img &src, float *dst, const Taps &t, int r, float *mm, int *status, cudaStream_t st) {
+int dispatch_r(const Img &src, float *dst, const Taps &t, int r, MinMaxState *mm, int *status, cudaStream_t st) {
     if constexpr (R > (Z ? kMaxFusedR3 : kMaxFusedR)) {
         set_error("internal: fused radius out of range");
         return CLE_ERR_ARG;
@@ -660,7 +657,7 @@ bool fused_blur_applies(const Img &src, double sx, double sy, double sz) {
     return r >= 1 && r <= (src.ndim == 3 ? kMaxFusedR3 : kMaxFusedR) && src.W < (1 << 30) && src.H < (1 << 30);
 }
 
-int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, float *mm, int *status) {
+int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, MinMaxState *mm, int *status) {
     Taps t;
     CLE_TRY(make_gauss_taps(sigma, t));
     const int r = (t.n - 1) / 2;
@@ -673,35 +670,14 @@ int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, float 
     }
 }
 
-size_t blur_minmax_workspace_bytes(const Img &src) {
-    // any sigma: the three-pass path with its min / max, or the fused partials
-    // (at most fused_chunk_cap z chunks per tile)
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int64_t tiles = ((src.W + kTX - 1) / kTX) * ((src.H + kTY - 1) / kTY);
-    const int64_t chunks = fused_chunk_cap(tiles, std::max<int64_t>(src.D, 1), num_sms(dev));
-    const size_t fused = sizeof(float) * 2 * (size_t)(tiles * chunks) + 256;
-    return std::max(fused, std::max(separable_minmax_workspace_bytes(src),
-                                    separable_workspace_bytes(src) + minmax_workspace_bytes(src)));
-}
-
-int blur_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st,
-                int *status) {
-    if (!fused_blur_applies(src, sigma, sigma, sigma)) {
-        if (sigma > 0) return separable_minmax(src, dst, sigma, d_minmax, ws, st);
-        CLE_TRY(gaussian_blur(src, dst, sigma, sigma, sigma, ws, st, status));
-        Img T = src;
-        T.data = dst;
-        T.dtype = CLE_F32;
-        return minmax(T, d_minmax, ws, st);
-    }
-    int zchunk = 1;
-    const dim3 g = fused_grid(src, (sigma_to_kernel_size(sigma) - 1) / 2, zchunk);
-    const int ctas = (int)(g.x * g.y * g.z);
-    float *partial = ws.take<float>(2 * (size_t)ctas);
-    if (!ws.ok()) { set_error("gaussian_blur: workspace too small"); return CLE_ERR_WORKSPACE; }
-    CLE_TRY(fused_blur(src, dst, sigma, st, partial, status));
-    return minmax_finish(partial, ctas, d_minmax, st);
+int blur_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st, int *status) {
+    if (fused_blur_applies(src, sigma, sigma, sigma)) return fused_blur(src, dst, sigma, st, mm, status);
+    if (sigma > 0) return separable_minmax(src, dst, sigma, mm, ws, st);
+    CLE_TRY(gaussian_blur(src, dst, sigma, sigma, sigma, ws, st, status));
+    Img T = src;
+    T.data = dst;
+    T.dtype = CLE_F32;
+    return minmax(T, mm->out, ws, st);
 }
 
 }  // namespace cle

@@ -136,8 +136,7 @@ int cle_threshold_otsu(const cle_tensor *src, const cle_tensor *dst, double *d_t
     float *hist = ar.take<float>(256);
     double *thr = ar.take<double>(4);
     CLE_TRY(minmax(a, mm, ar, S(stream)));
-    CLE_TRY(histogram(a, 256, mm, hist, ar, S(stream)));
-    CLE_TRY(otsu(hist, mm, d_thr ? d_thr : thr, mm + 2, S(stream)));
+    CLE_TRY(histogram_otsu(a, mm, hist, d_thr ? d_thr : thr, mm + 2, ar, S(stream)));
     return greater_constant(a, b, 0.0f, mm + 2, S(stream));
 }
 

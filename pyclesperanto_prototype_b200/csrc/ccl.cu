@@ -460,94 +460,159 @@ __global__ void ccl_label_list(uint32_t *__restrict__ lab, const uint32_t *__res
     }
 }
 
-__global__ void count_ranks_kernel(const uint32_t *__restrict__ bitmap,
-                                   const uint32_t *__restrict__ prefix, uint32_t words,
-                                   uint32_t *__restrict__ out) {
-    *out = prefix[words - 1] + __popc(bitmap[words - 1]);
+// The whole list labelling of a small image in one CTA: unions, roots, marks,
+// ranks and labels with block barriers between them, one launch instead of
+// eight and a clear (256 x 256: 10.9 us against 34 and the launch gaps).
+constexpr int kListCta = 1024;
+constexpr int64_t kListCtaVoxels = int64_t(1) << 17;
+
+__global__ void __launch_bounds__(kListCta)
+ccl_list_small(uint32_t *lab, Geo g, const uint32_t *__restrict__ list, const uint32_t *__restrict__ d_count,
+               uint32_t *bitmap, uint32_t *prefix, uint32_t words, uint32_t *__restrict__ d_nlabels) {
+    __shared__ uint32_t s_w[kListCta / 32];
+    const uint32_t cnt = *d_count;
+    const uint32_t t = threadIdx.x;
+    const int lane = t & 31, warp = t >> 5;
+    for (uint32_t w = t; w < words; w += kListCta) st_cg(bitmap + w, 0u);
+    for (uint32_t i = t; i < cnt; i += kListCta) {
+        uint32_t x, y, z;
+        m2xyz(g, list[i], x, y, z);
+        union_back(lab, g, x, y, z);
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < cnt; i += kListCta) {
+        const uint32_t m = list[i];
+        const uint32_t v = ld_cg(lab + m), r = find_root(lab, g, v - 1u) + 1u;
+        uint32_t x, y, z;
+        m2xyz(g, m, x, y, z);
+        if (r - 1u == xyz2k(g, x, y, z)) {   // a root
+            const uint32_t idx = fkey_index((float)r);
+            atomicOr(bitmap + (idx >> 5), 1u << (idx & 31));
+        }
+        if (r != v) st_cg(lab + m, r);
+    }
+    __syncthreads();
+    // bits before each word: every thread a stretch of words
+    const uint32_t per = (words + kListCta - 1) / kListCta;
+    const uint32_t w0 = min(words, t * per), w1 = min(words, w0 + per);
+    uint32_t c = 0;
+    for (uint32_t w = w0; w < w1; ++w) c += (uint32_t)__popc(ld_cg(bitmap + w));
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - c, all = 0;
+    for (int k = 0; k < kListCta / 32; ++k) {
+        if (k < warp) at += s_w[k];
+        all += s_w[k];
+    }
+    for (uint32_t w = w0; w < w1; ++w) {
+        st_cg(prefix + w, at);
+        at += (uint32_t)__popc(ld_cg(bitmap + w));
+    }
+    if (t == 0 && d_nlabels) *d_nlabels = all;
+    __syncthreads();
+    for (uint32_t i = t; i < cnt; i += kListCta) {
+        const uint32_t m = list[i], idx = fkey_index((float)ld_cg(lab + m)), w = idx >> 5;
+        st_cg(lab + m, ld_cg(prefix + w) + (uint32_t)__popc(ld_cg(bitmap + w) & ((1u << (idx & 31)) - 1u)) + 1u);
+    }
 }
 
 // ---- rank machinery -------------------------------------------------------
-__global__ void chunk_count_kernel(const uint32_t *__restrict__ bitmap, uint32_t words,
-                                   uint32_t *__restrict__ chunk) {
-    const uint32_t nchunks = (words + 31) / 32;
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += gridDim.x * blockDim.x) {
-        uint32_t s = 0;
-        const uint32_t w1 = min(words, (c + 1) * 32);
-        for (uint32_t w = c * 32; w < w1; ++w) s += __popc(bitmap[w]);
-        chunk[c] = s;
+// Per bitmap word the number of set bits before it, in two launches: bits per
+// block of `per` words, then every block adds up the blocks before it (at most
+// kRankBlocks of them) and scans its words, 4 per thread and round.  The last
+// block also writes the total.
+constexpr uint32_t kRankBlocks = 2048, kRankRound = 4 * kT;
+
+__global__ void __launch_bounds__(kT)
+rank_sums_kernel(const uint32_t *__restrict__ bitmap, uint32_t words, uint32_t per, uint32_t *__restrict__ sums) {
+    const uint32_t w0 = blockIdx.x * per, w1 = min(words, w0 + per);
+    uint32_t c = 0;
+    for (uint32_t w = w0 + 4 * threadIdx.x; w < w1; w += kRankRound)   // per and w0 are multiples of 4
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (w + k < w1) c += (uint32_t)__popc(bitmap[w + k]);
+    c = __reduce_add_sync(0xffffffffu, c);
+    __shared__ uint32_t s_c[kT / 32];
+    if ((threadIdx.x & 31) == 0) s_c[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kT / 32; ++k) c += s_c[k];
+        sums[blockIdx.x] = c;
     }
 }
 
-// Exclusive scan of n uint32 in place, one CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) scan_single_cta(uint32_t *__restrict__ a, uint32_t n) {
-    __shared__ uint32_t warp_tot[32];
-    const uint32_t per = (n + 1023) / 1024;
-    const uint32_t b0 = threadIdx.x * per;
-    const uint32_t b1 = min(n, b0 + per);
-    uint32_t s = 0;
-    for (uint32_t i = b0; i < b1; ++i) s += a[i];
-    // inclusive scan of s over the block
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t v = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
-    }
-    if (lane == 31) warp_tot[wid] = v;
+__global__ void __launch_bounds__(kT)
+rank_prefix_kernel(const uint32_t *__restrict__ bitmap, uint32_t words, uint32_t per, const uint32_t *__restrict__ sums,
+                   uint32_t *__restrict__ prefix, uint32_t *__restrict__ total) {
+    __shared__ uint32_t s_w[kT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // bits before this block
+    uint32_t before = 0;
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kT) before += sums[i];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) s_w[warp] = before;
     __syncthreads();
-    if (wid == 0) {
-        uint32_t t = warp_tot[lane];
+    before = 0;
+    for (int k = 0; k < kT / 32; ++k) before += s_w[k];
+    const uint32_t w0 = blockIdx.x * per, w1 = min(words, w0 + per);
+    for (uint32_t base = w0; base < w1; base += kRankRound) {
+        const uint32_t w = base + 4 * threadIdx.x;
+        uint32_t c[4], x = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            c[k] = x;
+            x += w + k < w1 ? (uint32_t)__popc(bitmap[w + k]) : 0u;
+        }
+        uint32_t incl = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t u = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += u;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
         }
-        warp_tot[lane] = t;
-    }
-    __syncthreads();
-    uint32_t run = v - s + (wid ? warp_tot[wid - 1] : 0u);
-    for (uint32_t i = b0; i < b1; ++i) {
-        uint32_t x = a[i];
-        a[i] = run;
-        run += x;
-    }
-}
-
-__global__ void word_prefix_kernel(const uint32_t *__restrict__ bitmap, uint32_t words,
-                                   const uint32_t *__restrict__ chunk, uint32_t *__restrict__ prefix) {
-    const uint32_t nchunks = (words + 31) / 32;
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += gridDim.x * blockDim.x) {
-        uint32_t run = chunk[c];
-        const uint32_t w1 = min(words, (c + 1) * 32);
-        for (uint32_t w = c * 32; w < w1; ++w) {
-            prefix[w] = run;
-            run += __popc(bitmap[w]);
+        __syncthreads();
+        if (lane == 31) s_w[warp] = incl;
+        __syncthreads();
+        uint32_t at = before + incl - x, all = 0;
+        for (int k = 0; k < kT / 32; ++k) {
+            if (k < warp) at += s_w[k];
+            all += s_w[k];
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (w + k < w1) prefix[w + k] = at + c[k];
+        before += all;
     }
+    if (total && blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) *total = before;
 }
 
 struct Rank {
-    uint32_t *bitmap, *chunk, *prefix;
-    uint32_t words, nchunks;
+    uint32_t *bitmap, *sums, *prefix;
+    uint32_t words, per, blocks;
 };
 
 Rank take_rank(Arena &ws, uint64_t bits) {
     Rank r;
     r.words = (uint32_t)((bits + 31) / 32 + 1);
-    r.nchunks = (r.words + 31) / 32;
+    // whole rounds per block
+    r.per = ((r.words + kRankBlocks - 1) / kRankBlocks + kRankRound - 1) / kRankRound * kRankRound;
+    r.blocks = (r.words + r.per - 1) / r.per;
     r.bitmap = ws.take<uint32_t>(r.words);
-    r.chunk = ws.take<uint32_t>(r.nchunks);
+    r.sums = ws.take<uint32_t>(r.blocks);
     r.prefix = ws.take<uint32_t>(r.words);
     return r;
 }
 
-int rank_build(const Rank &r, cudaStream_t st) {
-    const int b = launch_blocks(r.nchunks, kT);
-    chunk_count_kernel<<<b, kT, 0, st>>>(r.bitmap, r.words, r.chunk);
-    scan_single_cta<<<1, 1024, 0, st>>>(r.chunk, r.nchunks);
-    word_prefix_kernel<<<b, kT, 0, st>>>(r.bitmap, r.words, r.chunk, r.prefix);
-    CLE_LAUNCH_CHECK_N("rank build", 3);
+// prefix from bitmap; *total (optional): the number of set bits
+int rank_build(const Rank &r, cudaStream_t st, uint32_t *total = nullptr) {
+    rank_sums_kernel<<<r.blocks, kT, 0, st>>>(r.bitmap, r.words, r.per, r.sums);
+    rank_prefix_kernel<<<r.blocks, kT, 0, st>>>(r.bitmap, r.words, r.per, r.sums, r.prefix, total);
+    CLE_LAUNCH_CHECK_N("rank build", 2);
     return CLE_OK;
 }
 
@@ -698,19 +763,20 @@ int ccl_list(const Geo &g, int64_t n, uint32_t *lab, const uint32_t *list,
              uint32_t *d_nlabels) {
     Rank r = take_rank(ws, fkey_bits_for(n));
     if (!ws.ok()) { set_error("seed labeling: workspace too small"); return CLE_ERR_WORKSPACE; }
+    if (n <= kListCtaVoxels) {
+        ccl_list_small<<<1, kListCta, 0, st>>>(lab, g, list, d_count, r.bitmap, r.prefix, r.words, d_nlabels);
+        CLE_LAUNCH_CHECK("ccl list (one CTA)");
+        return CLE_OK;
+    }
     const int b = launch_blocks(cap, kT);
     ccl_union_list<<<b, kT, 0, st>>>(lab, g, list, d_count);
     ccl_flatten_list<<<b, kT, 0, st>>>(lab, g, list, d_count);
     CLE_CUDA(cudaMemsetAsync(r.bitmap, 0, sizeof(uint32_t) * r.words, st));
     ccl_mark_list<<<b, kT, 0, st>>>(lab, g, list, d_count, r.bitmap);
     CLE_LAUNCH_CHECK_N("ccl list", 3);
-    CLE_TRY(rank_build(r, st));
+    CLE_TRY(rank_build(r, st, d_nlabels));
     ccl_label_list<<<b, kT, 0, st>>>(lab, list, d_count, r.bitmap, r.prefix);
     CLE_LAUNCH_CHECK("ccl list label");
-    if (d_nlabels) {
-        count_ranks_kernel<<<1, 1, 0, st>>>(r.bitmap, r.prefix, r.words, d_nlabels);
-        CLE_LAUNCH_CHECK("label count");
-    }
     return CLE_OK;
 }
 

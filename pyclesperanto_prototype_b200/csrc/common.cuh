@@ -125,6 +125,30 @@ __device__ __forceinline__ float ord2f(int i) {
     return __int_as_float(i >= 0 ? i : i ^ 0x7FFFFFFF);
 }
 
+// Order-preserving float -> unsigned mapping and back; 0 is below every number.
+__device__ __forceinline__ uint32_t f2u(float f) { return (uint32_t)f2ord(f) ^ 0x80000000u; }
+__device__ __forceinline__ float u2f(uint32_t u) { return ord2f((int)(u ^ 0x80000000u)); }
+
+// Min / max of an image over the CTAs that produce it.  The words start at 0;
+// the last CTA to add its own writes {min, max}.
+struct MinMaxState {
+    uint32_t not_min, max;   // ~f2u(min), f2u(max)
+    uint32_t done;           // CTAs that have added theirs
+    uint32_t pad;
+    float out[2];            // {min, max}
+};
+// One thread per CTA, with the CTA's values (min = +inf and max = -inf: none).
+__device__ __forceinline__ void add_minmax(MinMaxState *m, float mn, float mx, uint32_t ctas) {
+    atomicMax(&m->not_min, ~f2u(mn));
+    atomicMax(&m->max, f2u(mx));
+    __threadfence();
+    if (atomicAdd(&m->done, 1u) + 1u == ctas) {
+        __threadfence();
+        m->out[0] = u2f(~*(volatile uint32_t *)&m->not_min);
+        m->out[1] = u2f(*(volatile uint32_t *)&m->max);
+    }
+}
+
 // L2-coherent loads/stores for data that other SMs update during a kernel.
 __device__ __forceinline__ uint32_t ld_cg(const uint32_t *p) { return __ldcg(p); }
 __device__ __forceinline__ void st_cg(uint32_t *p, uint32_t v) { __stcg(p, v); }

@@ -8,11 +8,10 @@ namespace cle {
 // blur.cu
 size_t separable_workspace_bytes(const Img &im);
 int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty, const Taps *tz,
-                     Arena &ws, cudaStream_t st, float *mm = nullptr);
-// Three-pass isotropic blur (sigma > 0) whose {min, max} lands in d_minmax,
-// reduced in the last pass (mm above: 2 floats per CTA of it).
-size_t separable_minmax_workspace_bytes(const Img &src);
-int separable_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st);
+                     Arena &ws, cudaStream_t st, MinMaxState *mm = nullptr);
+// Three-pass isotropic blur (sigma > 0) whose {min, max} lands in mm->out (the
+// state zeroed before), reduced in the last pass.
+int separable_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st);
 // status (optional): a device status word; given it, the fused path of a
 // volume may stage planes with TMA copies and reports a stage wait that ran
 // out there (CLE_ERR_ITER_LIMIT)
@@ -23,29 +22,27 @@ int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, A
 // kMaxFusedR3 in 3D
 constexpr int kMaxFusedR = 14, kMaxFusedR3 = 8;
 bool fused_blur_applies(const Img &src, double sx, double sy, double sz);
-// mm (optional): 2 floats per CTA, the CTA's min / max of the result
-int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, float *mm = nullptr,
+// mm (optional, zeroed before): the result's min / max
+int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, MinMaxState *mm = nullptr,
                int *status = nullptr);
-// Isotropic blur whose {min, max} lands in d_minmax (device): the fused
-// launch's CTA partials and a one-CTA finish, or blur + minmax otherwise.
-size_t blur_minmax_workspace_bytes(const Img &src);
-int blur_minmax(const Img &src, float *dst, double sigma, float *d_minmax, Arena &ws, cudaStream_t st,
+// Isotropic blur whose {min, max} lands in mm->out (the state zeroed before).
+// Workspace: separable_workspace_bytes and minmax_workspace_bytes.
+int blur_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st,
                 int *status = nullptr);
 
 // reduce.cu
 size_t minmax_workspace_bytes(const Img &im);
 // Writes {min, max} to d_out (device) without host synchronisation.
 int minmax(const Img &im, float *d_out, Arena &ws, cudaStream_t st);
-// {min, max} of `blocks` partial pairs into d_out (one CTA).
-int minmax_finish(const float *partial, int blocks, float *d_out, cudaStream_t st);
 size_t histogram_workspace_bytes(const Img &im, int bins);
 // Row-partial histogram + float32 row sum (reference order); d_minmax holds {min,max}.
 int histogram(const Img &im, int bins, const float *d_minmax, float *d_hist, Arena &ws,
               cudaStream_t st);
-// Otsu on a 256-bin float32 histogram, device float64.  Writes the float64
-// threshold to d_thr (may be null) and its float32 cast to d_thr32.
-int otsu(const float *d_hist, const float *d_minmax, double *d_thr, float *d_thr32,
-         cudaStream_t st);
+// The 256-bin histogram and Otsu on it (device float64), by the last CTA of the
+// row sums.  Writes the float64 threshold to d_thr (may be null) and its
+// float32 cast to d_thr32.
+int histogram_otsu(const Img &im, const float *d_minmax, float *d_hist, double *d_thr, float *d_thr32, Arena &ws,
+                   cudaStream_t st);
 int greater_constant(const Img &src, const Img &dst, float c, const float *d_c, cudaStream_t st);
 int binary_and(const Img &a, const Img &b, const Img &dst, cudaStream_t st);
 int mask_op(const Img &src, const Img &mask, const Img &dst, cudaStream_t st);
@@ -100,23 +97,16 @@ int relabel_sequential(const Img &src, const Img &dst, uint32_t max_label, Arena
 size_t rank_workspace_bytes(uint64_t bits);
 
 // voronoi.cu
-size_t voronoi_frontier_workspace_bytes(const Img &im);
-// Frontier-queued Jacobi growth.  labels: u32 with seed labels, 0 elsewhere;
-// seg: u8 mask (0/1); seeds: device list of seed memory indices (count in
-// d_seed_count).  d_status receives 0 or an error.
-// gate: when set, the launch returns at once unless *gate != 0 on the device.
-int voronoi_frontier(const Img &shape, uint32_t *labels, const uint8_t *seg,
-                     const uint32_t *seeds, const uint32_t *d_seed_count, int *d_status,
-                     Arena &ws, cudaStream_t st, const Limits &lim, const int *gate = nullptr);
-// The same growth by arrival keys (bricks relaxed to convergence per visit,
-// rounds instead of steps), for labels up to 2^24 - 1 (d_max_label: the
-// largest seed label on the device) and up to 120 steps; otherwise the labels
-// are left as given and the frontier kernel above grows them.  seg: mask
-// bytes as the seed passes write them (kMaskByte); the growth keeps each
-// labelled voxel's arrival step in them.  segments: the mask is the whole
-// image, the list holds one labelled voxel per 8-voxel row segment and the
-// mask bytes of labelled voxels are 0x80 already.  Workspace includes the
-// frontier kernel's.
+// Growth of seed labels inside a mask: labels u32 with the seeds' labels, 0
+// elsewhere; seeds: device list of seed memory indices (count in
+// d_seed_count); d_status receives 0 or an error.  By arrival keys (bricks
+// relaxed to convergence per visit, rounds instead of steps), for labels up to
+// 2^24 - 1 (d_max_label: the largest seed label on the device) and up to 120
+// steps; otherwise the labels are left as given and the brick kernel behind it
+// grows them step by step.  seg: mask bytes as the seed passes write them
+// (kMaskByte); the growth keeps each labelled voxel's arrival step in them.
+// segments: the mask is the whole image, the list holds one labelled voxel per
+// 8-voxel row segment and the mask bytes of labelled voxels are 0x80 already.
 size_t voronoi_grow_workspace_bytes(const Img &im);
 int voronoi_grow(const Img &shape, uint32_t *labels, uint8_t *seg, const uint32_t *seeds,
                  const uint32_t *d_seed_count, const uint32_t *d_max_label, int *d_status, Arena &ws,

@@ -75,8 +75,7 @@ int threshold_otsu_noalloc(const Img &a, const Img &b, cudaStream_t st) {
     float *hist = ar.take<float>(256);
     double *thr = ar.take<double>(4);
     CLE_TRY(minmax(a, mm, ar, st));
-    CLE_TRY(histogram(a, 256, mm, hist, ar, st));   // clears its row partials first
-    CLE_TRY(otsu(hist, mm, thr, mm + 2, st));
+    CLE_TRY(histogram_otsu(a, mm, hist, thr, mm + 2, ar, st));   // clears its row partials first
     return greater_constant(a, b, 0.0f, mm + 2, st);
 }
 

@@ -23,7 +23,7 @@ struct Scalars {
     uint32_t seed_count;
     uint32_t nlabels;        // labels of the last call (= its maximum label)
     uint32_t pad0;
-    float minmax[2];
+    MinMaxState mm;          // of the outline blur
     float thr32;
     float pad;
     double thr;
@@ -369,7 +369,7 @@ size_t vol_workspace_bytes(const Img &im) {
     size_t tail = 0;
     tail = std::max(tail, separable_workspace_bytes(im));
     tail = std::max(tail, minmax_workspace_bytes(im) + histogram_workspace_bytes(im, 256));
-    tail = std::max(tail, blur_minmax_workspace_bytes(im));
+    tail = std::max(tail, separable_workspace_bytes(im) + minmax_workspace_bytes(im));
     tail = std::max(tail, rank_workspace_bytes(fkey_bits_for(im.n())));
     tail = std::max(tail, voronoi_grow_workspace_bytes(im));
     return base + tail;
@@ -400,7 +400,7 @@ int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma, dou
     // threshold, as the reference's second blur would have recomputed it.
     const bool same_blur = (float)spot_sigma == (float)outline_sigma &&
                            sigma_to_kernel_size(spot_sigma) == sigma_to_kernel_size(outline_sigma);
-    if (same_blur) CLE_TRY(blur_minmax(src, l.T, spot_sigma, l.sc->minmax, ws, st, &l.sc->status));
+    if (same_blur) CLE_TRY(blur_minmax(src, l.T, spot_sigma, &l.sc->mm, ws, st, &l.sc->status));
     else CLE_TRY(gaussian_blur(src, l.T, spot_sigma, spot_sigma, spot_sigma, ws, st, &l.sc->status));
     stage_mark(1, st);
     ws.off = tail_off;
@@ -415,14 +415,13 @@ int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma, dou
     if (!same_blur) CLE_TRY(detect_maxima(Ti, Si, st));
     stage_mark(2, st);
     // the outline blur also reduces the blurred image's min / max (step 4)
-    if (!same_blur) CLE_TRY(blur_minmax(src, l.T, outline_sigma, l.sc->minmax, ws, st, &l.sc->status));
+    if (!same_blur) CLE_TRY(blur_minmax(src, l.T, outline_sigma, &l.sc->mm, ws, st, &l.sc->status));
     ws.off = tail_off;
     stage_mark(3, st);
 
     // 4-6: threshold on the device
-    CLE_TRY(histogram(Ti, 256, l.sc->minmax, l.sc->hist, ws, st));
+    CLE_TRY(histogram_otsu(Ti, l.sc->mm.out, l.sc->hist, &l.sc->thr, &l.sc->thr32, ws, st));
     ws.off = tail_off;
-    CLE_TRY(otsu(l.sc->hist, l.sc->minmax, &l.sc->thr, &l.sc->thr32, st));
     stage_mark(4, st);
 
     // 7: segmentation, seeds, seed keys

@@ -137,7 +137,7 @@ template <typename T>
 __global__ void __launch_bounds__(kHistThreads)
 hist_rows_kernel(const T *__restrict__ src, int64_t D, int64_t H, int64_t W, int bins,
                  int zchunk, const float *__restrict__ d_minmax, uint32_t *__restrict__ part,
-                 FastDiv fw, FastDiv fw4) {
+                 FastDiv fw, FastDiv fw4, uint32_t *__restrict__ done) {
     extern __shared__ uint32_t sh[];   // (warps x bins) when private, else bins
     const int nwarps = kHistThreads / 32;
     const bool priv = bins <= 512;
@@ -256,7 +256,90 @@ merge:
     for (int b = threadIdx.x; b < bins; b += kHistThreads) {
         uint32_t c = 0;
         for (int k = 0; k < ncopies; ++k) c += sh[k * bins + b];
-        if (c) atomicAdd(&part[y * bins + b], c);
+        // a row in one chunk is stored, the chunks of a row are added up
+        if (gridDim.y == 1) part[y * bins + b] = c;
+        else if (c) atomicAdd(&part[y * bins + b], c);
+    }
+    if (done && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *done = 0u;
+}
+
+// A7: scikit-image Otsu on the histogram, float64, no contraction, numpy's
+// sequential cumsum, first-occurrence argmax with NaN as maximum
+// (_tier9/_threshold_otsu.py:38-49, :83-106).  Only the four running sums are
+// sequential (numpy's cumsum order): one lane of a warp each, from products
+// formed before and values loaded 16 at a time, so that a step costs one
+// addition; everything else runs in parallel.  A CTA of 256 threads or more
+// calls it.  Row sums and Otsu of a 256 x 256 image take 8.4 us in one launch
+// (19.4 in two, with two sums to a thread, product and loads inside the chain
+// and a sequential argmax).
+struct OtsuShared {
+    double bc[256], c[256], p[256], w1[256], w2[256], s1[256], s2[256];
+    double best[8];
+    int at[8];
+};
+
+// out[i] = running sum of v in index order (or from the end backwards)
+template <bool BACK>
+__device__ __forceinline__ void running_sum(const double *v, double *out) {
+    double acc = 0.0;
+#pragma unroll 2
+    for (int i0 = 0; i0 < 256; i0 += 16) {
+        double x[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) x[k] = v[BACK ? 255 - (i0 + k) : i0 + k];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            acc = __dadd_rn(acc, x[k]);
+            out[BACK ? 255 - (i0 + k) : i0 + k] = acc;
+        }
+    }
+}
+
+// a beats b in numpy's argmax (b has the smaller index)
+__device__ __forceinline__ bool beats(double a, double b) { return b == b && (a != a || a > b); }
+
+__device__ __forceinline__ void otsu_block(OtsuShared &o, const volatile float *hist, const float *d_minmax, double *d_thr,
+                                           float *d_thr32) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const float mn = d_minmax[0];
+    const float range32 = __fsub_rn(d_minmax[1], mn);
+    if (t < 256) {
+        o.bc[t] = __dadd_rn(__ddiv_rn(__dmul_rn((double)t, (double)range32), 255.0), (double)mn);
+        o.c[t] = (double)hist[t];
+        o.p[t] = __dmul_rn(o.c[t], o.bc[t]);
+    }
+    __syncthreads();
+    if (t == 0) running_sum<false>(o.p, o.s1);
+    else if (t == 32) running_sum<true>(o.p, o.s2);
+    else if (t == 64) running_sum<false>(o.c, o.w1);
+    else if (t == 96) running_sum<true>(o.c, o.w2);
+    __syncthreads();
+    if (t < 256) {
+        double v = -INFINITY;   // below every variance (they are squares times counts, or NaN)
+        int at = t;
+        if (t < 255) {
+            const double m1 = __ddiv_rn(o.s1[t], o.w1[t]);
+            const double m2 = __ddiv_rn(o.s2[t + 1], o.w2[t + 1]);
+            const double d = __dsub_rn(m1, m2);
+            v = __dmul_rn(__dmul_rn(o.w1[t], o.w2[t + 1]), __dmul_rn(d, d));
+        }
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {   // the lower lane keeps ties: the first occurrence
+            const double w = __shfl_down_sync(0xffffffffu, v, k);
+            const int wa = __shfl_down_sync(0xffffffffu, at, k);
+            if (beats(w, v)) { v = w; at = wa; }
+        }
+        if (lane == 0) { o.best[warp] = v; o.at[warp] = at; }
+    }
+    __syncthreads();
+    if (t == 0) {
+        int idx = o.at[0];
+        double v = o.best[0];
+        for (int k = 1; k < 8; ++k)
+            if (beats(o.best[k], v)) { v = o.best[k]; idx = o.at[k]; }
+        const double thr = o.bc[idx];
+        if (d_thr) *d_thr = thr;
+        if (d_thr32) *d_thr32 = __double2float_rn(thr);
     }
 }
 
@@ -268,10 +351,14 @@ merge:
 // warp each; the others take their exact total.  A CTA owns 32 bins: warp w
 // adds rows w, w + 32, ... of its lane's bin with 8 loads in flight, so the
 // totals take a few memory round trips instead of one per row.
+// With OTSU (256 bins) the last CTA to finish runs Otsu on the histogram; `done`
+// counts the finished CTAs (0 at the start).
 constexpr int kRowsumBins = 32;
+template <bool OTSU>
 __global__ void __launch_bounds__(1024)
-hist_rowsum_kernel(const uint32_t *__restrict__ part, int64_t H, int bins,
-                   float *__restrict__ hist) {
+hist_rowsum_kernel(const uint32_t *__restrict__ part, int64_t H, int bins, float *hist,
+                   const float *__restrict__ d_minmax, double *__restrict__ d_thr, float *__restrict__ d_thr32,
+                   uint32_t *__restrict__ done) {
     __shared__ unsigned long long s_tot[32][kRowsumBins + 1];
     __shared__ unsigned long long s_bin[kRowsumBins];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -300,73 +387,30 @@ hist_rowsum_kernel(const uint32_t *__restrict__ part, int64_t H, int bins,
     // ordered float32 sums: warp j takes bin j of the CTA when its total is
     // at or above 2^24
     const int bb = blockIdx.x * kRowsumBins + warp;
-    if (bb >= bins || s_bin[warp] < (1ull << 24)) return;
-    float acc32 = 0.0f;
-    for (int64_t y0 = 0; y0 < H; y0 += 32) {
-        const int64_t y = y0 + lane;
-        const uint32_t v = (y < H) ? part[y * bins + bb] : 0u;
-        const int n = (H - y0 < 32) ? (int)(H - y0) : 32;
+    if (bb < bins && s_bin[warp] >= (1ull << 24)) {
+        float acc32 = 0.0f;
+        for (int64_t y0 = 0; y0 < H; y0 += 32) {
+            const int64_t y = y0 + lane;
+            const uint32_t v = (y < H) ? part[y * bins + bb] : 0u;
+            const int n = (H - y0 < 32) ? (int)(H - y0) : 32;
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            const uint32_t x = __shfl_sync(0xffffffffu, v, k);
-            if (k < n) acc32 = __fadd_rn(acc32, (float)x);
+            for (int k = 0; k < 32; ++k) {
+                const uint32_t x = __shfl_sync(0xffffffffu, v, k);
+                if (k < n) acc32 = __fadd_rn(acc32, (float)x);
+            }
         }
+        if (lane == 0) hist[bb] = acc32;
     }
-    if (lane == 0) hist[bb] = acc32;
-}
-
-// A7: scikit-image Otsu on the histogram, float64, no contraction, numpy's
-// sequential cumsum, first-occurrence argmax with NaN as maximum
-// (_tier9/_threshold_otsu.py:38-49, :83-106).  Only the running sums are
-// sequential (numpy's cumsum order); the divisions and the between-class
-// variances are elementwise and run in parallel.
-__global__ void __launch_bounds__(256)
-otsu_kernel(const float *__restrict__ hist, const float *__restrict__ d_minmax,
-            double *__restrict__ d_thr, float *__restrict__ d_thr32) {
-    constexpr int B = 256;
-    __shared__ double bc[B], c[B], w1[B], w2[B], s1[B], s2[B], var[B];
-    const int t = threadIdx.x;
-    const float mn = d_minmax[0];
-    const float range32 = __fsub_rn(d_minmax[1], mn);
-    bc[t] = __dadd_rn(__ddiv_rn(__dmul_rn((double)t, (double)range32), 255.0), (double)mn);
-    c[t] = (double)hist[t];
-    __syncthreads();
-    if (t == 0) {
-        double acc = 0.0, accm = 0.0;
-        for (int i = 0; i < B; ++i) {
-            acc = __dadd_rn(acc, c[i]);
-            accm = __dadd_rn(accm, __dmul_rn(c[i], bc[i]));
-            w1[i] = acc;
-            s1[i] = accm;
-        }
-    } else if (t == 32) {
-        double acc = 0.0, accm = 0.0;
-        for (int i = B - 1; i >= 0; --i) {
-            acc = __dadd_rn(acc, c[i]);
-            accm = __dadd_rn(accm, __dmul_rn(c[i], bc[i]));
-            w2[i] = acc;
-            s2[i] = accm;
-        }
-    }
-    __syncthreads();
-    if (t < B - 1) {
-        const double m1 = __ddiv_rn(s1[t], w1[t]);
-        const double m2 = __ddiv_rn(s2[t + 1], w2[t + 1]);
-        const double d = __dsub_rn(m1, m2);
-        var[t] = __dmul_rn(__dmul_rn(w1[t], w2[t + 1]), __dmul_rn(d, d));
-    }
-    __syncthreads();
-    if (t == 0) {
-        int idx = 0;
-        double best = 0.0;
-        for (int i = 0; i < B - 1; ++i) {
-            const double v = var[i];
-            if (v != v) { idx = i; break; }
-            if (i == 0 || v > best) { best = v; idx = i; }
-        }
-        const double thr = bc[idx];
-        if (d_thr) *d_thr = thr;
-        if (d_thr32) *d_thr32 = __double2float_rn(thr);
+    if constexpr (OTSU) {
+        __shared__ OtsuShared o;
+        __shared__ uint32_t s_ticket;
+        __threadfence();   // this CTA's bins before its ticket
+        __syncthreads();
+        if (threadIdx.x == 0) s_ticket = atomicAdd(done, 1u);
+        __syncthreads();
+        if (s_ticket + 1u != gridDim.x) return;
+        __threadfence();   // every other CTA's bins after theirs
+        otsu_block(o, hist, d_minmax, d_thr, d_thr32);
     }
 }
 
@@ -469,12 +513,6 @@ size_t minmax_workspace_bytes(const Img &im) {
     return a.off;
 }
 
-int minmax_finish(const float *partial, int blocks, float *d_out, cudaStream_t st) {
-    minmax_final_kernel<<<1, 1024, 0, st>>>(partial, blocks, d_out);
-    CLE_LAUNCH_CHECK("minmax finish");
-    return CLE_OK;
-}
-
 int minmax(const Img &im, float *d_out, Arena &ws, cudaStream_t st) {
     const int blocks = minmax_blocks(im.n());
     float *partial = ws.take<float>(2 * (size_t)blocks);
@@ -494,15 +532,24 @@ int minmax(const Img &im, float *d_out, Arena &ws, cudaStream_t st) {
 size_t histogram_workspace_bytes(const Img &im, int bins) {
     Arena a(nullptr, 0);
     a.take<uint32_t>((size_t)im.H * bins);
+    a.take<uint32_t>(1);
     return a.off;
 }
 
-int histogram(const Img &im, int bins, const float *d_minmax, float *d_hist, Arena &ws,
-              cudaStream_t st) {
+namespace {
+
+struct OtsuOut {
+    bool on = false;
+    double *thr = nullptr;
+    float *thr32 = nullptr;
+};
+
+int histogram_impl(const Img &im, int bins, const float *d_minmax, float *d_hist, const OtsuOut &o, Arena &ws,
+                   cudaStream_t st) {
     if (bins < 1) { set_error("histogram: num_bins must be >= 1"); return CLE_ERR_ARG; }
     uint32_t *part = ws.take<uint32_t>((size_t)im.H * bins);
+    uint32_t *done = ws.take<uint32_t>(1);
     if (!ws.ok()) { set_error("histogram: workspace too small"); return CLE_ERR_WORKSPACE; }
-    CLE_CUDA(cudaMemsetAsync(part, 0, sizeof(uint32_t) * im.H * bins, st));
     int dev = 0;
     cudaGetDevice(&dev);
     const int64_t target = (int64_t)num_sms(dev) * 8;
@@ -515,32 +562,45 @@ int histogram(const Img &im, int bins, const float *d_minmax, float *d_hist, Are
     dim3 grid((unsigned)im.H, (unsigned)zchunks);
     const size_t smem = sizeof(uint32_t) * bins * (bins <= 512 ? kHistThreads / 32 : 1);
     if (smem > 227 * 1024) { set_error("histogram: too many bins (%d)", bins); return CLE_ERR_ARG; }
+    if (zchunks > 1) CLE_CUDA(cudaMemsetAsync(part, 0, sizeof(uint32_t) * im.H * bins, st));
+    const FastDiv fw((uint32_t)im.W), fw4((uint32_t)std::max<int64_t>(1, im.W / 4));
     switch (im.dtype) {
         case CLE_F32:
             if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(hist_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            hist_rows_kernel<float><<<grid, kHistThreads, smem, st>>>((const float *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, FastDiv((uint32_t)im.W), FastDiv((uint32_t)std::max<int64_t>(1, im.W / 4)));
+            hist_rows_kernel<float><<<grid, kHistThreads, smem, st>>>((const float *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, fw, fw4, done);
             break;
         case CLE_U16:
             if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(hist_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            hist_rows_kernel<uint16_t><<<grid, kHistThreads, smem, st>>>((const uint16_t *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, FastDiv((uint32_t)im.W), FastDiv((uint32_t)std::max<int64_t>(1, im.W / 4)));
+            hist_rows_kernel<uint16_t><<<grid, kHistThreads, smem, st>>>((const uint16_t *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, fw, fw4, done);
             break;
         case CLE_U8:
             if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(hist_rows_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            hist_rows_kernel<uint8_t><<<grid, kHistThreads, smem, st>>>((const uint8_t *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, FastDiv((uint32_t)im.W), FastDiv((uint32_t)std::max<int64_t>(1, im.W / 4)));
+            hist_rows_kernel<uint8_t><<<grid, kHistThreads, smem, st>>>((const uint8_t *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, fw, fw4, done);
             break;
         default: set_error("histogram: unsupported dtype %d", im.dtype); return CLE_ERR_DTYPE;
     }
     CLE_LAUNCH_CHECK("histogram rows");
-    hist_rowsum_kernel<<<(bins + kRowsumBins - 1) / kRowsumBins, 1024, 0, st>>>(part, im.H, bins, d_hist);
+    const int sums = (bins + kRowsumBins - 1) / kRowsumBins;
+    if (o.on) hist_rowsum_kernel<true><<<sums, 1024, 0, st>>>(part, im.H, bins, d_hist, d_minmax, o.thr, o.thr32, done);
+    else hist_rowsum_kernel<false><<<sums, 1024, 0, st>>>(part, im.H, bins, d_hist, nullptr, nullptr, nullptr, nullptr);
     CLE_LAUNCH_CHECK("histogram rowsum");
     return CLE_OK;
 }
 
-int otsu(const float *d_hist, const float *d_minmax, double *d_thr, float *d_thr32,
-         cudaStream_t st) {
-    otsu_kernel<<<1, 256, 0, st>>>(d_hist, d_minmax, d_thr, d_thr32);
-    CLE_LAUNCH_CHECK("otsu");
-    return CLE_OK;
+}  // namespace
+
+int histogram(const Img &im, int bins, const float *d_minmax, float *d_hist, Arena &ws,
+              cudaStream_t st) {
+    return histogram_impl(im, bins, d_minmax, d_hist, OtsuOut(), ws, st);
+}
+
+int histogram_otsu(const Img &im, const float *d_minmax, float *d_hist, double *d_thr, float *d_thr32, Arena &ws,
+                   cudaStream_t st) {
+    OtsuOut o;
+    o.on = true;
+    o.thr = d_thr;
+    o.thr32 = d_thr32;
+    return histogram_impl(im, 256, d_minmax, d_hist, o, ws, st);
 }
 
 template <typename Ts>

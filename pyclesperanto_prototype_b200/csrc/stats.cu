@@ -48,10 +48,6 @@ struct alignas(32) Acc2 {
     float4 pc, pm;
 };
 
-// intensity order as unsigned
-__device__ __forceinline__ uint32_t f2u(float f) { return (uint32_t)f2ord(f) ^ 0x80000000u; }
-__device__ __forceinline__ float u2f(uint32_t u) { return ord2f((int)(u ^ 0x80000000u)); }
-
 // With a device label count (d_L) the init and finalise kernels touch only the
 // first min(count, L) labels; L stays the table's row stride.
 __device__ __forceinline__ int64_t live_labels(int64_t L, const uint32_t *d_L) {

@@ -986,41 +986,53 @@ uint32_t brick_count(const Img &im) { return bricks_z(im) * bricks_y(im) * brick
 
 }  // namespace
 
-size_t voronoi_frontier_workspace_bytes(const Img &im) {
+// The state a growth kernel needs cleared, in one stretch: control block, step
+// tags, queue and finished-brick bitmaps.
+template <typename St>
+struct Cleared {
+    St *S;
+    uint32_t *bstep;
+    BQueue Q;
+    char *begin, *end;
+};
+template <typename St>
+static Cleared<St> take_cleared(Arena &a, const Img &im) {
     const size_t nb = brick_count(im);
-    Arena a(nullptr, 0);
-    a.take<BState>(1);
-    a.take<uint32_t>(nb);        // list 0
-    a.take<uint32_t>(nb);        // list 1
-    a.take<uint32_t>(nb);        // per-brick step tags
-    a.take<uint32_t>(nb * 32 * (size_t)brick_planes(im));   // per-voxel phase-A results
-    a.take<uint32_t>(nb);        // per-entry pending flags
-    a.take<uint32_t>((nb + 31) / 32);   // queue bitmap
-    a.take<uint32_t>((nb + 31) / 32);   // finished-brick bitmap
-    a.take<uint32_t>(2048);             // per-CTA counts of the compaction
-    return a.off;
+    Cleared<St> c;
+    c.S = a.take<St>(1);
+    c.begin = (char *)c.S;
+    c.bstep = a.take<uint32_t>(nb);
+    c.Q.nwords = (uint32_t)((nb + 31) / 32);
+    c.Q.q = a.take<uint32_t>(c.Q.nwords);
+    c.Q.done = a.take<uint32_t>(c.Q.nwords);
+    c.end = (char *)(c.Q.done + c.Q.nwords);
+    return c;
 }
 
-int voronoi_frontier(const Img &im, uint32_t *lab, const uint8_t *seg, const uint32_t *seeds,
-                     const uint32_t *d_seed_count, int *d_status, Arena &ws, cudaStream_t st,
-                     const Limits &lim, const int *gate) {
+// Lists and results of the brick kernel (not cleared).
+struct FrontierLists {
+    uint32_t *B0, *B1, *Mv, *Pf, *ccount;
+};
+static FrontierLists take_frontier_lists(Arena &a, const Img &im) {
     const size_t nb = brick_count(im);
-    BState *S = ws.take<BState>(1);
-    uint32_t *B0 = ws.take<uint32_t>(nb);
-    uint32_t *B1 = ws.take<uint32_t>(nb);
-    uint32_t *bstep = ws.take<uint32_t>(nb);
-    uint32_t *Mv = ws.take<uint32_t>(nb * 32 * (size_t)brick_planes(im));
-    uint32_t *Pf = ws.take<uint32_t>(nb);
-    BQueue Qb;
-    Qb.nwords = (uint32_t)((nb + 31) / 32);
-    Qb.q = ws.take<uint32_t>(Qb.nwords);
-    Qb.done = ws.take<uint32_t>(Qb.nwords);
-    Qb.ccount = ws.take<uint32_t>(2048);
-    if (!ws.ok()) { set_error("masked_voronoi_labeling: workspace too small"); return CLE_ERR_WORKSPACE; }
-    CLE_CUDA(cudaMemsetAsync(Qb.q, 0, sizeof(uint32_t) * (size_t)Qb.nwords, st));
-    CLE_CUDA(cudaMemsetAsync(Qb.done, 0, sizeof(uint32_t) * (size_t)Qb.nwords, st));
-    CLE_CUDA(cudaMemsetAsync(S, 0, sizeof(BState), st));
-    CLE_CUDA(cudaMemsetAsync(bstep, 0, sizeof(uint32_t) * nb, st));
+    FrontierLists f;
+    f.B0 = a.take<uint32_t>(nb);
+    f.B1 = a.take<uint32_t>(nb);
+    f.Mv = a.take<uint32_t>(nb * 32 * (size_t)brick_planes(im));   // per-voxel phase-A results
+    f.Pf = a.take<uint32_t>(nb);                                   // per-entry pending flags
+    f.ccount = a.take<uint32_t>(2048);                             // per-CTA counts of the compaction
+    return f;
+}
+
+// The brick growth with its cleared state `c` (gate: see voronoi_grow below).
+static int launch_frontier(const Img &im, uint32_t *lab, const uint8_t *seg, const uint32_t *seeds,
+                           const uint32_t *d_seed_count, int *d_status, const Cleared<BState> &c, const FrontierLists &f,
+                           cudaStream_t st, const Limits &lim, const int *gate) {
+    const size_t nb = brick_count(im);
+    BState *S = c.S;
+    uint32_t *B0 = f.B0, *B1 = f.B1, *bstep = c.bstep, *Mv = f.Mv, *Pf = f.Pf;
+    BQueue Qb = c.Q;
+    Qb.ccount = f.ccount;
     BGeo G;
     G.g = make_geo(im);
     G.WB = bricks_x(im);
@@ -1063,49 +1075,34 @@ int voronoi_frontier(const Img &im, uint32_t *lab, const uint8_t *seg, const uin
     return CLE_OK;
 }
 
-namespace {
-
-size_t keys_part_bytes(const Img &im) {
-    const size_t nb = brick_count(im);
-    Arena a(nullptr, 0);
-    a.take<KState>(1);
-    a.take<uint32_t>(nb);               // list 0
-    a.take<uint32_t>(nb);               // list 1
-    a.take<uint32_t>(nb);               // per-brick round tags
-    a.take<uint32_t>((nb + 31) / 32);   // queue bitmap
-    a.take<uint32_t>((nb + 31) / 32);   // bricks without candidates
-    a.take<uint32_t>(2048);             // per-CTA counts of the compaction
-    return a.off;
-}
-
-}  // namespace
-
 size_t voronoi_grow_workspace_bytes(const Img &im) {
-    return voronoi_frontier_workspace_bytes(im) + keys_part_bytes(im);
+    Arena a(nullptr, 0);
+    take_frontier_lists(a, im);
+    take_cleared<BState>(a, im);
+    take_cleared<KState>(a, im);
+    a.take<uint32_t>(brick_count(im));   // the key growth's lists
+    a.take<uint32_t>(brick_count(im));
+    a.take<uint32_t>(2048);
+    return a.off;
 }
 
 int voronoi_grow(const Img &im, uint32_t *lab, uint8_t *seg, const uint32_t *seeds,
                  const uint32_t *d_seed_count, const uint32_t *d_max_label, int *d_status, Arena &ws,
                  cudaStream_t st, const Limits &lim, int segments) {
-    // the key kernel's state sits behind the brick kernel's workspace, so the
-    // gate word survives that kernel's set-up
-    const size_t off0 = ws.off;
-    ws.off = off0 + voronoi_frontier_workspace_bytes(im);
     const size_t nb = brick_count(im);
-    KState *S = ws.take<KState>(1);
+    const FrontierLists f = take_frontier_lists(ws, im);
+    const Cleared<BState> cb = take_cleared<BState>(ws, im);
+    const Cleared<KState> ck = take_cleared<KState>(ws, im);
     uint32_t *B0 = ws.take<uint32_t>(nb);
     uint32_t *B1 = ws.take<uint32_t>(nb);
-    uint32_t *bstep = ws.take<uint32_t>(nb);
-    BQueue Qb;
-    Qb.nwords = (uint32_t)((nb + 31) / 32);
-    Qb.q = ws.take<uint32_t>(Qb.nwords);
-    Qb.done = ws.take<uint32_t>(Qb.nwords);
+    KState *S = ck.S;
+    uint32_t *bstep = ck.bstep;
+    BQueue Qb = ck.Q;
     Qb.ccount = ws.take<uint32_t>(2048);
     if (!ws.ok()) { set_error("masked_voronoi_labeling: workspace too small"); return CLE_ERR_WORKSPACE; }
-    CLE_CUDA(cudaMemsetAsync(S, 0, sizeof(KState), st));
-    CLE_CUDA(cudaMemsetAsync(bstep, 0, sizeof(uint32_t) * nb, st));
-    // q and done are adjacent: one clear
-    CLE_CUDA(cudaMemsetAsync(Qb.q, 0, (size_t)((char *)(Qb.done + Qb.nwords) - (char *)Qb.q), st));
+    // both kernels' states lie side by side: one clear (seven before, more
+    // launch time than the growth of a small image needs for two rounds)
+    CLE_CUDA(cudaMemsetAsync(cb.begin, 0, (size_t)(ck.end - cb.begin), st));
     BGeo G;
     G.g = make_geo(im);
     G.WB = bricks_x(im);
@@ -1137,8 +1134,7 @@ int voronoi_grow(const Img &im, uint32_t *lab, uint8_t *seg, const uint32_t *see
     CLE_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kKeyBT), args, smem, st));
     count_launches(1);
     // the brick kernel, which returns at once unless the gate was raised
-    ws.off = off0;
-    return voronoi_frontier(im, lab, seg, seeds, d_seed_count, d_status, ws, st, lim, &S->gate);
+    return launch_frontier(im, lab, seg, seeds, d_seed_count, d_status, cb, f, st, lim, &S->gate);
 }
 
 }  // namespace cle
