@@ -114,121 +114,305 @@ int erode_dst(const Img &src, const Img &dst, cudaStream_t st) {
 // N = int(2*radius + 1), reads clamped to the edge (so the window is the
 // in-range part of it); a pass with radius <= 0 is a copy.  min/max are exact,
 // so the float32 result does not depend on the order of the comparisons.
-constexpr int kLX = 256;        // x pass: outputs per CTA
-constexpr int kLT = 64;         // y/z passes: outputs per CTA along the axis
-constexpr int kLC = 32;         // y/z passes: columns per CTA
+// A thread makes 8 consecutive outputs along the pass axis.  Their windows share
+// all but 7 values at each end, so it takes the minimum of the shared core once
+// and running minima of the two ends: (2r + 8) / 8 loads and about as many
+// comparisons per output instead of 2r.  Loads have immediate offsets (a case
+// per window length modulo 8).  The first pass reads 8/16-bit sources as they are
+// and the last pass of top_hat_box subtracts, so neither has a pass of its own.
+// What bounds it: reading and writing the image in each pass.  r = 10 on 100 x 512 x
+// 512 uint16: x 55 us a pass (141 with a window scan per output), y and z 41 to 51
+// (98), 32 at copy bandwidth; top_hat_box 0.77 -> 0.31 ms.
+constexpr int kBK = 8;            // outputs per thread along the axis
+constexpr int kBT = 256;          // threads per CTA
+constexpr int kBRow = 256;        // x pass: most outputs of a row per CTA
+constexpr int kBPitch = kBK + 1;  // x pass: 8 staged values on 9 words (lanes on different banks)
 
 template <bool MAX>
 __device__ __forceinline__ float mm(float a, float b) { return MAX ? fmaxf(a, b) : fminf(a, b); }
 
-template <bool MAX>
-__global__ void __launch_bounds__(kLX)
-minmax_x_kernel(const float *__restrict__ src, float *__restrict__ dst, int W, int r) {
-    extern __shared__ float row[];                 // [kLX + 2r]
-    const int64_t line = (int64_t)blockIdx.z * gridDim.y + blockIdx.y;
-    const float *s = src + line * W;
-    const int x0 = blockIdx.x * kLX;
-    for (int i = threadIdx.x; i < kLX + 2 * r; i += kLX) row[i] = s[clampi(x0 - r + i, 0, W - 1)];
-    __syncthreads();
-    const int x = x0 + (int)threadIdx.x;
-    if (x >= W) return;
-    float m = row[threadIdx.x];
-    for (int i = 1; i <= 2 * r; ++i) m = mm<MAX>(m, row[threadIdx.x + i]);
-    dst[line * W + x] = m;
+// out[k] = min / max of the w = 8 q + S staged values from k on, k = 0..7 (w is odd).
+// p: the thread's first value; staged value 8 j + k lies at p + j * BLK + k * STR,
+// so that k is an immediate offset.
+template <bool MAX, int S, int BLK, int STR>
+__device__ __forceinline__ void window_of(const float *p, int q, float (&out)[kBK]) {
+    if (q == 0) {
+        float v[kBK + S - 1];
+#pragma unroll
+        for (int i = 0; i < kBK + S - 1; ++i) v[i] = p[i / kBK * BLK + i % kBK * STR];
+#pragma unroll
+        for (int k = 0; k < kBK; ++k) {
+            out[k] = v[k];
+#pragma unroll
+            for (int i = 1; i < S; ++i) out[k] = mm<MAX>(out[k], v[k + i]);
+        }
+        return;
+    }
+    // the core every window holds: values 7 .. w - 1
+    float v[kBK];
+#pragma unroll
+    for (int k = 0; k < kBK; ++k) v[k] = p[k * STR];
+    float core = v[7];
+    const float *b = p + BLK;
+#pragma unroll 2
+    for (int j = 1; j < q; ++j, b += BLK) {
+        float u[kBK];
+#pragma unroll
+        for (int k = 0; k < kBK; ++k) u[k] = b[k * STR];
+#pragma unroll
+        for (int k = 0; k < kBK; k += 2) core = mm<MAX>(mm<MAX>(core, u[k]), u[k + 1]);
+    }
+    float e[kBK + S - 1];   // from value 8 q on
+#pragma unroll
+    for (int i = 0; i < kBK + S - 1; ++i) e[i] = b[i / kBK * BLK + i % kBK * STR];
+#pragma unroll
+    for (int i = 0; i < S; ++i) core = mm<MAX>(core, e[i]);
+    // left ends: values k .. 6, right ends: values w .. w + k - 1
+    float l = core;
+    out[7] = core;
+#pragma unroll
+    for (int k = 6; k >= 0; --k) {
+        l = mm<MAX>(l, v[k]);
+        out[k] = l;
+    }
+    float r = e[S];
+    out[1] = mm<MAX>(out[1], r);
+#pragma unroll
+    for (int k = 2; k < kBK; ++k) {
+        r = mm<MAX>(r, e[S + k - 1]);
+        out[k] = mm<MAX>(out[k], r);
+    }
 }
-
-// Pass along an axis of length L and element stride S (y: S = W, z: S = H*W);
-// blockIdx.z indexes the remaining coordinate with stride OS.
-template <bool MAX>
-__global__ void __launch_bounds__(kLC * 8)
-minmax_axis_kernel(const float *__restrict__ src, float *__restrict__ dst, int W, int L, int64_t S,
-                   int64_t OS, int r) {
-    extern __shared__ float tile[];                // [kLT + 2r][kLC]
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x = blockIdx.x * kLC + tx;
-    const int a0 = blockIdx.y * kLT;
-    const int64_t base = (int64_t)blockIdx.z * OS + min(x, W - 1);
-    for (int i = ty; i < kLT + 2 * r; i += 8) tile[i * kLC + tx] = src[base + (int64_t)clampi(a0 - r + i, 0, L - 1) * S];
-    __syncthreads();
-    if (x >= W) return;
-    for (int o = ty; o < kLT; o += 8) {
-        const int a = a0 + o;
-        if (a >= L) break;
-        float m = tile[o * kLC + tx];
-        for (int i = 1; i <= 2 * r; ++i) m = mm<MAX>(m, tile[(o + i) * kLC + tx]);
-        dst[(int64_t)blockIdx.z * OS + x + (int64_t)a * S] = m;
+template <bool MAX, int BLK, int STR>
+__device__ __forceinline__ void window8(const float *p, int w, float (&out)[kBK]) {
+    switch (w % kBK) {
+        case 1: window_of<MAX, 1, BLK, STR>(p, w / kBK, out); break;
+        case 3: window_of<MAX, 3, BLK, STR>(p, w / kBK, out); break;
+        case 5: window_of<MAX, 5, BLK, STR>(p, w / kBK, out); break;
+        default: window_of<MAX, 7, BLK, STR>(p, w / kBK, out); break;
     }
 }
 
-constexpr int kMaxBoxRadius = 700;   // shared tile (kLT + 2r) x 32 floats <= 187 KB
-
-template <bool MAX>
-int minmax_pass(const float *src, float *dst, const Img &im, int axis, int r, cudaStream_t st) {
-    const int64_t n = im.n();
-    if (r <= 0) {
-        if (dst != src) CLE_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-        return CLE_OK;
+// x pass: np rows per CTA, an x tile of `tile` outputs (a multiple of 8) of each.
+template <bool MAX, typename Tin>
+__global__ void __launch_bounds__(kBT)
+minmax_row_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t rows, int W, int r, int tile, int np,
+                  FastDiv fper) {
+    extern __shared__ float sm[];
+    const int span = tile + 2 * r, pitch = (span / kBK + 2) * kBPitch;
+    const int x0 = blockIdx.x * tile, lane = threadIdx.x & 31;
+    const int64_t row0 = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * np;
+    if (row0 >= rows) return;
+    for (int q = threadIdx.x >> 5; q < np; q += kBT / 32) {
+        const Tin *p = src + min(row0 + q, rows - 1) * W;
+        float *ln = sm + q * pitch;
+        for (int c0 = lane; c0 < span; c0 += 4 * 32) {
+            float v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c0 + 32 * u < span) v[u] = to_f32(__ldg(p + clampi(x0 - r + c0 + 32 * u, 0, W - 1)));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = c0 + 32 * u;
+                if (c < span) ln[c + c / kBK] = v[u];
+            }
+        }
     }
+    __syncthreads();
+    const int per = tile / kBK;
+    for (int e = threadIdx.x; e < np * per; e += kBT) {
+        const int q = (int)fper.div((uint32_t)e), c = e - q * per, x = x0 + c * kBK;
+        if (row0 + q >= rows || x >= W) continue;
+        const float *base = sm + q * pitch + c * kBPitch;
+        float out[kBK];
+        window8<MAX, kBPitch, 1>(base, 2 * r + 1, out);
+        float *o = dst + (row0 + q) * W + x;
+        if ((W & 3) == 0 && x + kBK <= W && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            reinterpret_cast<float4 *>(o)[0] = make_float4(out[0], out[1], out[2], out[3]);
+            reinterpret_cast<float4 *>(o)[1] = make_float4(out[4], out[5], out[6], out[7]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kBK; ++k)
+                if (x + k < W) o[k] = out[k];
+        }
+    }
+}
+
+// Pass along an axis of length L with element stride `inner`, for a volume
+// viewed as [outer][L][inner]: a CTA takes NG x 8 outputs along the axis and
+// 2 x 256 / NG columns, a thread two adjacent columns.
+template <bool MAX, typename Tin, int NG, typename Ts>
+__global__ void __launch_bounds__(kBT)
+minmax_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t inner, int L, int r, int vec,
+                  const Ts *__restrict__ minus) {
+    constexpr int NC = kBT / NG, COLS = 2 * NC, ROWS = NG * kBK;
+    extern __shared__ __align__(16) float sm[];
+    const int64_t c0 = (int64_t)blockIdx.x * COLS, base = (int64_t)blockIdx.z * L * inner;
+    const int l0 = blockIdx.y * ROWS;
+    const int span = ROWS + 2 * r;   // rows past the axis repeat its last value
+    if (vec) {   // float32, inner a multiple of 4: asynchronous 16-byte copies
+        constexpr int QPR = COLS / 4, STEP = kBT / QPR;
+        const int c = 4 * (threadIdx.x % QPR);
+        const Tin *p = src + base + min(c0 + c, inner - 4);
+        for (int j = threadIdx.x / QPR; j < span; j += STEP)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(sm + j * COLS + c)),
+                         "l"(p + (int64_t)clampi(l0 - r + j, 0, L - 1) * inner)
+                         : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        constexpr int STEP = kBT / COLS;
+        const int c = threadIdx.x % COLS;
+        const Tin *p = src + base + min(c0 + c, inner - 1);
+        for (int j0 = threadIdx.x / COLS; j0 < span; j0 += 8 * STEP) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (j0 + u * STEP < span) v[u] = to_f32(__ldg(p + (int64_t)clampi(l0 - r + j0 + u * STEP, 0, L - 1) * inner));
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (j0 + u * STEP < span) sm[(j0 + u * STEP) * COLS + c] = v[u];
+        }
+    }
+    __syncthreads();
+    const int cp = threadIdx.x % NC, g = threadIdx.x / NC;
+    const int64_t c = c0 + 2 * cp;
+    const int left = L - (l0 + g * kBK);
+    if (c >= inner || left <= 0) return;
+    const float *col = sm + g * kBK * COLS + 2 * cp;
+    float a[kBK], b[kBK];
+    const int64_t at = base + (int64_t)(l0 + g * kBK) * inner + c;
+    const bool two = c + 1 < inner, pair = (inner & 1) == 0 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0;
+    // minus (add_images_weighted(source, opening, 1, -1)): the source's values
+    // are on their way while the windows are computed
+    Ts sa[kBK], sb[kBK];
+    if (minus) {
+#pragma unroll
+        for (int k = 0; k < kBK; ++k) {
+            const int64_t i = at + (int64_t)min(k, left - 1) * inner;
+            sa[k] = __ldg(minus + i);
+            sb[k] = two ? __ldg(minus + i + 1) : Ts(0);
+        }
+    }
+    window8<MAX, kBK * COLS, COLS>(col, 2 * r + 1, a);
+    window8<MAX, kBK * COLS, COLS>(col + 1, 2 * r + 1, b);
+    if (minus) {
+#pragma unroll
+        for (int k = 0; k < kBK; ++k) {
+            a[k] = __fsub_rn(to_f32(sa[k]), a[k]);
+            b[k] = __fsub_rn(to_f32(sb[k]), b[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kBK; ++k)
+        if (k < left) {
+            const int64_t i = at + (int64_t)k * inner;
+            if (pair) {
+                *reinterpret_cast<float2 *>(dst + i) = make_float2(a[k], b[k]);
+            } else {
+                dst[i] = a[k];
+                if (two) dst[i + 1] = b[k];
+            }
+        }
+}
+
+constexpr int kMaxBoxRadius = 700;
+
+// src (x pass only: any source type) -> dst; axis 0 = x, 1 = y, 2 = z
+template <bool MAX, typename Tin, int NG, typename Ts>
+int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, int r, const Ts *minus, cudaStream_t st) {
+    constexpr int COLS = 2 * (kBT / NG), ROWS = NG * kBK;
+    auto kern = minmax_col_kernel<MAX, Tin, NG, Ts>;
+    const size_t smem = sizeof(float) * COLS * (size_t)(ROWS + 2 * r);
+    if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((L + ROWS - 1) / ROWS), (unsigned)outer);
+    const int vec = sizeof(Tin) == 4 && inner % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
+    kern<<<grid, kBT, smem, st>>>(src, dst, inner, L, r, vec, minus);
+    return CLE_OK;
+}
+
+template <bool MAX, typename Tin, typename Ts>
+int minmax_pass(const Tin *src, float *dst, const Img &im, int axis, int r, const Ts *minus, cudaStream_t st) {
     if (im.H > 65535 || im.D > 65535) { set_error("minimum/maximum box: image too large"); return CLE_ERR_TOO_LARGE; }
     if (axis == 0) {
         r = (int)std::min<int64_t>(r, im.W - 1);
-        const size_t smem = sizeof(float) * (kLX + 2 * r);
-        CLE_CUDA(cudaFuncSetAttribute(minmax_x_kernel<MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        minmax_x_kernel<MAX><<<dim3((unsigned)((im.W + kLX - 1) / kLX), (unsigned)im.H, (unsigned)im.D), kLX, smem,
-                               st>>>(src, dst, (int)im.W, r);
+        const int64_t rows = im.D * im.H;
+        const int tiles = (int)((im.W + kBRow - 1) / kBRow);
+        const int tile = (int)(((im.W + tiles - 1) / tiles + kBK - 1) / kBK * kBK);
+        // rows to fill the CTA's threads, as far as long windows fit 64 KB
+        const int pitch = ((tile + 2 * r) / kBK + 2) * kBPitch;
+        const int np = (int)std::max<size_t>(1, std::min<size_t>(std::min(kBT / (tile / kBK), 32), 65536 / (sizeof(float) * pitch)));
+        const size_t smem = sizeof(float) * (size_t)np * pitch;
+        auto kern = minmax_row_kernel<MAX, Tin>;
+        if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const int64_t ctas = (rows + np - 1) / np;
+        const dim3 grid((unsigned)((im.W + tile - 1) / tile), (unsigned)std::min<int64_t>(ctas, 65535),
+                        (unsigned)((ctas + 65534) / 65535));
+        kern<<<grid, kBT, smem, st>>>(src, dst, rows, (int)im.W, r, tile, np, FastDiv((uint32_t)(tile / kBK)));
     } else {
         const int64_t L = axis == 1 ? im.H : im.D;
         r = (int)std::min<int64_t>(r, L - 1);
-        if (r == 0) {
-            CLE_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-            return CLE_OK;
-        }
-        const int64_t S = axis == 1 ? im.W : im.H * im.W;
-        const int64_t other = axis == 1 ? im.D : im.H;
-        const int64_t OS = axis == 1 ? im.H * im.W : im.W;
-        const size_t smem = sizeof(float) * (size_t)(kLT + 2 * r) * kLC;
-        CLE_CUDA(cudaFuncSetAttribute(minmax_axis_kernel<MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        minmax_axis_kernel<MAX><<<dim3((unsigned)((im.W + kLC - 1) / kLC), (unsigned)((L + kLT - 1) / kLT),
-                                       (unsigned)other), dim3(kLC, 8), smem, st>>>(src, dst, (int)im.W, (int)L, S, OS, r);
+        const int64_t inner = axis == 1 ? im.W : im.H * im.W, outer = axis == 1 ? im.D : 1;
+        // short axes take fewer outputs and more columns per CTA
+        if (L <= 64 && r <= 64) CLE_TRY((launch_col<MAX, Tin, 8, Ts>(src, dst, inner, (int)L, outer, r, minus, st)));
+        else CLE_TRY((launch_col<MAX, Tin, 16, Ts>(src, dst, inner, (int)L, outer, r, minus, st)));
     }
     CLE_LAUNCH_CHECK("minimum/maximum box");
     return CLE_OK;
 }
 
-__global__ void to_f32_kernel_any_u8(const uint8_t *s, float *d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = s[i];
+template <typename Ts>
+__global__ void minus_kernel(const Ts *__restrict__ src, const float *v, float *d, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        d[i] = __fsub_rn(to_f32(src[i]), v[i]);
 }
-__global__ void to_f32_kernel_any_u16(const uint16_t *s, float *d, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = s[i];
+template <typename Ts>
+__global__ void to_f32_kernel(const Ts *__restrict__ s, float *__restrict__ d, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) d[i] = to_f32(s[i]);
 }
 
-__global__ void top_hat_sub_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ d,
-                                   int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        d[i] = __fsub_rn(a[i], b[i]);            // add_images_weighted(a, b, 1, -1)
+// A sequence of passes over the axes with r > 0, from `src` into `out` (not
+// aliasing it), through out and tmp in turn; `minus`: out = *minus - result.
+struct Step {
+    bool is_max;
+    int axis, r;
+};
+template <typename Ts>
+int run_steps(const Ts *src, float *out, float *tmp, const Img &im, const Step *steps, int n, const Ts *minus,
+              cudaStream_t st) {
+    const int64_t nv = im.n();
+    if (n == 0) {
+        to_f32_kernel<Ts><<<launch_blocks(nv, 256), 256, 0, st>>>(src, out, nv);
+        if (minus) minus_kernel<Ts><<<launch_blocks(nv, 256), 256, 0, st>>>(minus, out, out, nv);
+        CLE_LAUNCH_CHECK_N("minimum/maximum box", minus ? 2 : 1);
+        return CLE_OK;
+    }
+    const float *cur = nullptr;
+    for (int i = 0; i < n; ++i) {
+        // the last pass lands in out
+        float *o = ((n - 1 - i) & 1) ? tmp : out;
+        // a y or z pass can subtract; an x pass is followed by a pass that does
+        const Ts *m = i == n - 1 && steps[i].axis != 0 ? minus : nullptr;
+        if (i == 0) CLE_TRY(steps[i].is_max ? minmax_pass<true>(src, o, im, steps[i].axis, steps[i].r, m, st)
+                                            : minmax_pass<false>(src, o, im, steps[i].axis, steps[i].r, m, st));
+        else CLE_TRY(steps[i].is_max ? minmax_pass<true>(cur, o, im, steps[i].axis, steps[i].r, m, st)
+                                     : minmax_pass<false>(cur, o, im, steps[i].axis, steps[i].r, m, st));
+        cur = o;
+    }
+    if (minus && steps[n - 1].axis == 0) {
+        minus_kernel<Ts><<<launch_blocks(nv, 256), 256, 0, st>>>(minus, out, out, nv);
+        CLE_LAUNCH_CHECK("top_hat_box");
+    }
+    return CLE_OK;
 }
 
 }  // namespace
 
 size_t box_filter_workspace_bytes(const Img &im) {
     Arena a(nullptr, 0);
-    a.take<float>(im.n());      // source as float32 (u8/u16 sources)
+    a.take<float>(im.n());      // the source of an in-place call
     a.take<float>(im.n());      // pass temporary
-    a.take<float>(im.n());      // second temporary (top-hat opening)
     return a.off;
-}
-
-// min (MAX=false) or max box of `in` (float32) into `out` (not aliasing `in`);
-// tmp: n floats
-template <bool MAX>
-static int box3(const float *in, float *out, float *tmp, const Img &im, const int r[3], cudaStream_t st) {
-    if (im.ndim == 3) {                // x -> out, y -> tmp, z -> out
-        CLE_TRY(minmax_pass<MAX>(in, out, im, 0, r[0], st));
-        CLE_TRY(minmax_pass<MAX>(out, tmp, im, 1, r[1], st));
-        return minmax_pass<MAX>(tmp, out, im, 2, r[2], st);
-    }
-    CLE_TRY(minmax_pass<MAX>(in, tmp, im, 0, r[0], st));   // x -> tmp, y -> out
-    return minmax_pass<MAX>(tmp, out, im, 1, r[1], st);
 }
 
 static int radii(const Img &im, double rx, double ry, double rz, int r[3]) {
@@ -246,60 +430,51 @@ static int radii(const Img &im, double rx, double ry, double rz, int r[3]) {
     return CLE_OK;
 }
 
-// The source as float32: in place when it is float32 and not the destination,
-// else converted / copied into the workspace.
-static int float_source(const Img &src, const Img &dst, Arena &ws, const float **out, cudaStream_t st) {
-    float *f = ws.take<float>(src.n());
-    if (src.dtype == CLE_F32 && src.data != dst.data) { *out = (const float *)src.data; return CLE_OK; }
-    if (src.dtype == CLE_F32) {
-        if (f) CLE_CUDA(cudaMemcpyAsync(f, src.data, sizeof(float) * src.n(), cudaMemcpyDeviceToDevice, st));
-        *out = f;
-        return CLE_OK;
+// minimum_box / maximum_box (hat: top_hat_box, source - maximum(minimum)); the
+// passes with r > 0 along x, y (, z), for top_hat_box the minima then the maxima
+template <typename Ts>
+static int box_typed(const Img &src, float *dst, const int r[3], bool is_max, bool hat, Arena &ws, cudaStream_t st) {
+    const int64_t n = src.n();
+    float *copy = ws.take<float>(n);
+    float *tmp = ws.take<float>(n);
+    if (!ws.ok()) { set_error("minimum/maximum box: workspace too small"); return CLE_ERR_WORKSPACE; }
+    if (n == 0) return CLE_OK;
+    const Ts *in = (const Ts *)src.data;
+    if (src.data == (void *)dst) {   // float32 in place
+        CLE_CUDA(cudaMemcpyAsync(copy, src.data, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+        in = (const Ts *)copy;
     }
-    const int b = launch_blocks(src.n(), 256);
-    if (src.dtype == CLE_U8) to_f32_kernel_any_u8<<<b, 256, 0, st>>>((const uint8_t *)src.data, f, src.n());
-    else if (src.dtype == CLE_U16) to_f32_kernel_any_u16<<<b, 256, 0, st>>>((const uint16_t *)src.data, f, src.n());
-    else { set_error("box filter: unsupported source dtype %d", src.dtype); return CLE_ERR_DTYPE; }
-    CLE_LAUNCH_CHECK("to float32");
-    *out = f;
-    return CLE_OK;
+    Step steps[6];
+    int k = 0;
+    const int64_t len[3] = {src.W, src.H, src.D};
+    for (int p = 0; p < (hat ? 2 : 1); ++p)
+        for (int a = 0; a < src.ndim; ++a)
+            if (r[a] > 0 && len[a] > 1) steps[k++] = {hat ? p == 1 : is_max, a, r[a]};
+    return run_steps<Ts>(in, dst, tmp, src, steps, k, hat ? in : nullptr, st);
+}
+
+static int box_any(const Img &src, const Img &dst, double rx, double ry, double rz, bool is_max, bool hat, const char *name,
+                   Arena &ws, cudaStream_t st) {
+    CLE_TRY(same_shape(src, dst, "source", "destination"));
+    if (dst.dtype != CLE_F32) { set_error("%s: destination must be float32", name); return CLE_ERR_DTYPE; }
+    int r[3];
+    CLE_TRY(radii(src, rx, ry, rz, r));
+    switch (src.dtype) {
+        case CLE_F32: return box_typed<float>(src, (float *)dst.data, r, is_max, hat, ws, st);
+        case CLE_U16: return box_typed<uint16_t>(src, (float *)dst.data, r, is_max, hat, ws, st);
+        case CLE_U8: return box_typed<uint8_t>(src, (float *)dst.data, r, is_max, hat, ws, st);
+        default: set_error("box filter: unsupported source dtype %d", src.dtype); return CLE_ERR_DTYPE;
+    }
 }
 
 int box_filter(const Img &src, const Img &dst, double rx, double ry, double rz, bool is_max, Arena &ws,
                cudaStream_t st) {
-    CLE_TRY(same_shape(src, dst, "source", "destination"));
-    if (dst.dtype != CLE_F32) { set_error("minimum/maximum box: destination must be float32"); return CLE_ERR_DTYPE; }
-    int r[3];
-    CLE_TRY(radii(src, rx, ry, rz, r));
-    const float *in = nullptr;
-    CLE_TRY(float_source(src, dst, ws, &in, st));
-    float *tmp = ws.take<float>(src.n());
-    if (!ws.ok()) { set_error("minimum/maximum box: workspace too small"); return CLE_ERR_WORKSPACE; }
-    if (src.n() == 0) return CLE_OK;
-    return is_max ? box3<true>(in, (float *)dst.data, tmp, src, r, st)
-                  : box3<false>(in, (float *)dst.data, tmp, src, r, st);
+    return box_any(src, dst, rx, ry, rz, is_max, false, "minimum/maximum box", ws, st);
 }
 
 // top_hat_box: _tier2/_top_hat_box.py:37-43
 int top_hat_box(const Img &src, const Img &dst, double rx, double ry, double rz, Arena &ws, cudaStream_t st) {
-    CLE_TRY(same_shape(src, dst, "source", "destination"));
-    if (dst.dtype != CLE_F32) { set_error("top_hat_box: destination must be float32"); return CLE_ERR_DTYPE; }
-    int r[3];
-    CLE_TRY(radii(src, rx, ry, rz, r));
-    const float *in = nullptr;
-    CLE_TRY(float_source(src, dst, ws, &in, st));
-    float *tmp = ws.take<float>(src.n());
-    float *open_ = ws.take<float>(src.n());
-    if (!ws.ok()) { set_error("top_hat_box: workspace too small"); return CLE_ERR_WORKSPACE; }
-    const int64_t n = src.n();
-    if (n == 0) return CLE_OK;
-    float *d = (float *)dst.data;
-    // opening: maximum_box(minimum_box(src)) into open_ (dst serves as a temporary)
-    CLE_TRY(box3<false>(in, d, tmp, src, r, st));
-    CLE_TRY(box3<true>(d, open_, tmp, src, r, st));
-    top_hat_sub_kernel<<<launch_blocks(n, 256), 256, 0, st>>>(in, open_, d, n);
-    CLE_LAUNCH_CHECK("top_hat_box");
-    return CLE_OK;
+    return box_any(src, dst, rx, ry, rz, false, true, "top_hat_box", ws, st);
 }
 
 int erode_box(const Img &src, const Img &dst, cudaStream_t st) {

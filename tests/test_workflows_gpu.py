@@ -223,6 +223,22 @@ def test_box_filters_match_oracle(cle, oracle, shape, radii):
     assert np.array_equal(cle.pull(cle.top_hat_box(a, None, *radii)), oracle.top_hat_box(a, *radii))
 
 
+# windows below, at and above the 8 outputs of a thread (r = 3, 4), windows longer
+# than the axis, one axis alone, axes with remainders of the CTA's 64 / 128 outputs,
+# vector and scalar staging, sources in their own type (min / max are exact)
+@pytest.mark.parametrize("shape", [(1, 1), (9, 300), (70, 64), (3, 5, 8), (65, 9, 36), (66, 130, 33), (20, 129, 260)])
+@pytest.mark.parametrize("radii", [(3, 3, 3), (4, 4, 4), (0, 3, 4), (5, 0, 0), (0, 0, 12), (13, 40, 2), (90, 1, 70), (0, 0, 0)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_box_filter_windows(cle, oracle, shape, radii, dtype):
+    r = np.random.default_rng(8)
+    a = (r.integers(0, np.iinfo(dtype).max, size=shape) if dtype != np.float32
+         else r.uniform(-1000, 1000, size=shape)).astype(dtype)
+    f = a.astype(np.float32)
+    assert np.array_equal(cle.pull(cle.minimum_box(a, None, *radii)), oracle.minimum_box(f, *radii))
+    assert np.array_equal(cle.pull(cle.maximum_box(a, None, *radii)), oracle.maximum_box(f, *radii))
+    assert np.array_equal(cle.pull(cle.top_hat_box(a, None, *radii)), oracle.top_hat_box(f, *radii))
+
+
 @pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
 def test_top_hat_box_narrow_input_and_in_place(cle, oracle, dtype):
     a = np.random.default_rng(9).integers(0, np.iinfo(dtype).max, (13, 70, 61)).astype(dtype)
