@@ -99,24 +99,21 @@ def config_of(name, nvox):
 
 # Algorithmic bytes per voxel of each stage (each input read once, each
 # output written once; uint16 source).  Index = stage event interval.
-STAGES = ["blur_spot", "detect_maxima", "blur_outline", "minmax_hist_otsu", "threshold_seeds",
-          "seed_ccl", "voronoi_growth", None, "stats_pass1", "stats_final1", "stats_pass2",
-          "stats_final2"]
-ALGO_BYTES = {"blur_spot": 2 + 4, "detect_maxima": 4 + 1, "blur_outline": 2 + 4,
-              "minmax_hist_otsu": 4 + 4, "threshold_seeds": 4 + 1 + 1 + 4,
+STAGES = ["blur_outline", "hist_otsu", "blur_spot", "maxima_seeds", "seed_ccl", "voronoi_growth", None,
+          None, "stats_pass1", "stats_final1", "stats_pass2", "stats_final2"]
+ALGO_BYTES = {"blur_outline": 2 + 4, "hist_otsu": 4, "blur_spot": 2 + 4, "maxima_seeds": 4 + 4 + 1 + 4,
               "voronoi_growth": 1 + 1 + 4, "stats_pass1": 4 + 2, "stats_pass2": 4 + 2}
 
 
 def algo_bytes(w, labelled_fraction=None):
-    """ALGO_BYTES for a workload: with equal spot and outline sigmas the blur
-    runs once (its stage carries the min / max) and the maxima are found in
-    the seed pass (read T, write the mask and the labels; no spots image, no
-    second blur).  The second statistics pass reads the label and intensity
-    of labelled voxels only."""
+    """ALGO_BYTES for a workload: the seed pass finds the maxima (reads both
+    blurs, writes the mask and the labels); with equal spot and outline sigmas
+    there is one blur.  The second statistics pass reads the label and
+    intensity of labelled voxels only."""
     b = dict(ALGO_BYTES)
     if w.get("spot") is not None and w.get("spot") == w.get("outline"):
-        b["threshold_seeds"] = 4 + 1 + 4
-        del b["detect_maxima"], b["blur_outline"]
+        b["maxima_seeds"] = 4 + 1 + 4
+        del b["blur_spot"]
     if labelled_fraction is not None:
         b["stats_pass2"] = (4 + 2) * labelled_fraction
     return b
@@ -131,19 +128,11 @@ PIPELINE_BYTES_PER_VOXEL = 8 + 4 + 10 + 6 + 8
 # dram__bytes_write.sum, or the DRAM bandwidth x the duration of the same
 # launch); the captures are summarised in profiles/<kernel>_<workload>.md.
 MEASURED_TRAFFIC = {
-    "nuclei": {"voronoi_growth": (0.347e9, "voronoi_keys_kernel_nuclei_128x512x512.md"),
-               "blur_spot": (67.164e6 + 81.208e6, "blur_fused_kernel_nuclei_128x512x512.md"),
-               "blur_outline": (67.155e6 + 81.081e6, "blur_fused_kernel_nuclei_128x512x512.md"),
-               "detect_maxima": (135.090e6 + 19.932e6, "maxima_kernel_nuclei_128x512x512.md"),
-               },
+    "nuclei": {"voronoi_growth": (0.347e9, "voronoi_keys_kernel_nuclei_128x512x512.md")},
     # slab captures (128x1024x1024) scaled by 4 to the 512x1024x1024 volume:
     # the same recipe and cell density, traffic in proportion to the voxels
-    "lightsheet": {"voronoi_growth": (4 * 1.494e9, "voronoi_keys_kernel_lightsheet_slab_128x1024x1024.md"),
-                   "blur_spot": (4 * 0.792e9, "blur_fused_kernel_lightsheet_slab_128x1024x1024.md"),
-                   "threshold_seeds": (4 * 1.165e9, "maxima_seeds_kernel_lightsheet_slab_128x1024x1024.md")},
-    "lightsheet_slab": {"voronoi_growth": (1.494e9, "voronoi_keys_kernel_lightsheet_slab_128x1024x1024.md"),
-                        "blur_spot": (0.792e9, "blur_fused_kernel_lightsheet_slab_128x1024x1024.md"),
-                        "threshold_seeds": (1.165e9, "maxima_seeds_kernel_lightsheet_slab_128x1024x1024.md")},
+    "lightsheet": {"voronoi_growth": (4 * 1.494e9, "voronoi_keys_kernel_lightsheet_slab_128x1024x1024.md")},
+    "lightsheet_slab": {"voronoi_growth": (1.494e9, "voronoi_keys_kernel_lightsheet_slab_128x1024x1024.md")},
 }
 
 # Algorithmic bytes per voxel of a whole gauss_otsu_labeling + statistics step

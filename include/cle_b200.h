@@ -103,9 +103,9 @@ unsigned long long cle_kernel_launches(void);
  * calls).  0 turns profiling off.
  * cle_profile_stage_ms() waits for the last recorded event and writes the
  * elapsed milliseconds between consecutive events (returns how many).
- * Events 0-7 (voronoi_otsu_labeling): blur(spot) | detect_maxima |
- * blur(outline) | min/max+histogram+Otsu | threshold+seeds | seed CCL |
- * Voronoi growth; events 8-12 (statistics): pass 1 | finalise 1 | pass 2 |
+ * Events 0-7 (voronoi_otsu_labeling): blur(outline) with min/max | histogram +
+ * Otsu | blur(spot) (empty with equal sigmas) | maxima + seeds | seed CCL |
+ * Voronoi growth | (empty); events 8-12 (statistics): pass 1 | finalise 1 | pass 2 |
  * finalise 2.  Interval 7 (between the two ops) is host time. */
 int cle_profile_enable(int flags);
 int cle_profile_stage_ms(float *out, int max);

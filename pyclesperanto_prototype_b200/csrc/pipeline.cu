@@ -1,16 +1,16 @@
 // pipeline.cu -- voronoi_otsu_labeling (_tier9/_voronoi_otsu_labeling.py:49-73) as one
 // stream-ordered sequence with no host round trip:
-//   T = gaussian_blur(src, spot_sigma)            (blur.cu)
-//   spots = detect_maxima_box(T)                  (maxima.cu; mean_box r=0 is a copy)
-//   T = gaussian_blur(src, outline_sigma)
-//   {min,max} -> histogram -> Otsu -> t32         (reduce.cu, all on the device)
-//   seg = T > t32; seeds = spots & seg            (seed kernel below; emits the seed list
-//                                                  and the seeds' initial CCL keys)
+//   O = gaussian_blur(src, outline_sigma), {min, max}   (blur_fused.cu, blur.cu)
+//   histogram -> Otsu -> t32                      (reduce.cu, all on the device)
+//   T = gaussian_blur(src, spot_sigma)            (O itself when the sigmas are equal)
+//   seg = O > t32; seeds = detect_maxima_box(T) & seg   (maxima.cu, one pass; emits the
+//                                                  seed list and the initial CCL keys;
+//                                                  mean_box r=0 is a copy)
 //   labels(seeds) = CCL                           (ccl.cu, list form)
 //   labels = masked Voronoi growth inside seg     (voronoi.cu, frontier form)
 // The label output buffer is the CCL parent store and the Voronoi state, so
-// the only full-size scratch is T (f32), spots/seg (u8), the seed list and
-// the two frontier arrays (which also serve as the blur's temporaries).
+// the only full-size scratch is O (f32), seg (u8), the seed list and a tail the
+// phases share: the blurs' temporaries, the spot blur, the growth's lists.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -29,39 +29,6 @@ struct Scalars {
     double thr;
     float hist[256];
 };
-
-__global__ void seeds_kernel(const float *__restrict__ T, const uint8_t *__restrict__ spots,
-                             const float *__restrict__ d_thr32, Geo g, int64_t n,
-                             uint8_t *__restrict__ seg, uint32_t *__restrict__ lab,
-                             uint32_t *__restrict__ seeds, uint32_t *__restrict__ d_count) {
-    const float t = *d_thr32;
-    const int lane = threadIdx.x & 31;
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n;
-         base += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        bool s = false, seed = false;
-        uint32_t key = 0;
-        if (i < n) {
-            s = T[i] > t;
-            seed = s && spots[i] != 0;
-            if (seed) {
-                uint32_t x, y, z;
-                m2xyz(g, (uint32_t)i, x, y, z);
-                key = xyz2k(g, x, y, z) + 1u;
-            }
-            seg[i] = s ? kMaskByte : 0;
-            lab[i] = key;
-        }
-        const unsigned b = __ballot_sync(0xffffffffu, seed);
-        if (b) {
-            uint32_t base_pos = 0;
-            const int leader = __ffs(b) - 1;
-            if (lane == leader) base_pos = atomicAdd(d_count, (uint32_t)__popc(b));
-            base_pos = __shfl_sync(0xffffffffu, base_pos, leader);
-            if (seed) seeds[base_pos + __popc(b & ((1u << lane) - 1u))] = (uint32_t)i;
-        }
-    }
-}
 
 // Seeds of masked_voronoi_labeling with a 0/1 mask: seg = mask != 0,
 // seed = binary != 0 inside the mask; seeds get their CCL key and are listed.
@@ -105,8 +72,8 @@ __global__ void u32_to_f32(const uint32_t *__restrict__ s, float *__restrict__ d
 
 struct Layout {
     Scalars *sc;
-    float *T;
-    uint8_t *spots, *seg;
+    float *O;
+    uint8_t *seg;
     uint32_t *seeds;
     size_t fixed_end;
 };
@@ -114,8 +81,7 @@ struct Layout {
 Layout take_layout(Arena &a, const Img &im) {
     Layout l;
     l.sc = a.take<Scalars>(1);
-    l.T = a.take<float>(im.n());
-    l.spots = a.take<uint8_t>(im.n());
+    l.O = a.take<float>(im.n());
     l.seg = a.take<uint8_t>(im.n());
     l.seeds = a.take<uint32_t>(im.n());
     l.fixed_end = a.off;
@@ -392,66 +358,59 @@ int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma, dou
     stage_mark(0, st);
     CLE_CUDA(cudaMemsetAsync(l.sc, 0, sizeof(Scalars), st));
 
-    // 1-3: blurs and maxima (the blur's temporaries live in the tail).  The
-    // two blurs build their taps from the float32 sigma and the kernel size
-    // int(8 sigma)|1, so equal float32 sigmas with equal kernel sizes give the
-    // same image bit for bit: then it is computed once (with the min / max the
-    // outline blur reduces) and serves both the spot detection and the
-    // threshold, as the reference's second blur would have recomputed it.
+    // 1: the outline blur with its min / max (temporaries in the tail), 2: the
+    // threshold, on the device
+    CLE_TRY(blur_minmax(src, l.O, outline_sigma, &l.sc->mm, ws, st, &l.sc->status));
+    ws.off = tail_off;
+    stage_mark(1, st);
+    Img Oi = src;
+    Oi.data = l.O;
+    Oi.dtype = CLE_F32;
+    CLE_TRY(histogram_otsu(Oi, l.sc->mm.out, l.sc->hist, &l.sc->thr, &l.sc->thr32, ws, st));
+    ws.off = tail_off;
+    stage_mark(2, st);
+
+    // 3: the spot blur.  The two blurs build their taps from the float32 sigma
+    // and the kernel size int(8 sigma)|1, so equal float32 sigmas with equal
+    // kernel sizes give the same image bit for bit: then the outline blur serves
+    // both the spot detection and the threshold.  Otherwise the spot blur goes to
+    // the tail: to the second of the three-pass blur's temporaries in 2D (its
+    // last pass reads the first) and to the first in 3D (it reads the second).
     const bool same_blur = (float)spot_sigma == (float)outline_sigma &&
                            sigma_to_kernel_size(spot_sigma) == sigma_to_kernel_size(outline_sigma);
-    if (same_blur) CLE_TRY(blur_minmax(src, l.T, spot_sigma, &l.sc->mm, ws, st, &l.sc->status));
-    else CLE_TRY(gaussian_blur(src, l.T, spot_sigma, spot_sigma, spot_sigma, ws, st, &l.sc->status));
-    stage_mark(1, st);
-    ws.off = tail_off;
-    Img Ti = src;
-    Ti.data = l.T;
-    Ti.dtype = CLE_F32;
-    Img Si = src;
-    Si.data = l.spots;
-    Si.dtype = CLE_U8;
-    // with one blur the maxima are found in the seed pass below (the spots
-    // image is never stored)
-    if (!same_blur) CLE_TRY(detect_maxima(Ti, Si, st));
-    stage_mark(2, st);
-    // the outline blur also reduces the blurred image's min / max (step 4)
-    if (!same_blur) CLE_TRY(blur_minmax(src, l.T, outline_sigma, &l.sc->mm, ws, st, &l.sc->status));
-    ws.off = tail_off;
+    Img Ti = Oi;
+    if (!same_blur) {
+        float *t1 = ws.take<float>(n), *t2 = ws.take<float>(n);
+        ws.off = tail_off;
+        Ti.data = src.ndim == 3 ? t1 : t2;
+        CLE_TRY(gaussian_blur(src, (float *)Ti.data, spot_sigma, spot_sigma, spot_sigma, ws, st, &l.sc->status));
+        ws.off = tail_off;
+    }
     stage_mark(3, st);
 
-    // 4-6: threshold on the device
-    CLE_TRY(histogram_otsu(Ti, l.sc->mm.out, l.sc->hist, &l.sc->thr, &l.sc->thr32, ws, st));
-    ws.off = tail_off;
+    // 4: segmentation, maxima, seeds, seed keys
+    uint32_t *lab = (dst.dtype == CLE_U32) ? (uint32_t *)dst.data : (uint32_t *)l.O;
+    const Geo g = make_geo(src);
+    const float *O = l.O;
+    if (dst.dtype == CLE_F32) {
+        // the labels are built in O's buffer; the seed pass reads a copy in dst
+        CLE_CUDA(cudaMemcpyAsync(dst.data, l.O, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+        O = (const float *)dst.data;
+        if (same_blur) Ti.data = dst.data;
+    }
+    CLE_TRY(maxima_seeds(Ti, O, &l.sc->thr32, l.seg, lab, l.seeds, &l.sc->seed_count, st));
     stage_mark(4, st);
 
-    // 7: segmentation, seeds, seed keys
-    uint32_t *lab = (dst.dtype == CLE_U32) ? (uint32_t *)dst.data : (uint32_t *)l.T;
-    const Geo g = make_geo(src);
-    const float *Tsrc = l.T;
-    if (dst.dtype == CLE_F32) {
-        // the labels are built in T's buffer; the seed pass reads a copy in dst
-        CLE_CUDA(cudaMemcpyAsync(dst.data, l.T, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
-        Tsrc = (const float *)dst.data;
-    }
-    if (same_blur) {
-        Img Tc = Ti;
-        Tc.data = (void *)Tsrc;
-        CLE_TRY(maxima_seeds(Tc, &l.sc->thr32, l.seg, lab, l.seeds, &l.sc->seed_count, st));
-    } else {
-        seeds_kernel<<<launch_blocks(n, 256), 256, 0, st>>>(Tsrc, l.spots, &l.sc->thr32, g, n, l.seg, lab, l.seeds, &l.sc->seed_count);
-        CLE_LAUNCH_CHECK("seeds");
-    }
-    stage_mark(5, st);
-
-    // 8: label the seeds
+    // 5: label the seeds
     CLE_TRY(ccl_list(g, n, lab, l.seeds, &l.sc->seed_count, n, ws, st, &l.sc->nlabels));
     ws.off = tail_off;
-    stage_mark(6, st);
+    stage_mark(5, st);
 
-    // 9: grow inside the segmentation
+    // 6: grow inside the segmentation
     CLE_TRY(voronoi_grow(src, lab, l.seg, l.seeds, &l.sc->seed_count, &l.sc->nlabels, &l.sc->status, ws, st,
                          lim));
     ws.off = tail_off;
+    stage_mark(6, st);
     stage_mark(7, st);
 
     if (dst.dtype == CLE_F32) {
