@@ -184,6 +184,25 @@ def test_histogram_smooth_image_exact(cle, oracle, shape, bins):
     assert np.array_equal(h, oracle.histogram(a, bins))
 
 
+@pytest.mark.parametrize("bins", [2, 255, 256, 257])
+@pytest.mark.parametrize("lo,hi", [(0.0, 510.0), (-3.7, 1.3e-2), (1e-38, 3e-38), (-1e30, 2.5e36), (7.0, 7.0)])
+@pytest.mark.parametrize("width", [1, 64, 67])
+def test_histogram_beside_bin_edges_exact(cle, oracle, bins, lo, hi, width):
+    # every edge of a bin and up to 3 representable values to each side of it,
+    # where the reciprocal's bin may not be taken for the quotient's
+    lo, hi = np.float32(lo), np.float32(hi)
+    e = (lo.astype(np.float64) + (np.arange(bins + 1) - 0.5) * (np.float64(hi) - lo) / (bins - 1)).astype(np.float32)
+    vals, up, down = [e], e, e
+    for _ in range(3):
+        up, down = np.nextafter(up, np.float32(np.inf)), np.nextafter(down, np.float32(-np.inf))
+        vals += [up, down]
+    v = np.concatenate(vals)
+    a = np.resize(v, (2, -(-v.size // (2 * width)), width)).astype(np.float32)
+    h = cle.pull(cle.histogram(a, num_bins=bins, minimum_intensity=float(lo), maximum_intensity=float(hi),
+                               determine_min_max=False))
+    assert np.array_equal(h, oracle.histogram(a, bins, float(lo), float(hi)))
+
+
 @pytest.mark.parametrize("bins", [256, 9])
 def test_histogram_nan_inf_given_range(cle, oracle, bins):
     # NaN / +-inf voxels among plateaus of equal values, with the range given
