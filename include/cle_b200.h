@@ -335,6 +335,13 @@ int cle_voronoi_labeling(const cle_tensor *binary, const cle_tensor *dst,
                          const cle_call_options *options, void *workspace,
                          size_t workspace_bytes, void *stream);
 
+/* ---- gauss_otsu_labeling -----------------------------------------------
+ * replaces _tier9/_gauss_otsu_labeling.py:6-45: gaussian_blur, threshold_otsu,
+ * connected_components_labeling_box.  src: u8/u16/f32; dst: u32 or f32. */
+size_t cle_gauss_otsu_labeling_workspace_bytes(const cle_tensor *src);
+int cle_gauss_otsu_labeling(const cle_tensor *src, const cle_tensor *dst, double outline_sigma,
+                            void *workspace, size_t workspace_bytes, void *stream);
+
 /* ---- voronoi_otsu_labeling ---------------------------------------------
  * replaces _tier9/_voronoi_otsu_labeling.py:11-73.  src: u8/u16/f32 (u8 and
  * u16 are converted on the fly, exactly as push's float32 cast would);

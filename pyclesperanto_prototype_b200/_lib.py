@@ -138,6 +138,8 @@ _SIGS = {
     "cle_voronoi_labeling": (ctypes.c_int, [_T, _T, _O, _P, _SZ, _P]),
     "cle_masked_voronoi_labeling_binary_workspace_bytes": (_SZ, [_T]),
     "cle_masked_voronoi_labeling_binary": (ctypes.c_int, [_T, _T, _T, _O, _P, _SZ, _P]),
+    "cle_gauss_otsu_labeling_workspace_bytes": (_SZ, [_T]),
+    "cle_gauss_otsu_labeling": (ctypes.c_int, [_T, _T, ctypes.c_double, _P, _SZ, _P]),
     "cle_voronoi_otsu_labeling_workspace_bytes": (_SZ, [_T]),
     "cle_voronoi_otsu_labeling": (ctypes.c_int, [_T, _T, ctypes.c_double, ctypes.c_double, _O, _P, _SZ, _P]),
     "cle_vol_batch_plan": (ctypes.c_int, [_T, ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_int, _O,

@@ -733,12 +733,13 @@ def erode_box(source: Image, destination: Image = None) -> Image:
 def gauss_otsu_labeling(source: Image, label_image_destination: Image = None,
                         outline_sigma: float = 2) -> Image:
     """Gaussian blur, Otsu threshold, connected components (box) of the binary
-    image (_tier9/_gauss_otsu_labeling.py:6-45); every step a device kernel,
-    no host round trip."""
-    temp = create(source)                       # float32, like the reference's create(source)
-    gaussian_blur(source, temp, outline_sigma, outline_sigma, outline_sigma)
-    segmentation = threshold_otsu(temp)
-    return connected_components_labeling_box(segmentation, label_image_destination)
+    image (_tier9/_gauss_otsu_labeling.py:6-45); one stream-ordered call, no
+    host round trip."""
+    s, d = _T(source), _T(label_image_destination)
+    ws = _ws("cle_gauss_otsu_labeling_workspace_bytes", _lib.ref(s))
+    _call("cle_gauss_otsu_labeling", _lib.ref(s), _lib.ref(d), float(outline_sigma), _ptr(ws), ws.numel(),
+          _lib.stream_ptr())
+    return label_image_destination
 
 
 @plugin_function(categories=['label', 'in assistant'], output_creator=create_labels_like,

@@ -497,6 +497,24 @@ int cle_masked_voronoi_labeling_binary(const cle_tensor *bin, const cle_tensor *
     return masked_voronoi_binary(a, m, d, ar, S(stream), lim);
 }
 
+// ---- gauss_otsu_labeling ------------------------------------------------------------
+size_t cle_gauss_otsu_labeling_workspace_bytes(const cle_tensor *src) {
+    Img im;
+    if (to_img(src, im, "source")) return 0;
+    return gauss_otsu_workspace_bytes(im);
+}
+
+int cle_gauss_otsu_labeling(const cle_tensor *src, const cle_tensor *dst, double outline_sigma, void *ws,
+                            size_t ws_bytes, void *stream) {
+    Img a, d;
+    CLE_TRY(to_img(src, a, "source"));
+    CLE_TRY(to_img(dst, d, "label_image_destination"));
+    CLE_TRY(ws_check(ws, ws_bytes, gauss_otsu_workspace_bytes(a), "gauss_otsu_labeling"));
+    CLE_TRY(set_device_of(a, src));
+    Arena ar(ws, ws_bytes);
+    return gauss_otsu_labeling(a, d, outline_sigma, ar, S(stream));
+}
+
 // ---- voronoi_otsu_labeling ----------------------------------------------------------
 size_t cle_voronoi_otsu_labeling_workspace_bytes(const cle_tensor *src) {
     Img im;

@@ -177,12 +177,25 @@ __device__ __forceinline__ uint32_t via_row(int k, const uint32_t (&q)[4]) {
     return k == 2 ? q[0] : q[2];
 }
 
+// Foreground: what is not zero, or what lies above a threshold on the device (a
+// blurred image is labelled without its binary image being written and read).
+template <typename T>
+struct NonZero {
+    using Value = T;
+    __device__ __forceinline__ bool operator()(T v) const { return v != T(0); }
+};
+struct Above {
+    using Value = float;
+    const float *threshold;
+    __device__ __forceinline__ bool operator()(float v) const { return v > __ldg(threshold); }
+};
+
 // A tile of 32 x TY x TZ voxels per CTA: lab = compact id + 1 of the voxel's
 // component in the tile (0: background), bits = the row masks, parent[id] = id,
 // minkey[id] = the component's smallest key.
-template <typename T, int TY, int TZ, bool DIAMOND>
+template <typename FG, int TY, int TZ, bool DIAMOND>
 __global__ void __launch_bounds__(kTileThreads, 6)
-ccl_tile_kernel(const T *bin, uint32_t *lab, uint32_t *__restrict__ bits, uint32_t *__restrict__ parent,
+ccl_tile_kernel(const typename FG::Value *bin, FG fg, uint32_t *lab, uint32_t *__restrict__ bits, uint32_t *__restrict__ parent,
                 uint32_t *__restrict__ minkey, uint32_t *__restrict__ d_count, Geo g, Tiles t) {
     constexpr int ROWS = TY * TZ, WARPS = kTileThreads / 32, RPW = ROWS / WARPS, PARTS = kTileThreads / ROWS;
     static_assert(ROWS % WARPS == 0 && kTileThreads % ROWS == 0, "rows per warp and threads per row");
@@ -200,12 +213,17 @@ ccl_tile_kernel(const T *bin, uint32_t *lab, uint32_t *__restrict__ bits, uint32
     const uint32_t nrow = z < g.D && y0 < g.H ? min((uint32_t)RPW, g.H - y0) : 0u;   // rows inside the image
     const uint32_t at0 = (z * g.H + y0) * g.W + x, bit0 = (z * g.H + y0) * t.ws + tx;
     const bool xin = x < g.W;
-    T v[RPW];
-    bool some = false;
+    typename FG::Value v[RPW];
+    bool in[RPW], some = false;
 #pragma unroll
     for (int k = 0; k < RPW; ++k) {
-        v[k] = (uint32_t)k < nrow && xin ? bin[at0 + (uint32_t)k * g.W] : T(0);
-        some |= v[k] != T(0);
+        in[k] = (uint32_t)k < nrow && xin;
+        v[k] = in[k] ? bin[at0 + (uint32_t)k * g.W] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < RPW; ++k) {
+        in[k] = in[k] && fg(v[k]);
+        some |= in[k];
     }
     if (!__syncthreads_or(some)) {
         // nothing here (most tiles of a sparse mask)
@@ -221,7 +239,7 @@ ccl_tile_kernel(const T *bin, uint32_t *lab, uint32_t *__restrict__ bits, uint32
 #pragma unroll
     for (int k = 0; k < RPW; ++k) {
         const uint32_t r = r0 + (uint32_t)k;
-        const uint32_t m = __ballot_sync(0xffffffffu, v[k] != T(0));
+        const uint32_t m = __ballot_sync(0xffffffffu, in[k]);
         if (lane == 0) {
             mask[r] = m;
             if ((uint32_t)k < nrow) bits[bit0 + (uint32_t)k * t.ws] = m;
@@ -636,8 +654,8 @@ Dense take_dense(Arena &ws, const Img &im, bool diamond) {
     return d;
 }
 
-template <typename T, int TY, int TZ, bool DIAMOND>
-int dense_tiles(const Img &bin, uint32_t *lab, const Dense &d, const Geo &g, cudaStream_t st) {
+template <typename FG, int TY, int TZ, bool DIAMOND>
+int dense_tiles(const Img &bin, FG fg, uint32_t *lab, const Dense &d, const Geo &g, cudaStream_t st) {
     Tiles t;
     t.nx = t.ws = (uint32_t)((bin.W + 31) / 32);
     t.ny = (uint32_t)((bin.H + TY - 1) / TY);
@@ -645,19 +663,24 @@ int dense_tiles(const Img &bin, uint32_t *lab, const Dense &d, const Geo &g, cud
     t.fnx = FastDiv(t.nx);
     t.fny = FastDiv(t.ny);
     const uint32_t nseg = (uint32_t)(bin.D * bin.H) * t.ws;
-    ccl_tile_kernel<T, TY, TZ, DIAMOND><<<t.nx * t.ny * t.nz, kTileThreads, 0, st>>>(
-        (const T *)bin.data, lab, d.bits, d.parent, d.minkey, d.count, g, t);
+    ccl_tile_kernel<FG, TY, TZ, DIAMOND><<<t.nx * t.ny * t.nz, kTileThreads, 0, st>>>(
+        (const typename FG::Value *)bin.data, fg, lab, d.bits, d.parent, d.minkey, d.count, g, t);
     ccl_merge_kernel<TY, TZ, DIAMOND><<<(nseg + kT - 1) / kT, kT, 0, st>>>(lab, d.bits, d.parent, g, t,
                                                                                FastDiv(t.ws), nseg);
     CLE_LAUNCH_CHECK_N("ccl tiles", 2);
     return CLE_OK;
 }
 
+// 16 x 8 rows per tile in volumes, 64 rows in images (and volumes of one plane)
+template <bool DIAMOND, typename FG>
+int dense_typed(const Img &bin, FG fg, uint32_t *lab, const Dense &d, const Geo &g, cudaStream_t st) {
+    if (bin.D > 1) return dense_tiles<FG, 16, 8, DIAMOND>(bin, fg, lab, d, g, st);
+    return dense_tiles<FG, 64, 1, DIAMOND>(bin, fg, lab, d, g, st);
+}
+
 template <typename T>
 int dense_typed(const Img &bin, uint32_t *lab, const Dense &d, const Geo &g, bool diamond, cudaStream_t st) {
-    // 16 x 8 rows per tile in volumes, 64 rows in images (and volumes of one plane)
-    if (bin.D > 1) return diamond ? dense_tiles<T, 16, 8, true>(bin, lab, d, g, st) : dense_tiles<T, 16, 8, false>(bin, lab, d, g, st);
-    return diamond ? dense_tiles<T, 64, 1, true>(bin, lab, d, g, st) : dense_tiles<T, 64, 1, false>(bin, lab, d, g, st);
+    return diamond ? dense_typed<true>(bin, NonZero<T>(), lab, d, g, st) : dense_typed<false>(bin, NonZero<T>(), lab, d, g, st);
 }
 
 // ---- relabel ------------------------------------------------------------
@@ -730,7 +753,7 @@ size_t ccl_workspace_bytes(const Img &im, bool diamond) {
     return a.off;
 }
 
-int ccl_dense(const Img &bin, uint32_t *lab, Arena &ws, cudaStream_t st, bool diamond) {
+int ccl_dense(const Img &bin, uint32_t *lab, Arena &ws, cudaStream_t st, bool diamond, const float *d_above) {
     const Dense d = take_dense(ws, bin, diamond);
     const Rank &r = d.rank;
     if (!ws.ok()) { set_error("connected_components_labeling_box: workspace too small"); return CLE_ERR_WORKSPACE; }
@@ -740,7 +763,10 @@ int ccl_dense(const Img &bin, uint32_t *lab, Arena &ws, cudaStream_t st, bool di
     switch (bin.dtype) {
         case CLE_U8: CLE_TRY(dense_typed<uint8_t>(bin, lab, d, g, diamond, st)); break;
         case CLE_U32: CLE_TRY(dense_typed<uint32_t>(bin, lab, d, g, diamond, st)); break;
-        case CLE_F32: CLE_TRY(dense_typed<float>(bin, lab, d, g, diamond, st)); break;
+        case CLE_F32:
+            if (d_above) CLE_TRY(dense_typed<false>(bin, Above{d_above}, lab, d, g, st));
+            else CLE_TRY(dense_typed<float>(bin, lab, d, g, diamond, st));
+            break;
         case CLE_U16: CLE_TRY(dense_typed<uint16_t>(bin, lab, d, g, diamond, st)); break;
         default: set_error("connected_components_labeling_box: unsupported dtype %d", bin.dtype); return CLE_ERR_DTYPE;
     }

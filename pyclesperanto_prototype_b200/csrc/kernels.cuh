@@ -83,7 +83,9 @@ int maxima_seeds(const Img &T, const float *O, const float *d_thr32, uint8_t *se
 size_t ccl_workspace_bytes(const Img &im, bool diamond = false);
 // Dense CCL of (binary != 0) into u32 labels (x-major float32 key ranks).
 // diamond: face connectivity (4 in 2D, 6 in 3D) instead of the 3^d box
-int ccl_dense(const Img &binary, uint32_t *labels, Arena &ws, cudaStream_t st, bool diamond = false);
+// d_above (float32, box): the binary image is image > *d_above
+int ccl_dense(const Img &binary, uint32_t *labels, Arena &ws, cudaStream_t st, bool diamond = false,
+              const float *d_above = nullptr);
 // CCL restricted to a device list of voxel indices whose entries in `labels`
 // already hold (own x-major key + 1); on return those entries hold labels.
 // d_count: device count of list entries; cap: list capacity.
@@ -127,6 +129,8 @@ int label_centroids(const Img &labels, int64_t n, float *pts, Arena &ws, cudaStr
 size_t vol_workspace_bytes(const Img &im);
 int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma,
                           double outline_sigma, Arena &ws, cudaStream_t st, const Limits &lim);
+size_t gauss_otsu_workspace_bytes(const Img &im);
+int gauss_otsu_labeling(const Img &src, const Img &dst, double sigma, Arena &ws, cudaStream_t st);
 
 // masked_voronoi_labeling for a 0/1 mask with every seed inside it (the
 // composite's case), on the active-brick growth.

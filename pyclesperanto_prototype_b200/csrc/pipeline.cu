@@ -420,4 +420,56 @@ int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma, dou
     return CLE_OK;
 }
 
+// ---- gauss_otsu_labeling ------------------------------------------------------
+// _tier9/_gauss_otsu_labeling.py:6-45: blur with its min / max, histogram, Otsu,
+// connected components of what lies above the threshold.  The labelling compares
+// as it loads and the blur reduces as it stores, so the binary image and the pass
+// for the extremes are gone: 128 x 1024 x 1024 uint16, sigma 2: 1.46 -> 1.32 ms.
+namespace {
+
+struct DenseLayout {
+    Scalars *sc;
+    float *O;
+};
+
+DenseLayout take_dense_layout(Arena &a, const Img &im) {
+    DenseLayout l;
+    l.sc = a.take<Scalars>(1);
+    l.O = a.take<float>(im.n());
+    return l;
+}
+
+}  // namespace
+
+size_t gauss_otsu_workspace_bytes(const Img &im) {
+    Arena a(nullptr, 0);
+    take_dense_layout(a, im);
+    const size_t tail = std::max(separable_workspace_bytes(im) + minmax_workspace_bytes(im),
+                                 std::max(histogram_workspace_bytes(im, 256), ccl_workspace_bytes(im)));
+    return a.off + tail;
+}
+
+int gauss_otsu_labeling(const Img &src, const Img &dst, double sigma, Arena &ws, cudaStream_t st) {
+    CLE_TRY(same_shape(src, dst, "source", "label_image_destination"));
+    if (dst.dtype != CLE_U32 && dst.dtype != CLE_F32) {
+        set_error("gauss_otsu_labeling: destination must be uint32 or float32");
+        return CLE_ERR_DTYPE;
+    }
+    DenseLayout l = take_dense_layout(ws, src);
+    const size_t tail_off = ws.off;
+    if (!ws.ok()) { set_error("gauss_otsu_labeling: workspace too small"); return CLE_ERR_WORKSPACE; }
+    CLE_CUDA(cudaMemsetAsync(l.sc, 0, sizeof(Scalars), st));
+    CLE_TRY(blur_minmax(src, l.O, sigma, &l.sc->mm, ws, st, &l.sc->status));
+    ws.off = tail_off;
+    Img Oi = src;
+    Oi.data = l.O;
+    Oi.dtype = CLE_F32;
+    CLE_TRY(histogram_otsu(Oi, l.sc->mm.out, l.sc->hist, &l.sc->thr, &l.sc->thr32, ws, st));
+    ws.off = tail_off;
+    uint32_t *lab = ws.take<uint32_t>(dst.n());
+    if (dst.dtype == CLE_U32) lab = (uint32_t *)dst.data;
+    CLE_TRY(ccl_dense(Oi, lab, ws, st, false, &l.sc->thr32));
+    return dst.dtype == CLE_F32 ? ccl_to_dst(lab, dst, st) : CLE_OK;
+}
+
 }  // namespace cle

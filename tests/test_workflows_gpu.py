@@ -79,6 +79,28 @@ def _blob_image(shape, seed):
     return rng.poisson(img).astype(np.float32)
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (70, 33), (5, 1, 40), (1, 65, 31), (17, 33, 95), (9, 18, 64)])
+@pytest.mark.parametrize("sigma", [0, 1.0, 3.0])
+@pytest.mark.parametrize("kind", ["uint8", "uint16", "float32", "constant", "nan"])
+def test_gauss_otsu_labeling_is_its_three_steps(cle, shape, sigma, kind):
+    # the labelling that compares as it loads against the same steps through a
+    # stored binary image
+    rng = np.random.default_rng(31)
+    img = rng.integers(0, 200, shape) * (rng.uniform(size=shape) < 0.3)
+    img = img.astype(kind if kind in ("uint8", "uint16") else np.float32)
+    if kind == "constant":
+        img[:] = 3.0
+    elif kind == "nan":
+        img.reshape(-1)[:: 41] = np.nan
+        img.reshape(-1)[7:: 53] = np.inf
+    a = cle.push(img)
+    steps = cle.connected_components_labeling_box(cle.threshold_otsu(cle.gaussian_blur(a, None, sigma, sigma, sigma)))
+    assert np.array_equal(cle.pull(cle.gauss_otsu_labeling(a, None, sigma)), cle.pull(steps))
+    as_float = cle.create(img.shape)
+    cle.gauss_otsu_labeling(a, as_float, sigma)
+    assert np.array_equal(cle.pull(as_float), cle.pull(steps).astype(np.float32))
+
+
 @pytest.mark.parametrize("shape,sigma", [((64, 80), 1.0), ((200, 150), 2.0), ((256, 256), 5.0),
                                          ((20, 60, 70), 1.0), ((33, 80, 65), 2.0)])
 def test_gauss_otsu_labeling_matches_oracle(cle, oracle, shape, sigma):
