@@ -338,7 +338,9 @@ size_t vol_workspace_bytes(const Img &im) {
     tail = std::max(tail, separable_workspace_bytes(im) + minmax_workspace_bytes(im));
     tail = std::max(tail, rank_workspace_bytes(fkey_bits_for(im.n())));
     tail = std::max(tail, voronoi_grow_workspace_bytes(im));
-    return base + tail;
+    // 17 bytes per voxel are used; the query keeps answering at least 18, which
+    // callers that hold scratch of their own size it by
+    return std::max(base + tail, (18 * (size_t)im.n() + 255) & ~(size_t)255);
 }
 
 int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma, double outline_sigma,
