@@ -261,6 +261,21 @@ def test_box_filter_windows(cle, oracle, shape, radii, dtype):
     assert np.array_equal(cle.pull(cle.top_hat_box(a, None, *radii)), oracle.top_hat_box(f, *radii))
 
 
+# x and y in one pass: edges of its 64 x 64 tiles, its smallest and largest radius
+# and the first one beyond, unequal radii, images narrower than a window
+@pytest.mark.parametrize("shape", [(2, 7), (64, 64), (65, 129), (3, 63, 66), (2, 130, 5), (2, 4, 200)])
+@pytest.mark.parametrize("radii", [(1, 1, 1), (16, 16, 2), (1, 16, 0), (16, 2, 0), (17, 3, 1), (7, 12, 5)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_box_filter_planes(cle, oracle, shape, radii, dtype):
+    r = np.random.default_rng(18)
+    a = (r.integers(0, np.iinfo(dtype).max, size=shape) if dtype != np.float32
+         else r.uniform(-1000, 1000, size=shape)).astype(dtype)
+    f = a.astype(np.float32)
+    assert np.array_equal(cle.pull(cle.minimum_box(a, None, *radii)), oracle.minimum_box(f, *radii))
+    assert np.array_equal(cle.pull(cle.maximum_box(a, None, *radii)), oracle.maximum_box(f, *radii))
+    assert np.array_equal(cle.pull(cle.top_hat_box(a, None, *radii)), oracle.top_hat_box(f, *radii))
+
+
 @pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
 def test_top_hat_box_narrow_input_and_in_place(cle, oracle, dtype):
     a = np.random.default_rng(9).integers(0, np.iinfo(dtype).max, (13, 70, 61)).astype(dtype)
