@@ -122,8 +122,8 @@ int erode_dst(const Img &src, const Img &dst, cudaStream_t st) {
 // and the last pass of top_hat_box subtracts, so neither has a pass of its own.
 // What bounds it: reading and writing the image in each pass.  r = 10 on 100 x 512 x
 // 512 uint16: x 55 us a pass (141 with a window scan per output), y and z 41 to 51
-// (98), 32 at copy bandwidth; top_hat_box 0.77 -> 0.31 ms, 0.24 with x and y in one
-// pass (below).
+// (98), 32 at copy bandwidth; top_hat_box 0.77 -> 0.31 ms, 0.22 with x and y in one
+// pass and the minimum and maximum along z in another (below).
 constexpr int kBK = 8;            // outputs per thread along the axis
 constexpr int kBT = 256;          // threads per CTA
 constexpr int kBRow = 256;        // x pass: most outputs of a row per CTA
@@ -317,6 +317,105 @@ minmax_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t 
         }
 }
 
+// Minimum, then maximum along an axis (the opening of top_hat_box along z) in one
+// launch: a CTA stages 128 outputs with 2 r on each side, makes the minima in the
+// place of the staged values, 128 rows at a time, and the maxima from those.  A
+// position outside the axis is none of the maximum's: its minimum is NaN, which
+// fmaxf passes over.  100 x 512 x 512, r = 10: 69 us against 93 in two launches;
+// 509 x 511 planes (scalar staging) 70 us less.
+// NG: groups of 8 outputs along the axis (128 outputs of 32 columns with 16).
+template <int NG>
+__global__ void __launch_bounds__(kBT)
+open_col_kernel(const float *__restrict__ src, float *__restrict__ dst, int64_t inner, int L, int r, int span, int vec) {
+    constexpr int NC = kBT / NG, kOCols = 2 * NC, kORows = NG * kBK;
+    extern __shared__ __align__(16) float sm[];
+    const int64_t c0 = (int64_t)blockIdx.x * kOCols;
+    const int l0 = blockIdx.y * kORows, tid = threadIdx.x;
+    if (vec) {   // inner a multiple of 4: asynchronous 16-byte copies
+        constexpr int QPR = kOCols / 4, STEP = kBT / QPR;
+        const int c = 4 * (tid % QPR);
+        const float *p = src + min(c0 + c, inner - 4);
+        for (int j = tid / QPR; j < span; j += STEP)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(sm + j * kOCols + c)),
+                         "l"(p + (int64_t)clampi(l0 - 2 * r + j, 0, L - 1) * inner)
+                         : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        constexpr int STEP = kBT / kOCols;   // (span is a multiple of 8 of them)
+        const float *p = src + min(c0 + tid % kOCols, inner - 1);
+        float *o = sm + tid;
+        for (int j0 = tid / kOCols; j0 < span; j0 += 8 * STEP, o += 8 * STEP * kOCols) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = __ldg(p + (int64_t)clampi(l0 - 2 * r + j0 + u * STEP, 0, L - 1) * inner);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) o[u * STEP * kOCols] = v[u];
+        }
+    }
+    __syncthreads();
+    const int g = tid / NC, w = 2 * r + 1, need = kORows + 2 * r;
+    float *col = sm + g * kBK * kOCols + 2 * (tid % NC);
+    float a[kBK], b[kBK];
+    for (int q = 0; q < need; q += kORows, col += kORows * kOCols) {
+        const int row = q + g * kBK, at = l0 - r + row;   // first minimum: its row, its position
+        const bool on = row < need && at < L && at + kBK > 0;
+        if (on) {
+            window8<false, kBK * kOCols, kOCols>(col, w, a);
+            window8<false, kBK * kOCols, kOCols>(col + 1, w, b);
+        }
+        __syncthreads();
+        if (row < need) {
+#pragma unroll
+            for (int k = 0; k < kBK; ++k) {
+                const bool in = on && at + k >= 0 && at + k < L;
+                col[k * kOCols] = in ? a[k] : NAN;
+                col[k * kOCols + 1] = in ? b[k] : NAN;
+            }
+        }
+    }
+    __syncthreads();
+    const int64_t c = c0 + 2 * (tid % NC);
+    const int left = L - (l0 + g * kBK);
+    if (c >= inner || left <= 0) return;
+    col = sm + g * kBK * kOCols + 2 * (tid % NC);
+    window8<true, kBK * kOCols, kOCols>(col, w, a);
+    window8<true, kBK * kOCols, kOCols>(col + 1, w, b);
+    const bool two = c + 1 < inner, pair = (inner & 1) == 0 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0;
+    float *o = dst + (int64_t)(l0 + g * kBK) * inner + c;
+#pragma unroll
+    for (int k = 0; k < kBK; ++k, o += inner)
+        if (k < left) {
+            if (pair) {
+                *reinterpret_cast<float2 *>(o) = make_float2(a[k], b[k]);
+            } else {
+                o[0] = a[k];
+                if (two) o[1] = b[k];
+            }
+        }
+}
+
+template <int NG>
+int launch_open(const float *src, float *dst, const Img &im, int r, cudaStream_t st) {
+    constexpr int COLS = 2 * (kBT / NG), ROWS = NG * kBK, STEP = 8 * kBT / COLS;
+    const int64_t inner = im.H * im.W;
+    const int span = (ROWS + 4 * r + kBK + STEP - 1) / STEP * STEP;
+    const size_t smem = sizeof(float) * COLS * (size_t)span;
+    if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(open_col_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((im.D + ROWS - 1) / ROWS));
+    const int vec = inner % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
+    open_col_kernel<NG><<<grid, kBT, smem, st>>>(src, dst, inner, (int)im.D, r, span, vec);
+    CLE_LAUNCH_CHECK("top_hat_box");
+    return CLE_OK;
+}
+
+int open_z(const float *src, float *dst, const Img &im, int r, cudaStream_t st) {
+    // short axes take fewer outputs and more columns per CTA
+    if (im.D <= 32) return launch_open<4>(src, dst, im, r, st);
+    if (im.D <= 64) return launch_open<8>(src, dst, im, r, st);
+    return launch_open<16>(src, dst, im, r, st);
+}
+
 // x and y passes of an image (or of every plane of a volume) in one launch: a CTA
 // stages 64 x 64 outputs with their halo, makes the x windows of all staged rows
 // (a warp per 8 columns, a lane per row) and the y windows of those (a warp per 8
@@ -419,6 +518,7 @@ int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, 
 
 // axis kXY: radius r along x and ry along y
 constexpr int kXY = 3;
+constexpr int kOpenZ = 4;   // minimum, then maximum along z
 template <bool MAX, typename Tin, typename Ts>
 int minmax_pass(const Tin *src, float *dst, const Img &im, int axis, int r, int ry, const Ts *minus, cudaStream_t st) {
     if (im.H > 65535 || im.D > 65535) { set_error("minimum/maximum box: image too large"); return CLE_ERR_TOO_LARGE; }
@@ -489,6 +589,11 @@ int run_steps(const Ts *src, float *out, float *tmp, const Img &im, const Step *
         // a y or z pass can subtract; an x pass is followed by a pass that does
         const Ts *m = i == n - 1 && steps[i].axis != 0 ? minus : nullptr;
         const Step &t = steps[i];
+        if (t.axis == kOpenZ) {   // behind an x, y pass
+            CLE_TRY(open_z(cur, o, im, t.r, st));
+            cur = o;
+            continue;
+        }
         if (i == 0) CLE_TRY(t.is_max ? minmax_pass<true>(src, o, im, t.axis, t.r, t.ry, m, st)
                                      : minmax_pass<false>(src, o, im, t.axis, t.r, t.ry, m, st));
         else CLE_TRY(t.is_max ? minmax_pass<true>(cur, o, im, t.axis, t.r, t.ry, m, st)
@@ -503,6 +608,12 @@ int run_steps(const Ts *src, float *out, float *tmp, const Img &im, const Step *
 }
 
 }  // namespace
+
+// top_hat_box's opening along z in one launch up to radius 24 (behind an x, y pass),
+// where it was the faster form for every size tried; the minima of 2 r more rows
+// per 128 outputs outweigh the saved pass from about 32 on (300 x 256 x 256, x and y
+// r = 3: r = 10 164 against 178 us, 24 201 : 204, 32 229 : 219).
+constexpr int kMaxOpenR = 24;
 
 // x and y in one pass up to radius 16 (its staging's 96 columns), where it was the
 // faster form for every size tried: 100 x 512 x 512 r = 1 60 against 92 us, r = 16 82
@@ -553,6 +664,7 @@ static int box_typed(const Img &src, float *dst, const int r[3], bool is_max, bo
     int k = 0;
     const int64_t len[3] = {src.W, src.H, src.D};
     const bool xy = plane_pass(src, r[0], r[1]);
+    const bool open = hat && xy && r[2] > 0 && len[2] > 1 && std::min<int64_t>(r[2], len[2] - 1) <= kMaxOpenR;
     for (int p = 0; p < (hat ? 2 : 1); ++p) {
         const bool mx = hat ? p == 1 : is_max;
         auto pass = [&](int a) {
@@ -560,10 +672,14 @@ static int box_typed(const Img &src, float *dst, const int r[3], bool is_max, bo
         };
         // the order of the axes does not change a minimum or maximum: the last
         // pass is one that can subtract
-        if (p == 1 && xy) pass(2);
+        if (open) {
+            if (p == 1) steps[k++] = {false, kOpenZ, (int)std::min<int64_t>(r[2], len[2] - 1), 0};
+        } else if (p == 1 && xy) {
+            pass(2);
+        }
         if (xy) steps[k++] = {mx, kXY, r[0], r[1]};
         else { pass(0); pass(1); }
-        if (p == 0 || !xy) pass(2);
+        if ((p == 0 && !open) || !xy) pass(2);
     }
     return run_steps<Ts>(in, dst, tmp, src, steps, k, hat ? in : nullptr, st);
 }

@@ -276,6 +276,23 @@ def test_box_filter_planes(cle, oracle, shape, radii, dtype):
     assert np.array_equal(cle.pull(cle.top_hat_box(a, None, *radii)), oracle.top_hat_box(f, *radii))
 
 
+# the opening along z in one launch: depths around its 32 / 64 / 128 outputs per CTA,
+# more than one CTA along z, its largest radius and the next, scalar staging
+@pytest.mark.parametrize("shape", [(2, 9, 8), (32, 5, 12), (33, 7, 7), (65, 3, 40), (128, 4, 4), (300, 3, 37)])
+@pytest.mark.parametrize("rz", [1, 4, 10, 24, 25])
+def test_top_hat_box_opening_along_z(cle, oracle, shape, rz):
+    a = np.random.default_rng(19).uniform(-1000, 1000, size=shape).astype(np.float32)
+    assert np.array_equal(cle.pull(cle.top_hat_box(a, None, 1, 2, rz)), oracle.top_hat_box(a, 1, 2, rz))
+    # NaN and infinities, windows of NaN alone among them: as the two filters
+    f = a.reshape(-1)
+    f[::7], f[1::11], f[2::13] = np.nan, np.inf, -np.inf
+    a[shape[0] // 2:, :3] = np.nan
+    s = cle.push(a)
+    opened = cle.pull(cle.maximum_box(cle.minimum_box(s, None, 1, 2, rz), None, 1, 2, rz))
+    with np.errstate(invalid="ignore"):
+        assert np.array_equal(cle.pull(cle.top_hat_box(s, None, 1, 2, rz)), a - opened, equal_nan=True)
+
+
 @pytest.mark.parametrize("dtype", [np.uint8, np.uint16])
 def test_top_hat_box_narrow_input_and_in_place(cle, oracle, dtype):
     a = np.random.default_rng(9).integers(0, np.iinfo(dtype).max, (13, 70, 61)).astype(dtype)
