@@ -98,7 +98,7 @@ int relabel_sequential(const Img &src, const Img &dst, uint32_t max_label, Arena
                        cudaStream_t st);
 size_t rank_workspace_bytes(uint64_t bits);
 
-// voronoi.cu
+// voronoi_bricks.cu (general masks: voronoi.cu)
 // Growth of seed labels inside a mask: labels u32 with the seeds' labels, 0
 // elsewhere; seeds: device list of seed memory indices (count in
 // d_seed_count); d_status receives 0 or an error.  By arrival keys (bricks

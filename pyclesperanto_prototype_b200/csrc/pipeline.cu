@@ -7,7 +7,7 @@
 //                                                  seed list and the initial CCL keys;
 //                                                  mean_box r=0 is a copy)
 //   labels(seeds) = CCL                           (ccl.cu, list form)
-//   labels = masked Voronoi growth inside seg     (voronoi.cu, frontier form)
+//   labels = masked Voronoi growth inside seg     (voronoi_bricks.cu)
 // The label output buffer is the CCL parent store and the Voronoi state, so
 // the only full-size scratch is O (f32), seg (u8), the seed list and a tail the
 // phases share: the blurs' temporaries, the spot blur, the growth's lists.
