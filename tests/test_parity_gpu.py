@@ -431,6 +431,26 @@ def test_vol_equal_sigmas_into_dirty_or_aliased_destination(cle, oracle, shape):
     assert np.array_equal(got, ref)
 
 
+# two blurs: column pairs and single columns, one to several planes, edges of the
+# warps' 60 and 30 columns and 4 and 8 rows, spot blurs of each form (a copy, one
+# launch, three passes), labels over the source, float32 labels
+@pytest.mark.parametrize("shape", [(1, 1), (40, 31), (65, 60), (1, 9, 61), (2, 33, 62), (3, 8, 121), (5, 40, 120), (9, 21, 30)])
+@pytest.mark.parametrize("spot,outline", [(2, 1), (1, 3), (0, 1), (3.5, 0), (1, 0.5)])
+def test_vol_two_sigmas_exact(cle, oracle, shape, spot, outline):
+    import torch
+    r = rng(35)
+    img = (r.uniform(0, 50, shape) + 400 * (r.uniform(size=shape) < 0.03)).astype(np.float32)
+    img[..., : shape[-1] // 3] = np.round(img[..., : shape[-1] // 3] / 40) * 40   # ties between neighbours
+    ref = oracle.voronoi_otsu_labeling(img, spot, outline)
+    src = torch.from_numpy(img.copy()).cuda()
+    assert np.array_equal(cle.pull(cle.voronoi_otsu_labeling(cle.B200Array(src), spot_sigma=spot, outline_sigma=outline)), ref)
+    as_float = cle.create(img.shape)
+    cle.voronoi_otsu_labeling(cle.B200Array(src), as_float, spot, outline)
+    assert np.array_equal(cle.pull(as_float), ref.astype(np.float32))
+    over = cle.B200Array(src.view(torch.uint32))
+    assert np.array_equal(cle.pull(cle.voronoi_otsu_labeling(cle.B200Array(src), over, spot, outline)), ref)
+
+
 def test_vol_edge_cases(cle):
     assert cle.pull(cle.voronoi_otsu_labeling(np.full((16, 16), 3.0, np.float32))).max() == 0
     assert cle.pull(cle.voronoi_otsu_labeling(np.zeros((1, 1), np.float32))).max() == 0
