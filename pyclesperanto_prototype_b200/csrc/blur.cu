@@ -308,8 +308,7 @@ int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, 
     constexpr int COLS = 2 * (kSepThreads / NG), ROWS = NG * kK;
     const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((L + ROWS - 1) / ROWS), (unsigned)outer);
     const size_t smem = sizeof(float2) * tap_slots(t.n) + sizeof(float) * COLS * kK * line_blocks(ROWS, t.n);
-    if (smem > 48 * 1024)
-        CLE_CUDA(cudaFuncSetAttribute(blur_col_kernel<Tin, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CLE_TRY(allow_smem(blur_col_kernel<Tin, NG>, smem, sizeof(float) * 2 * (kSepThreads / 32)));
     const int vec = inner % 4 == 0 && reinterpret_cast<uintptr_t>(src) % (4 * sizeof(Tin)) == 0;
     blur_col_kernel<Tin, NG><<<grid, kSepThreads, smem, st>>>(src, dst, inner, L, vec, t, mm);
     return CLE_OK;
@@ -329,8 +328,7 @@ int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps 
         const dim3 grid((unsigned)((im.W + tile - 1) / tile), (unsigned)std::min<int64_t>(ctas, 65535),
                         (unsigned)((ctas + 65534) / 65535));
         const size_t smem = sizeof(float2) * (tap_slots(t.n) + (size_t)np * kBlk * line_blocks(tile, t.n));
-        if (smem > 48 * 1024)
-            CLE_CUDA(cudaFuncSetAttribute(blur_row_kernel<Tin>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CLE_TRY(allow_smem(blur_row_kernel<Tin>, smem));
         const int vec = im.W % 4 == 0 && reinterpret_cast<uintptr_t>(src) % (4 * sizeof(Tin)) == 0;
         blur_row_kernel<Tin><<<grid, kSepThreads, smem, st>>>(src, dst, rows, (int)im.W, tile, np,
                                                               FastDiv((uint32_t)(tile / kK)), vec, t);

@@ -52,6 +52,21 @@ int cuda_error(cudaError_t e, const char *where);
         if (s_ != CLE_OK) return s_;                                          \
     } while (0)
 
+// Shared memory a CTA can have on sm_100.
+static constexpr size_t kMaxSmem = 227 * 1024;
+// Lets `kern` be launched with `smem` bytes of dynamic shared memory.  The limit
+// belongs to the kernel in its context, not to the launch, and another host
+// thread may be launching the same kernel with another size: a limit at this
+// call's size could drop below what that launch needs.  So it is always set to
+// the same value, the most the kernel can have (`fixed`: what its static shared
+// memory takes of it).
+template <typename K>
+inline int allow_smem(K *kern, size_t smem, size_t fixed = 0) {
+    if (smem > 48 * 1024)
+        CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxSmem - fixed)));
+    return CLE_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Images
 // ---------------------------------------------------------------------------

@@ -401,7 +401,7 @@ int launch_open(const float *src, float *dst, const Img &im, int r, cudaStream_t
     const int64_t inner = im.H * im.W;
     const int span = (ROWS + 4 * r + kBK + STEP - 1) / STEP * STEP;
     const size_t smem = sizeof(float) * COLS * (size_t)span;
-    if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(open_col_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CLE_TRY(allow_smem(open_col_kernel<NG>, smem));
     const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((im.D + ROWS - 1) / ROWS));
     const int vec = inner % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
     open_col_kernel<NG><<<grid, kBT, smem, st>>>(src, dst, inner, (int)im.D, r, span, vec);
@@ -509,7 +509,7 @@ int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, 
     constexpr int COLS = 2 * (kBT / NG), ROWS = NG * kBK;
     auto kern = minmax_col_kernel<MAX, Tin, NG, Ts>;
     const size_t smem = sizeof(float) * COLS * (size_t)(ROWS + 2 * r);
-    if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CLE_TRY(allow_smem(kern, smem));
     const dim3 grid((unsigned)((inner + COLS - 1) / COLS), (unsigned)((L + ROWS - 1) / ROWS), (unsigned)outer);
     const int vec = sizeof(Tin) == 4 && inner % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
     kern<<<grid, kBT, smem, st>>>(src, dst, inner, L, r, vec, minus);
@@ -526,7 +526,7 @@ int minmax_pass(const Tin *src, float *dst, const Img &im, int axis, int r, int 
         auto kern = minmax_plane_kernel<MAX, Tin, Ts>;
         const int rows = plane_rows(ry);
         const size_t smem = sizeof(float) * (size_t)rows * kBIn;
-        CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CLE_TRY(allow_smem(kern, smem));
         const dim3 grid((unsigned)((im.W + kBP - 1) / kBP), (unsigned)((im.H + kBP - 1) / kBP), (unsigned)im.D);
         kern<<<grid, kBT, smem, st>>>(src, dst, (int)im.H, (int)im.W, r, ry, rows, minus);
     } else if (axis == 0) {
@@ -539,7 +539,7 @@ int minmax_pass(const Tin *src, float *dst, const Img &im, int axis, int r, int 
         const int np = (int)std::max<size_t>(1, std::min<size_t>(std::min(kBT / (tile / kBK), 32), 65536 / (sizeof(float) * pitch)));
         const size_t smem = sizeof(float) * (size_t)np * pitch;
         auto kern = minmax_row_kernel<MAX, Tin>;
-        if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CLE_TRY(allow_smem(kern, smem));
         const int64_t ctas = (rows + np - 1) / np;
         const dim3 grid((unsigned)((im.W + tile - 1) / tile), (unsigned)std::min<int64_t>(ctas, 65535),
                         (unsigned)((ctas + 65534) / 65535));

@@ -304,7 +304,7 @@ int average_distance_of_n_distances(const Img &dm, int n, int exclude_self, cons
     if (dm.W == 0) return CLE_OK;
     size_t smem = 0;
     const int t = buffer_threads(std::max(n, 1), 0, smem);
-    CLE_CUDA(cudaFuncSetAttribute(n_distances_matrix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CLE_TRY(allow_smem(n_distances_matrix_kernel, smem));
     n_distances_matrix_kernel<<<(unsigned)((dm.W + t - 1) / t), t, smem, st>>>((const float *)dm.data, dm.H, dm.W, n,
                                                                               exclude_self, (float *)dst.data);
     CLE_LAUNCH_CHECK("n distances");
@@ -334,7 +334,7 @@ int average_distance_of_n_points(const Img &a, const Img &b, int n, int exclude_
     CLE_TRY(vector_out(dst, na + 1, "average distance"));
     size_t smem = 0;
     const int t = buffer_threads(std::max(n, 1), sizeof(float) * 3 * kPtsTile, smem);
-    CLE_CUDA(cudaFuncSetAttribute(n_distances_points_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CLE_TRY(allow_smem(n_distances_points_kernel, smem));
     n_distances_points_kernel<<<(unsigned)((na + 1 + t - 1) / t), t, smem, st>>>(
         (const float *)a.data, na, (const float *)b.data, nb, da, n, exclude_self, (float *)dst.data);
     CLE_LAUNCH_CHECK("n nearest points");

@@ -536,20 +536,20 @@ int histogram_impl(const Img &im, int bins, const float *d_minmax, float *d_hist
     if (im.H > 2147483647 || zchunks > 65535) { set_error("histogram: image too large"); return CLE_ERR_TOO_LARGE; }
     dim3 grid((unsigned)im.H, (unsigned)zchunks);
     const size_t smem = sizeof(uint32_t) * bins * (bins <= 512 ? kHistThreads / 32 : 1);
-    if (smem > 227 * 1024) { set_error("histogram: too many bins (%d)", bins); return CLE_ERR_ARG; }
+    if (smem > kMaxSmem) { set_error("histogram: too many bins (%d)", bins); return CLE_ERR_ARG; }
     if (zchunks > 1) CLE_CUDA(cudaMemsetAsync(part, 0, sizeof(uint32_t) * im.H * bins, st));
     const FastDiv fw((uint32_t)im.W), fw4((uint32_t)std::max<int64_t>(1, im.W / 4));
     switch (im.dtype) {
         case CLE_F32:
-            if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(hist_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CLE_TRY(allow_smem(hist_rows_kernel<float>, smem));
             hist_rows_kernel<float><<<grid, kHistThreads, smem, st>>>((const float *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, fw, fw4, done);
             break;
         case CLE_U16:
-            if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(hist_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CLE_TRY(allow_smem(hist_rows_kernel<uint16_t>, smem));
             hist_rows_kernel<uint16_t><<<grid, kHistThreads, smem, st>>>((const uint16_t *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, fw, fw4, done);
             break;
         case CLE_U8:
-            if (smem > 48 * 1024) CLE_CUDA(cudaFuncSetAttribute(hist_rows_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CLE_TRY(allow_smem(hist_rows_kernel<uint8_t>, smem));
             hist_rows_kernel<uint8_t><<<grid, kHistThreads, smem, st>>>((const uint8_t *)im.data, im.D, im.H, im.W, bins, zchunk, d_minmax, part, fw, fw4, done);
             break;
         default: set_error("histogram: unsupported dtype %d", im.dtype); return CLE_ERR_DTYPE;
