@@ -1,0 +1,39 @@
+"""Images longer along one axis than a CUDA grid's second and third axes reach
+(65535), and destinations that start in the middle of an allocation."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cle():
+    import pyclesperanto_prototype_b200 as m
+    from pyclesperanto_prototype_b200 import _build
+    _build.build()
+    return m
+
+
+def _image(shape, dtype, seed=5):
+    return np.random.default_rng(seed).integers(0, 60000, size=shape).astype(dtype)
+
+
+# radius 12 takes the three-pass form, 8 the fused one; the y pass of a volume runs
+# over all its planes at once, a long image has many tiles along y
+@pytest.mark.parametrize("shape,sigma", [((65537, 2, 3), (3, 3, 3)), ((65537, 2, 4), (3, 3, 3)), ((65537, 2, 3), (2, 2, 2)),
+                                         ((70000, 3, 1), (0, 1, 0.5)), ((65536 * 128 + 1, 1), (0, 1.5, 0))])
+@pytest.mark.parametrize("dtype", [np.uint16, np.float32])
+def test_gaussian_blur_of_long_axes(cle, oracle, shape, sigma, dtype):
+    a = _image(shape, dtype)
+    got = cle.pull(cle.gaussian_blur(a, None, *sigma))
+    assert np.array_equal(got, oracle.gaussian_blur(a.astype(np.float32), *sigma))
+
+
+@pytest.mark.parametrize("sigma", [2.0, 3.0])
+def test_labelings_of_many_planes(cle, oracle, sigma):
+    a = _image((65537, 2, 3), np.uint16)
+    f = a.astype(np.float32)
+    assert np.array_equal(cle.pull(cle.gauss_otsu_labeling(a, outline_sigma=sigma)), oracle.gauss_otsu_labeling(f, sigma))
+    for spot, outline in ((sigma, sigma), (1.0, sigma), (sigma, 1.0)):
+        got = cle.pull(cle.voronoi_otsu_labeling(a, spot_sigma=spot, outline_sigma=outline))
+        assert np.array_equal(got, oracle.voronoi_otsu_labeling(f, spot, outline))
