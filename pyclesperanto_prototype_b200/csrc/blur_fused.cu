@@ -363,7 +363,9 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
     const int tx = (tid % kCP) * 2;
     const int ry0 = (tid / kCP) * kRY;
     const bool c0_ok = (x0 + tx) < W, c1_ok = (x0 + tx + 1) < W;
-    const bool pair_store = c1_ok && (W & 1) == 0;     // 8-byte aligned float2 store
+    // 8-byte stores: rows of an even length in a destination on an 8-byte boundary
+    // (a view may start at any element)
+    const bool pair_store = c1_ok && (W & 1) == 0 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0;
     float vmin = INFINITY, vmax = -INFINITY;   // of the stored values (when mm)
     auto store2 = [&](float *o, float2 v) {
         if (pair_store) *reinterpret_cast<float2 *>(o) = v;

@@ -37,3 +37,21 @@ def test_labelings_of_many_planes(cle, oracle, sigma):
     for spot, outline in ((sigma, sigma), (1.0, sigma), (sigma, 1.0)):
         got = cle.pull(cle.voronoi_otsu_labeling(a, spot_sigma=spot, outline_sigma=outline))
         assert np.array_equal(got, oracle.voronoi_otsu_labeling(f, spot, outline))
+
+
+# a destination (and a source) that starts one element into its allocation, with
+# rows whose length alone would allow wide loads and stores
+@pytest.mark.parametrize("shape", [(40, 64), (7, 36, 64), (3, 5, 6)])
+@pytest.mark.parametrize("sigma", [(0.5, 0.5, 0.5), (2, 2, 2), (3.5, 3.5, 3.5), (1, 2, 0.5)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_gaussian_blur_of_views_off_alignment(cle, oracle, shape, sigma, dtype):
+    import torch
+    n = int(np.prod(shape))
+    a = np.random.default_rng(6).integers(0, 255, size=shape).astype(dtype)
+    src = torch.zeros(n + 1, dtype=getattr(torch, np.dtype(dtype).name), device="cuda")
+    src[1:].copy_(torch.from_numpy(a.reshape(-1)))
+    buf = torch.full((n + 3,), -1.0, device="cuda")
+    dst = cle.B200Array(buf[1:1 + n].view(shape))
+    cle.gaussian_blur(cle.B200Array(src[1:].view(shape)), dst, *sigma)
+    assert np.array_equal(cle.pull(dst), oracle.gaussian_blur(a.astype(np.float32), *sigma))
+    assert buf[0].item() == -1.0 and buf[-2:].eq(-1.0).all()
