@@ -9,7 +9,8 @@
 //   * planes go in groups of P (4, or 2 or 1 where shared memory is short).  The
 //     raw (kTY+2R) x (kTX+2R) tiles of a group are staged in shared memory in
 //     the source's own type, two groups deep.  On volumes whose rows are a
-//     multiple of 16 bytes (when the caller gives a status word) one thread
+//     multiple of 16 bytes and whose tiles mostly lie inside the image (tma_pays;
+//     when the caller gives a status word) one thread
 //     fetches a group with TMA copies (cp.async.bulk.tensor) an interval
 //     ahead, completion counted by an mbarrier per stage; otherwise each
 //     thread loads its share of a plane into registers through a table of
@@ -609,6 +610,18 @@ bool encode_source_map(const Img &src, CUtensorMap &map, cudaStream_t st) {
     return r == CUDA_SUCCESS;
 }
 
+// TMA staging pays where most tiles lie inside the image: a tile on its edge is
+// patched behind another barrier in every group.  Interior tiles: half of them
+// (8 x 8 tiles) for 8/16-bit sources, three quarters (16 x 16) for float32, whose
+// copies are longest.  Microseconds with TMA / through registers, uint16 sigma 2:
+// 16 x 16 x 16 29 / 18, 64 x 128 x 128 31 / 29, 512 x 1024 x 16 127 / 92, 64 x 256 x 256 44 / 43,
+// 100 x 512 x 512 141 / 157, 4 x 1024 x 1024 73 / 84; float32: 16 x 16 x 16 31 / 21,
+// 96 x 256 x 256 68 / 62, 100 x 512 x 512 180 / 178 (sigma 0.5: 63 / 91), 4 x 1024 x 1024 94 / 101.
+bool tma_pays(const dim3 &grid, int bytes) {
+    const int64_t gx = grid.x, gy = grid.y, inside = std::max<int64_t>(0, gx - 2) * std::max<int64_t>(0, gy - 2);
+    return bytes < 4 ? 2 * inside >= gx * gy : 4 * inside >= 3 * gx * gy;
+}
+
 template <typename Tin, int R, bool Z>
 int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, int *status, cudaStream_t st) {
     using G = Geom<Tin, R, Z>;
@@ -620,7 +633,7 @@ int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, i
     alignas(64) CUtensorMap map;
     std::memset(&map, 0, sizeof(map));
     if constexpr (Z) {
-        if (status != nullptr && encode_source_map<Tin, R>(src, map, st)) {
+        if (status != nullptr && tma_pays(grid, sizeof(Tin)) && encode_source_map<Tin, R>(src, map, st)) {
             auto kern = blur_fused_kernel<Tin, R, true, true>;
             // set on every call: the attribute belongs to the current device's context
             CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));

@@ -55,3 +55,45 @@ def test_gaussian_blur_of_views_off_alignment(cle, oracle, shape, sigma, dtype):
     cle.gaussian_blur(cle.B200Array(src[1:].view(shape)), dst, *sigma)
     assert np.array_equal(cle.pull(dst), oracle.gaussian_blur(a.astype(np.float32), *sigma))
     assert buf[0].item() == -1.0 and buf[-2:].eq(-1.0).all()
+
+
+# widths and heights on both sides of the tile counts from which volumes are staged
+# by TMA copies (8 x 8 tiles of 32 x 32 for 8/16-bit sources, 16 x 16 for float32)
+@pytest.mark.parametrize("dtype,width,height", [(np.uint8, 224, 256), (np.uint8, 240, 225), (np.uint16, 232, 224),
+                                                (np.uint16, 256, 250), (np.float32, 480, 481), (np.float32, 484, 481),
+                                                (np.float32, 512, 500)])
+@pytest.mark.parametrize("depth,sigma", [(1, 0.5), (3, 2.0), (9, 1.0), (21, 2.0)])
+def test_gaussian_blur_either_side_of_tma_staging(cle, oracle, dtype, width, height, depth, sigma):
+    a = np.random.default_rng(8).integers(0, 255, size=(depth, height, width)).astype(dtype)
+    got = cle.pull(cle.gaussian_blur(a, None, sigma, sigma, sigma))
+    assert np.array_equal(got, oracle.gaussian_blur(a.astype(np.float32), sigma, sigma, sigma))
+
+
+# a source that could be staged by TMA copies (16-byte aligned) is not slower than
+# the same one element further, which cannot (narrow and small volumes: 1.4 to 1.8
+# times the time while they were staged by TMA)
+@pytest.mark.parametrize("shape", [(16, 16, 16), (512, 8, 8), (512, 1024, 16), (128, 512, 512)])
+@pytest.mark.parametrize("dtype", ["uint16", "float32"])
+def test_aligned_sources_are_not_slower(cle, shape, dtype):
+    import torch
+    from pyclesperanto_prototype_b200 import _lib
+    lib, n = _lib.load(), int(np.prod(shape))
+    buf = torch.randint(0, 1000, (n + 1,), device="cuda", dtype=torch.int32).to(getattr(torch, dtype))
+    out = torch.empty(shape, device="cuda")
+    best = []
+    for src in (buf[:n].view(shape), buf[1:].view(shape)):
+        s, d = _lib.tensor_desc(src), _lib.tensor_desc(out)
+        ws = torch.empty(lib.cle_gaussian_blur_workspace_bytes(_lib.ref(s)), dtype=torch.uint8, device="cuda")
+        args = (_lib.ref(s), _lib.ref(d), 2.0, 2.0, 2.0, ws.data_ptr(), ws.numel(), _lib.stream_ptr())
+        times = []
+        for _ in range(8):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            e0.record()
+            for _ in range(40):
+                _lib.check(lib.cle_gaussian_blur(*args))
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        best.append(min(times))
+    assert best[0] <= 1.25 * best[1]
