@@ -337,7 +337,9 @@ int cle_voronoi_labeling(const cle_tensor *binary, const cle_tensor *dst,
 
 /* ---- gauss_otsu_labeling -----------------------------------------------
  * replaces _tier9/_gauss_otsu_labeling.py:6-45: gaussian_blur, threshold_otsu,
- * connected_components_labeling_box.  src: u8/u16/f32; dst: u32 or f32. */
+ * connected_components_labeling_box.  src: u8/u16/f32; dst: u32 or f32.  No host
+ * synchronisation, and no status to read: a blur of a volume whose copy waits
+ * ran out (2 s, see gaussian_blur) is made again without such copies. */
 size_t cle_gauss_otsu_labeling_workspace_bytes(const cle_tensor *src);
 int cle_gauss_otsu_labeling(const cle_tensor *src, const cle_tensor *dst, double outline_sigma,
                             void *workspace, size_t workspace_bytes, void *stream);

@@ -210,6 +210,8 @@ __device__ __forceinline__ void load_words(const uint8_t *p, uint32_t *w) {
 // TMA: stage planes with the tensor map `tmap` (3D only).  A stage wait that
 // runs out raises s_fail: no later wait blocks, no more copies are issued, the
 // copies in flight are waited for and *status is set.
+// Without TMA, a status word makes the launch the repeat of a TMA launch (same
+// grid): it returns at once unless a wait ran out there.
 template <typename Tin, int R, bool Z, bool TMA>
 __global__ void __launch_bounds__(kThreads, (min_ctas<R>()))
 blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorMap tmap,
@@ -224,6 +226,12 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
     uint8_t *raw = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
     float *Xo = reinterpret_cast<float *>(raw + (Z ? 2 * P : 1) * G::STAGE);
     int *tab = reinterpret_cast<int *>(Xo + (Z ? 2 * P : 1) * G::XBUF);
+
+    if constexpr (!TMA) {
+        if (status != nullptr && *(volatile int *)status == 0) return;
+    }
+    // CTAs that add to mm, those of the launch that is repeated among them
+    const uint32_t ctas = gridDim.x * gridDim.y * gridDim.z * (!TMA && status != nullptr ? 2u : 1u);
 
     // in 3D the taps stay in registers as packed pairs (w, w), read once
     // through shared memory: taken from the parameter they are fetched for
@@ -501,6 +509,7 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
             if (tid == 0) {
                 for (int q = max(0, issued - 2); q < issued; ++q) mbar_wait(&bars[q & 1], (uint32_t)(q >> 1) & 1u);
                 atomicCAS(status, 0, (int)CLE_ERR_ITER_LIMIT);
+                if (mm) add_minmax(mm, INFINITY, -INFINITY, ctas);
             }
             return;
         }
@@ -517,7 +526,7 @@ blur_fused_kernel(const Tin *__restrict__ src, const __grid_constant__ CUtensorM
         __syncthreads();
         if (tid == 0) {
             for (int w = 1; w < kWarps; ++w) { vmin = fminf(vmin, s_mn[w]); vmax = fmaxf(vmax, s_mx[w]); }
-            add_minmax(mm, vmin, vmax, gridDim.x * gridDim.y * gridDim.z);
+            add_minmax(mm, vmin, vmax, ctas);
         }
     }
 }
@@ -623,7 +632,7 @@ bool tma_pays(const dim3 &grid, int bytes) {
 }
 
 template <typename Tin, int R, bool Z>
-int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, int *status, cudaStream_t st) {
+int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, int *status, bool repeat, cudaStream_t st) {
     using G = Geom<Tin, R, Z>;
     int zchunk = 1;
     const dim3 grid = fused_grid(src, R, zchunk);
@@ -632,6 +641,7 @@ int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, i
     for (int i = 0; i <= R; ++i) pt.w[i] = t.w[i];
     alignas(64) CUtensorMap map;
     std::memset(&map, 0, sizeof(map));
+    int *gate = nullptr;
     if constexpr (Z) {
         if (status != nullptr && tma_pays(grid, sizeof(Tin)) && encode_source_map<Tin, R>(src, map, st)) {
             auto kern = blur_fused_kernel<Tin, R, true, true>;
@@ -640,25 +650,26 @@ int launch_fused_r(const Img &src, float *dst, const Taps &t, MinMaxState *mm, i
             kern<<<grid, kThreads, G::SMEM, st>>>((const Tin *)src.data, map, dst, (int)src.D, (int)src.H,
                                                         (int)src.W, zchunk, pt, mm, status);
             CLE_LAUNCH_CHECK("gaussian_blur fused (TMA)");
-            return CLE_OK;
+            if (!repeat) return CLE_OK;
+            gate = status;
         }
     }
     auto kern = blur_fused_kernel<Tin, R, Z, false>;
     CLE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::SMEM));
     kern<<<grid, kThreads, G::SMEM, st>>>((const Tin *)src.data, map, dst, (int)src.D, (int)src.H, (int)src.W,
-                                                zchunk, pt, mm, status);
+                                                zchunk, pt, mm, gate);
     CLE_LAUNCH_CHECK("gaussian_blur fused");
     return CLE_OK;
 }
 
 template <typename Tin, bool Z, int R = 1>
-int dispatch_r(const Img &src, float *dst, const Taps &t, int r, MinMaxState *mm, int *status, cudaStream_t st) {
+int dispatch_r(const Img &src, float *dst, const Taps &t, int r, MinMaxState *mm, int *status, bool repeat, cudaStream_t st) {
     if constexpr (R > (Z ? kMaxFusedR3 : kMaxFusedR)) {
         set_error("internal: fused radius out of range");
         return CLE_ERR_ARG;
     } else {
-        if (r == R) return launch_fused_r<Tin, R, Z>(src, dst, t, mm, status, st);
-        return dispatch_r<Tin, Z, R + 1>(src, dst, t, r, mm, status, st);
+        if (r == R) return launch_fused_r<Tin, R, Z>(src, dst, t, mm, status, repeat, st);
+        return dispatch_r<Tin, Z, R + 1>(src, dst, t, r, mm, status, repeat, st);
     }
 }
 
@@ -672,21 +683,22 @@ bool fused_blur_applies(const Img &src, double sx, double sy, double sz) {
     return r >= 1 && r <= (src.ndim == 3 ? kMaxFusedR3 : kMaxFusedR) && src.W < (1 << 30) && src.H < (1 << 30);
 }
 
-int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, MinMaxState *mm, int *status) {
+int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, MinMaxState *mm, int *status, bool repeat) {
     Taps t;
     CLE_TRY(make_gauss_taps(sigma, t));
     const int r = (t.n - 1) / 2;
     const bool z = src.ndim == 3;
     switch (src.dtype) {
-        case CLE_F32: return z ? dispatch_r<float, true>(src, dst, t, r, mm, status, st) : dispatch_r<float, false>(src, dst, t, r, mm, status, st);
-        case CLE_U16: return z ? dispatch_r<uint16_t, true>(src, dst, t, r, mm, status, st) : dispatch_r<uint16_t, false>(src, dst, t, r, mm, status, st);
-        case CLE_U8: return z ? dispatch_r<uint8_t, true>(src, dst, t, r, mm, status, st) : dispatch_r<uint8_t, false>(src, dst, t, r, mm, status, st);
+        case CLE_F32: return z ? dispatch_r<float, true>(src, dst, t, r, mm, status, repeat, st) : dispatch_r<float, false>(src, dst, t, r, mm, status, repeat, st);
+        case CLE_U16: return z ? dispatch_r<uint16_t, true>(src, dst, t, r, mm, status, repeat, st) : dispatch_r<uint16_t, false>(src, dst, t, r, mm, status, repeat, st);
+        case CLE_U8: return z ? dispatch_r<uint8_t, true>(src, dst, t, r, mm, status, repeat, st) : dispatch_r<uint8_t, false>(src, dst, t, r, mm, status, repeat, st);
         default: set_error("gaussian_blur: unsupported source dtype"); return CLE_ERR_DTYPE;
     }
 }
 
-int blur_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st, int *status) {
-    if (fused_blur_applies(src, sigma, sigma, sigma)) return fused_blur(src, dst, sigma, st, mm, status);
+int blur_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st, int *status,
+                bool repeat) {
+    if (fused_blur_applies(src, sigma, sigma, sigma)) return fused_blur(src, dst, sigma, st, mm, status, repeat);
     if (sigma > 0) return separable_minmax(src, dst, sigma, mm, ws, st);
     CLE_TRY(gaussian_blur(src, dst, sigma, sigma, sigma, ws, st, status));
     Img T = src;

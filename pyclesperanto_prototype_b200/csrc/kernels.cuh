@@ -22,13 +22,15 @@ int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, A
 // kMaxFusedR3 in 3D
 constexpr int kMaxFusedR = 14, kMaxFusedR3 = 8;
 bool fused_blur_applies(const Img &src, double sx, double sy, double sz);
-// mm (optional, zeroed before): the result's min / max
+// mm (optional, zeroed before): the result's min / max.  repeat: a blur whose
+// stage waits ran out is made again without TMA copies behind it on the stream,
+// for callers whose status word nobody reads
 int fused_blur(const Img &src, float *dst, double sigma, cudaStream_t st, MinMaxState *mm = nullptr,
-               int *status = nullptr);
+               int *status = nullptr, bool repeat = false);
 // Isotropic blur whose {min, max} lands in mm->out (the state zeroed before).
 // Workspace: separable_workspace_bytes and minmax_workspace_bytes.
 int blur_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st,
-                int *status = nullptr);
+                int *status = nullptr, bool repeat = false);
 
 // reduce.cu
 size_t minmax_workspace_bytes(const Img &im);

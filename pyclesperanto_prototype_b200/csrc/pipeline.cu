@@ -461,7 +461,9 @@ int gauss_otsu_labeling(const Img &src, const Img &dst, double sigma, Arena &ws,
     const size_t tail_off = ws.off;
     if (!ws.ok()) { set_error("gauss_otsu_labeling: workspace too small"); return CLE_ERR_WORKSPACE; }
     CLE_CUDA(cudaMemsetAsync(l.sc, 0, sizeof(Scalars), st));
-    CLE_TRY(blur_minmax(src, l.O, sigma, &l.sc->mm, ws, st, &l.sc->status));
+    // the call returns without a word that its caller would have to read, so a blur
+    // whose copies did not arrive is made again
+    CLE_TRY(blur_minmax(src, l.O, sigma, &l.sc->mm, ws, st, &l.sc->status, true));
     ws.off = tail_off;
     Img Oi = src;
     Oi.data = l.O;
