@@ -15,7 +15,7 @@
 // second needs the per-label centroid, mass centre and mean); the second takes
 // the labels and masks the first kept, 3.1 bytes per voxel of scratch at most,
 // and does not read the label image.  Coordinates and 8/16-bit intensities are
-// summed in exact integers, other intensities in float64; min / max through
+// summed in exact 64-bit integers (exact_sums), other intensities in float64; min / max through
 // order-preserving unsigned atomics.  The finalise kernels apply the reference's
 // float32 column arithmetic and its sentinels for labels absent from the image
 // (min FLT_MAX, max -FLT_MAX, sums 0, 0/0 = NaN).
@@ -38,7 +38,10 @@ constexpr int kMaxLabels = 24;   // labels of a brick reduced over the warp (few
 // Accumulators of a label: pass 1 ...
 struct alignas(32) Acc1 {
     unsigned long long s[4];   // sums of x, y, z, voxel count
-    double v[4];               // sums of intensity, intensity * x, * y, * z
+    union {                    // sums of intensity, intensity * x, * y, * z
+        double v[4];
+        unsigned long long u[4];   // (exact: see exact_sums)
+    };
     uint32_t lo[4], hi[4];     // smallest / largest x, y, z, ordered intensity
 };
 // ... and pass 2, with the label's centre and mean (pc) and mass centre and area (pm)
@@ -153,11 +156,12 @@ struct Sums {
         lo = min(lo, o.lo);
         hi = max(hi, o.hi);
     }
-    __device__ __forceinline__ void add_to(Acc1 *a) const {
+    __device__ __forceinline__ void add_to(Acc1 *a, bool exact) const {
         const int lane = threadIdx.x & 31;
         if (lane < 4) {
             atomicAdd(a->s + lane, s);
-            atomicAdd(a->v + lane, (double)v);   // integer totals stay far below 2^53: exact
+            if (INT && exact) atomicAdd(a->u + lane, (unsigned long long)v);
+            else atomicAdd(a->v + lane, (double)v);
             atomicMin(a->lo + lane, lo);
             atomicMax(a->hi + lane, hi);
         }
@@ -175,7 +179,7 @@ __device__ __forceinline__ T lane4(T a, T b, T c, T d) {
 template <typename TL, typename TI, int BY>
 __global__ void __launch_bounds__(kST, 2)
 brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bricks G, int64_t Lcap,
-                  const uint32_t *__restrict__ d_L, Acc1 *__restrict__ a1, Found F) {
+                  const uint32_t *__restrict__ d_L, Acc1 *__restrict__ a1, Found F, bool exact) {
     constexpr int BZ = 32 / BY;
     constexpr bool INT = sizeof(TI) <= 2 && !std::is_floating_point<TI>::value;
     const uint32_t L = (uint32_t)live_labels(Lcap, d_L);
@@ -242,15 +246,23 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
                     const uint32_t y = y0 + k % BY, z = z0 + k / BY;
                     const float f = to_f32(v[k]);
                     Acc1 *a = a1 + (l[k] - 1u);
-                    const double d = (double)f;
                     atomicAdd(a->s, (unsigned long long)x);
                     atomicAdd(a->s + 1, (unsigned long long)y);
                     atomicAdd(a->s + 2, (unsigned long long)z);
                     atomicAdd(a->s + 3, 1ull);
-                    atomicAdd(a->v, d);
-                    atomicAdd(a->v + 1, d * (double)x);
-                    atomicAdd(a->v + 2, d * (double)y);
-                    atomicAdd(a->v + 3, d * (double)z);
+                    if (INT && exact) {
+                        const unsigned long long u = (unsigned long long)v[k];
+                        atomicAdd(a->u, u);
+                        atomicAdd(a->u + 1, u * x);
+                        atomicAdd(a->u + 2, u * y);
+                        atomicAdd(a->u + 3, u * z);
+                    } else {
+                        const double d = (double)f;
+                        atomicAdd(a->v, d);
+                        atomicAdd(a->v + 1, d * (double)x);
+                        atomicAdd(a->v + 2, d * (double)y);
+                        atomicAdd(a->v + 3, d * (double)z);
+                    }
                     atomicMin(a->lo, x); atomicMin(a->lo + 1, y); atomicMin(a->lo + 2, z); atomicMin(a->lo + 3, f2u(f));
                     atomicMax(a->hi, x); atomicMax(a->hi + 1, y); atomicMax(a->hi + 2, z); atomicMax(a->hi + 3, f2u(f));
                 }
@@ -332,12 +344,12 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
             t.hi = lane4(bx * 32u + 31u - (uint32_t)__clz(cols), y0 + 31u - (uint32_t)__clz(ym), z0 + 31u - (uint32_t)__clz(zm), hi3);
             if (g == carried) {
                 carry.merge(t);
-            } else if (N >= 512u) {
-                if (carried) carry.add_to(a1 + (carried - 1u));
+            } else if (N >= 512u && (!INT || exact)) {
+                if (carried) carry.add_to(a1 + (carried - 1u), exact);
                 carry = t;
                 carried = g;
             } else {
-                t.add_to(a1 + (g - 1u));
+                t.add_to(a1 + (g - 1u), exact);
             }
             F.mask[((size_t)b * G.slots + found) * 32u + lane] = mine;
             if (lane == 0) F.label[(size_t)b * G.slots + found] = g;
@@ -345,7 +357,7 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
         }
         if (lane == 0) F.count[b] = (uint8_t)found;
     }
-    if (carried) carry.add_to(a1 + (carried - 1u));
+    if (carried) carry.add_to(a1 + (carried - 1u), exact);
 }
 
 // Pass 2 over the labels found in the bricks: the label's voxels are packed
@@ -455,14 +467,15 @@ enum {
 };
 static_assert(C_NCOLS == CLE_STATS_NCOLS, "table width");
 
-__global__ void stats_final1(const Acc1 *__restrict__ a, Acc2 *__restrict__ b, int64_t L, float *__restrict__ T, const uint32_t *__restrict__ d_L) {
+__global__ void stats_final1(const Acc1 *__restrict__ a, Acc2 *__restrict__ b, int64_t L, float *__restrict__ T, const uint32_t *__restrict__ d_L, bool exact) {
     const int64_t n = live_labels(L, d_L);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const Acc1 &A = a[i];
         const bool any = A.s[3] != 0ull;
         const float area = (float)A.s[3];
-        const float sum_i = (float)A.v[0];
+        auto total = [&](int k) { return exact ? (float)A.u[k] : (float)A.v[k]; };
+        const float sum_i = total(0);
         auto put = [&](int c, float v) { T[(int64_t)c * L + i] = v; };
         const float bx0 = any ? (float)A.lo[0] : FLT_MAX, bx1 = any ? (float)A.hi[0] : -FLT_MAX;
         const float by0 = any ? (float)A.lo[1] : FLT_MAX, by1 = any ? (float)A.hi[1] : -FLT_MAX;
@@ -478,7 +491,7 @@ __global__ void stats_final1(const Acc1 *__restrict__ a, Acc2 *__restrict__ b, i
         put(C_AREA, area);
         const float mean = __fdiv_rn(sum_i, area);
         put(C_MEAN_I, mean);
-        const float six = (float)A.v[1], siy = (float)A.v[2], siz = (float)A.v[3];
+        const float six = total(1), siy = total(2), siz = total(3);
         const float mxc = __fdiv_rn(six, sum_i), myc = __fdiv_rn(siy, sum_i), mzc = __fdiv_rn(siz, sum_i);
         put(C_SUM_IX, six); put(C_MASS_X, mxc);
         put(C_SUM_IY, siy); put(C_MASS_Y, myc);
@@ -598,16 +611,28 @@ StatsWs take_stats(Arena &a, const Img &labels, int64_t L) {
     return w;
 }
 
+// Intensity totals of 8/16-bit sources are kept in 64-bit integers wherever their
+// largest possible value fits (any image of up to 2^31 voxels with sides up to 65536);
+// in float64 they pass 2^53 from a label of 16 bits, full scale, in 512 x 1024 x 1024 on,
+// and further sums round in the order they arrive.
+template <typename TI>
+bool exact_sums(const Img &im) {
+    if (sizeof(TI) > 2) return false;
+    const double most = sizeof(TI) == 1 ? 255.0 : 65535.0;
+    return most * (double)im.n() * (double)std::max(im.W, std::max(im.H, im.D)) < 1.8e19;
+}
+
 template <typename TL, typename TI, int BY>
 int stats_typed(const Img &inten, const Img &lab, int64_t L, float *T, const StatsWs &w, cudaStream_t st,
                 const uint32_t *d_L) {
     const Bricks G = make_bricks(lab);
     const int blocks = launch_blocks((int64_t)G.n * 32, kST, 4);
+    const bool exact = exact_sums<TI>(lab);
     stage_mark(8, st);
     brick_sums_kernel<TL, TI, BY><<<blocks, kST, 0, st>>>((const TL *)lab.data, (const TI *)inten.data, G, L, d_L,
-                                                          w.a1, w.found);
+                                                          w.a1, w.found, exact);
     stage_mark(9, st);
-    stats_final1<<<launch_blocks(L, 256), 256, 0, st>>>(w.a1, w.a2, L, T, d_L);
+    stats_final1<<<launch_blocks(L, 256), 256, 0, st>>>(w.a1, w.a2, L, T, d_L, exact);
     stage_mark(10, st);
     brick_moments_kernel<TL, TI, BY><<<launch_blocks((int64_t)G.n * 32, kST, 16), kST, 0, st>>>(
         (const TL *)lab.data, (const TI *)inten.data, G, L, d_L, w.a2, w.found);
