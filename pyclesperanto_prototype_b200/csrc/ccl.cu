@@ -478,25 +478,43 @@ __global__ void ccl_label_list(uint32_t *__restrict__ lab, const uint32_t *__res
     }
 }
 
-// The whole list labelling of a small image in one CTA: unions, roots, marks,
-// ranks and labels with block barriers between them, one launch instead of
-// eight and a clear (256 x 256: 10.9 us against 34 and the launch gaps).
+// The whole list labelling of a small image in one launch: the unions by a thread
+// per listed voxel, then roots, marks, ranks and labels by the CTA that finishes
+// last, with block barriers between them, in place of eight launches and a clear.
+// That CTA takes 3 to 4 us for every 1024 listed voxels and the launches about 25 us in all,
+// so the line is one on the number of listed voxels, which only the device
+// knows.  Local maxima are few: voronoi_otsu_labeling of noise (256 x 256 0.18 against 0.23 ms
+// for the whole call, 362 x 362 0.20 : 0.24, 32 x 64 x 64 0.28 : 0.31).  A mask's voxels may be all
+// of them: masked_voronoi_labeling_binary of 90% masks 64 x 64 0.23 : 0.25, 16 x 32 x 32 0.52 : 0.54,
+// 256 x 256 0.31 : 0.27, 32 x 64 x 64 0.76 : 0.61.  With the unions in the one CTA too,
+// as this kernel was, the last took 11.1 ms.
 constexpr int kListCta = 1024;
-constexpr int64_t kListCtaVoxels = int64_t(1) << 17;
+constexpr int64_t kListSparseVoxels = int64_t(1) << 17, kListDenseVoxels = int64_t(1) << 15;
 
 __global__ void __launch_bounds__(kListCta)
 ccl_list_small(uint32_t *lab, Geo g, const uint32_t *__restrict__ list, const uint32_t *__restrict__ d_count,
-               uint32_t *bitmap, uint32_t *prefix, uint32_t words, uint32_t *__restrict__ d_nlabels) {
+               uint32_t *bitmap, uint32_t *prefix, uint32_t words, uint32_t *__restrict__ d_nlabels, uint32_t *d_done) {
     __shared__ uint32_t s_w[kListCta / 32];
+    __shared__ uint32_t s_ticket;
     const uint32_t cnt = *d_count;
     const uint32_t t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
-    for (uint32_t w = t; w < words; w += kListCta) st_cg(bitmap + w, 0u);
-    for (uint32_t i = t; i < cnt; i += kListCta) {
+    const uint32_t ctas = max(1u, min(gridDim.x, (cnt + kListCta - 1) / kListCta));   // that have voxels
+    if (blockIdx.x >= ctas) return;
+    for (uint32_t i = blockIdx.x * kListCta + t; i < cnt; i += ctas * kListCta) {
         uint32_t x, y, z;
         m2xyz(g, list[i], x, y, z);
         union_back(lab, g, x, y, z);
     }
+    if (ctas > 1) {
+        __threadfence();   // this CTA's unions before its ticket
+        __syncthreads();
+        if (t == 0) s_ticket = atomicAdd(d_done, 1u);
+        __syncthreads();
+        if (s_ticket + 1u != ctas) return;
+        __threadfence();   // the other CTAs' unions after theirs
+    }
+    for (uint32_t w = t; w < words; w += kListCta) st_cg(bitmap + w, 0u);
     __syncthreads();
     for (uint32_t i = t; i < cnt; i += kListCta) {
         const uint32_t m = list[i];
@@ -786,12 +804,13 @@ int ccl_dense(const Img &bin, uint32_t *lab, Arena &ws, cudaStream_t st, bool di
 
 int ccl_list(const Geo &g, int64_t n, uint32_t *lab, const uint32_t *list,
              const uint32_t *d_count, int64_t cap, Arena &ws, cudaStream_t st,
-             uint32_t *d_nlabels) {
+             uint32_t *d_nlabels, uint32_t *d_done, bool dense) {
     Rank r = take_rank(ws, fkey_bits_for(n));
     if (!ws.ok()) { set_error("seed labeling: workspace too small"); return CLE_ERR_WORKSPACE; }
-    if (n <= kListCtaVoxels) {
-        ccl_list_small<<<1, kListCta, 0, st>>>(lab, g, list, d_count, r.bitmap, r.prefix, r.words, d_nlabels);
-        CLE_LAUNCH_CHECK("ccl list (one CTA)");
+    if (n <= (dense ? kListDenseVoxels : kListSparseVoxels)) {
+        ccl_list_small<<<(unsigned)((n + kListCta - 1) / kListCta), kListCta, 0, st>>>(lab, g, list, d_count, r.bitmap, r.prefix,
+                                                                                   r.words, d_nlabels, d_done);
+        CLE_LAUNCH_CHECK("ccl list (one launch)");
         return CLE_OK;
     }
     const int b = launch_blocks(cap, kT);

@@ -90,10 +90,11 @@ int ccl_dense(const Img &binary, uint32_t *labels, Arena &ws, cudaStream_t st, b
               const float *d_above = nullptr);
 // CCL restricted to a device list of voxel indices whose entries in `labels`
 // already hold (own x-major key + 1); on return those entries hold labels.
-// d_count: device count of list entries; cap: list capacity.
+// d_count: device count of list entries; cap: list capacity; d_done: a device
+// word that is 0; dense: the list may hold every voxel (not only local maxima).
 int ccl_list(const Geo &g, int64_t n, uint32_t *labels, const uint32_t *list,
              const uint32_t *d_count, int64_t cap, Arena &ws, cudaStream_t st,
-             uint32_t *d_nlabels = nullptr);
+             uint32_t *d_nlabels, uint32_t *d_done, bool dense = false);
 int ccl_to_dst(const uint32_t *lab, const Img &dst, cudaStream_t st);
 size_t relabel_workspace_bytes(uint32_t max_label);
 int relabel_sequential(const Img &src, const Img &dst, uint32_t max_label, Arena &ws,

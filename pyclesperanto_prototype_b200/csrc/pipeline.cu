@@ -22,7 +22,7 @@ struct Scalars {
     int status;
     uint32_t seed_count;
     uint32_t nlabels;        // labels of the last call (= its maximum label)
-    uint32_t pad0;
+    uint32_t ccl_done;       // CTAs of the seed labelling that have finished
     MinMaxState mm;          // of the outline blur
     float thr32;
     float pad;
@@ -151,7 +151,8 @@ int masked_voronoi_binary(const Img &bin, const Img &mask, const Img &dst, Arena
         case CLE_U32: CLE_TRY(launch_mask_seeds<uint32_t>(bin, mask, g, l, lab, st)); break;
         default: set_error("masked_voronoi_labeling: unsupported binary dtype %d", bin.dtype); return CLE_ERR_DTYPE;
     }
-    CLE_TRY(ccl_list(g, bin.n(), lab, l.seeds, &l.sc->seed_count, bin.n(), ws, st, &l.sc->nlabels));
+    CLE_TRY(ccl_list(g, bin.n(), lab, l.seeds, &l.sc->seed_count, bin.n(), ws, st, &l.sc->nlabels,
+                     &l.sc->ccl_done, true));
     ws.off = tail_off;
     CLE_TRY(voronoi_grow(bin, lab, l.seg, l.seeds, &l.sc->seed_count, &l.sc->nlabels, &l.sc->status, ws, st,
                          lim));
@@ -404,7 +405,8 @@ int voronoi_otsu_labeling(const Img &src, const Img &dst, double spot_sigma, dou
     stage_mark(4, st);
 
     // 5: label the seeds
-    CLE_TRY(ccl_list(g, n, lab, l.seeds, &l.sc->seed_count, n, ws, st, &l.sc->nlabels));
+    CLE_TRY(ccl_list(g, n, lab, l.seeds, &l.sc->seed_count, n, ws, st, &l.sc->nlabels,
+                     &l.sc->ccl_done));
     ws.off = tail_off;
     stage_mark(5, st);
 
