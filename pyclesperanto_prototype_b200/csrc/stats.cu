@@ -8,14 +8,17 @@
 // each of them the warp builds every lane's bit mask of matching voxels (the
 // coordinate sums and the bounding box are popcounts and bit scans of it), sums
 // the intensities, reduces over the lanes and adds the result to the label's
-// accumulators, one record, with four atomic instructions.  Voxels of a brick
-// with more labels than are kept (kMaxLabels) are added one by one.  A label
+// accumulators, one record, with four atomic instructions.  Where labels are tiny
+// (kWorth) the voxels are added by themselves, those that touch along a lane's
+// column together.  A label
 // that fills half a brick (the background, where it counts as one) is carried
 // along in registers from brick to brick.  Two passes, as in the reference (the
 // second needs the per-label centroid, mass centre and mean); the second takes
-// the labels and masks the first kept, 3.1 bytes per voxel of scratch at most,
-// and does not read the label image.  Coordinates and 8/16-bit intensities are
-// summed in exact 64-bit integers (exact_sums), other intensities in float64; min / max through
+// the labels and masks the first kept, at most kMaxLabels of a brick (3.1 bytes per
+// voxel of scratch; images thinner than a brick in some direction keep at least one
+// label of each, up to 32 bytes per voxel where a brick holds 4), and does not read
+// the label image for those.  Coordinates and 8/16-bit intensities are summed in
+// exact 64-bit integers (exact_sums), other intensities in float64; min / max through
 // order-preserving unsigned atomics.  The finalise kernels apply the reference's
 // float32 column arithmetic and its sentinels for labels absent from the image
 // (min FLT_MAX, max -FLT_MAX, sums 0, 0/0 = NaN).
@@ -23,6 +26,9 @@
 // pipe 73% busy; 0.49 at copy bandwidth), pass 2 0.74 ms (issue 71%: two exact
 // square roots and three float64 sums a voxel).  The sorted form before it
 // (voxel indices scattered into label order, then swept) took 2.31 and 0.67 ms.
+// 128 x 512 x 512 full of blocks of 3 x 3 x 3, uint16 / float32: 2.01 / 2.14 ms (sorted 2.40 / 2.42; with
+// an atomic set per voxel beyond the kept labels 3.22 / 3.30); 5 x 5 x 5 1.03 / 1.37 (1.18 / 1.29); 4 x 4 x 4
+// 0.68 / 0.93 (1.38 / 1.40); 2 x 2 x 2 3.37 / 3.46 (4.80 / 4.77); a random label per voxel 3.98 (3.30).
 #include <cfloat>
 
 #include "common.cuh"
@@ -33,7 +39,11 @@ namespace cle {
 namespace {
 
 constexpr int kST = 256;
-constexpr int kMaxLabels = 24;   // labels of a brick reduced over the warp (fewer in thin images)
+constexpr int kMaxLabels = 24;   // labels of a brick kept for pass 2 (fewer in thin images)
+// Labels are reduced over the warp while they average kWorth voxels of the brick
+// (looked at from kTryLabels on): a reduction costs what adding that many voxels
+// by themselves does, more for float64 sums.
+constexpr uint32_t kTryLabels = 4, kWorthInt = 6, kWorthFloat = 12;
 
 // Accumulators of a label: pass 1 ...
 struct alignas(32) Acc1 {
@@ -109,11 +119,19 @@ __device__ __forceinline__ uint32_t live_label(const TL *lab, int64_t m, int64_t
 
 constexpr int kBatch = 4;   // row segments per warp round (loads in flight)
 
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
+// Sums of four values over the warp; lane l gets that of value l % 4.  The first two
+// steps halve what a lane carries: 6 exchanges instead of 20.
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d) {
+    const int lane = threadIdx.x & 31;
+    const bool odd = lane & 1, high = lane & 2;
+    double p = odd ? b : a, q = odd ? d : c;
+    p += __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+    q += __shfl_xor_sync(0xffffffffu, odd ? c : d, 1);
+    double r = high ? q : p;
+    r += __shfl_xor_sync(0xffffffffu, high ? p : q, 2);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    for (int o = 4; o < 32; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
 }
 // Distances of a voxel to its label's centroid and mass centre in float32
 // (relative error a few 1e-7) and its intensity's deviation from the mean; the
@@ -175,6 +193,66 @@ __device__ __forceinline__ T lane4(T a, T b, T c, T d) {
     return lane & 2 ? (lane & 1 ? d : c) : (lane & 1 ? b : a);
 }
 
+// What a lane has of a label in its column of the brick.
+template <bool INT>
+struct Column {
+    typename std::conditional<INT, unsigned long long, double>::type v, vy, vz;
+    uint32_t n, sy, sz, ylo, yhi, zlo, zhi, vlo, vhi;
+    __device__ __forceinline__ void clear() {
+        v = vy = vz = 0;
+        n = sy = sz = yhi = zhi = vhi = 0u;
+        ylo = zlo = vlo = 0xFFFFFFFFu;
+    }
+    template <typename TI>
+    __device__ __forceinline__ void add(uint32_t y, uint32_t z, TI w) {
+        const float f = to_f32(w);
+        const uint32_t o = f2u(f);
+        ++n;
+        sy += y;
+        sz += z;
+        if constexpr (INT) {
+            v += (unsigned long long)w;
+            vy += (unsigned long long)w * y;
+            vz += (unsigned long long)w * z;
+        } else {
+            v += (double)f;
+            vy += (double)f * (double)y;
+            vz += (double)f * (double)z;
+        }
+        ylo = min(ylo, y); yhi = max(yhi, y);
+        zlo = min(zlo, z); zhi = max(zhi, z);
+        vlo = min(vlo, o); vhi = max(vhi, o);
+    }
+    __device__ __forceinline__ void add_to(Acc1 *a, uint32_t x, bool exact) const {
+        // bounds that the record holds already need no atomic (they only widen, so
+        // an older value is as good)
+        const uint4 lo = *reinterpret_cast<const uint4 *>(a->lo), hi = *reinterpret_cast<const uint4 *>(a->hi);
+        atomicAdd(a->s, (unsigned long long)n * x);
+        atomicAdd(a->s + 1, (unsigned long long)sy);
+        atomicAdd(a->s + 2, (unsigned long long)sz);
+        atomicAdd(a->s + 3, (unsigned long long)n);
+        if (INT && exact) {
+            atomicAdd(a->u, (unsigned long long)v);
+            atomicAdd(a->u + 1, (unsigned long long)v * x);
+            atomicAdd(a->u + 2, (unsigned long long)vy);
+            atomicAdd(a->u + 3, (unsigned long long)vz);
+        } else {
+            atomicAdd(a->v, (double)v);
+            atomicAdd(a->v + 1, (double)v * (double)x);
+            atomicAdd(a->v + 2, (double)vy);
+            atomicAdd(a->v + 3, (double)vz);
+        }
+        if (x < lo.x) atomicMin(a->lo, x);
+        if (ylo < lo.y) atomicMin(a->lo + 1, ylo);
+        if (zlo < lo.z) atomicMin(a->lo + 2, zlo);
+        if (vlo < lo.w) atomicMin(a->lo + 3, vlo);
+        if (x > hi.x) atomicMax(a->hi, x);
+        if (yhi > hi.y) atomicMax(a->hi + 1, yhi);
+        if (zhi > hi.z) atomicMax(a->hi + 2, zhi);
+        if (vhi > hi.w) atomicMax(a->hi + 3, vhi);
+    }
+};
+
 // Pass 1 over the voxels of the bricks.
 template <typename TL, typename TI, int BY>
 __global__ void __launch_bounds__(kST, 2)
@@ -229,50 +307,21 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
                 else p += G.W;
             }
         }
-        uint32_t found = 0;
+        uint32_t found = 0, covered = 0, mask_all = 0;   // labels, their voxels, this lane's
+        uint32_t g = 0;
         for (;;) {
             // the largest label left in the brick
-            uint32_t g = 0;
+            g = 0;
 #pragma unroll
             for (int k = 0; k < 32; ++k) g = max(g, l[k]);
             g = __reduce_max_sync(0xffffffffu, g);
             if (g == 0u) break;
-            if (found == G.slots) {
-                // many small labels: the voxels left are added one by one
-                found |= kMore;
-#pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    if (l[k] == 0u) continue;
-                    const uint32_t y = y0 + k % BY, z = z0 + k / BY;
-                    const float f = to_f32(v[k]);
-                    Acc1 *a = a1 + (l[k] - 1u);
-                    atomicAdd(a->s, (unsigned long long)x);
-                    atomicAdd(a->s + 1, (unsigned long long)y);
-                    atomicAdd(a->s + 2, (unsigned long long)z);
-                    atomicAdd(a->s + 3, 1ull);
-                    if (INT && exact) {
-                        const unsigned long long u = (unsigned long long)v[k];
-                        atomicAdd(a->u, u);
-                        atomicAdd(a->u + 1, u * x);
-                        atomicAdd(a->u + 2, u * y);
-                        atomicAdd(a->u + 3, u * z);
-                    } else {
-                        const double d = (double)f;
-                        atomicAdd(a->v, d);
-                        atomicAdd(a->v + 1, d * (double)x);
-                        atomicAdd(a->v + 2, d * (double)y);
-                        atomicAdd(a->v + 3, d * (double)z);
-                    }
-                    atomicMin(a->lo, x); atomicMin(a->lo + 1, y); atomicMin(a->lo + 2, z); atomicMin(a->lo + 3, f2u(f));
-                    atomicMax(a->hi, x); atomicMax(a->hi + 1, y); atomicMax(a->hi + 2, z); atomicMax(a->hi + 3, f2u(f));
-                }
-                break;
-            }
+            if (found >= kTryLabels && covered < (INT ? kWorthInt : kWorthFloat) * found) break;   // many tiny labels
             Sums<INT> t;
             uint32_t mine = 0;                     // this lane's voxels of label g
             uint32_t vmin = 0xFFFFFFFFu, vmax = 0u;
             uint32_t iv = 0, ivy = 0, ivz = 0;      // 8/16-bit: a brick's sums fit 32 bits
-            double dv = 0.0, dvy = 0.0, dvz = 0.0;
+            double dvy = 0.0, dplane[BZ] = {};      // others: per plane, so that z costs nothing per voxel
 #pragma unroll
             for (int k = 0; k < 32; ++k) {
                 if (l[k] == g) {
@@ -288,9 +337,8 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
                     } else {
                         const float f = to_f32(v[k]);
                         const double d = (double)f;
-                        dv += d;
+                        dplane[k / BY] += d;
                         dvy += d * (double)(y0 + k % BY);
-                        dvz += d * (double)(z0 + k / BY);
                         vmin = min(vmin, f2u(f));
                         vmax = max(vmax, f2u(f));
                     }
@@ -309,6 +357,8 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
             kz /= (uint32_t)BY;
             const uint32_t n = (uint32_t)__popc(mine);
             const uint32_t N = __reduce_add_sync(0xffffffffu, n);
+            covered += N;
+            mask_all |= mine;
             const unsigned long long xb = bx * 32u;
             {
                 const uint32_t sx = __reduce_add_sync(0xffffffffu, n * lane);
@@ -324,9 +374,13 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
                 hi3 = f2u((float)__reduce_max_sync(0xffffffffu, vmax));
             } else {
                 // lanes without a voxel of the label add nothing (0 x infinity would)
-                const double V = warp_sum(dv), Vx = warp_sum(mine ? dv * (double)x : 0.0);
-                const double Vy = warp_sum(dvy), Vz = warp_sum(dvz);
-                t.v = lane4(V, Vx, Vy, Vz);
+                double dv = 0.0, dvz = 0.0;
+#pragma unroll
+                for (int j = 0; j < BZ; ++j) {
+                    dv += dplane[j];
+                    dvz += dplane[j] * (double)(z0 + j);
+                }
+                t.v = warp_sum4(dv, mine ? dv * (double)x : 0.0, dvy, dvz);
                 lo3 = __reduce_min_sync(0xffffffffu, vmin);
                 hi3 = __reduce_max_sync(0xffffffffu, vmax);
             }
@@ -351,11 +405,34 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
             } else {
                 t.add_to(a1 + (g - 1u), exact);
             }
-            F.mask[((size_t)b * G.slots + found) * 32u + lane] = mine;
-            if (lane == 0) F.label[(size_t)b * G.slots + found] = g;
+            if (found < G.slots) {
+                F.mask[((size_t)b * G.slots + found) * 32u + lane] = mine;
+                if (lane == 0) F.label[(size_t)b * G.slots + found] = g;
+            }
             ++found;
         }
-        if (lane == 0) F.count[b] = (uint8_t)found;
+        if (g != 0u) {
+            // the voxels left, one by one: each lane joins what touches along its
+            // column (the labels come from the L1 once more)
+            Column<INT> c;
+            uint32_t of = 0;   // label of c
+            c.clear();
+#pragma unroll 1
+            for (uint32_t k = 0; k < 32u; ++k) {
+                const uint32_t y = y0 + k % BY, z = z0 + k / BY, m = at + k / BY * HW + k % BY * G.W + lane;
+                uint32_t lk = 0;
+                if (!(mask_all >> k & 1u) && x < G.W && y < G.H && z < G.D) lk = lab_of(__ldg(lab + m));
+                if (lk > L) lk = 0u;
+                if (lk != of) {
+                    if (of) c.add_to(a1 + (of - 1u), x, exact);
+                    c.clear();
+                    of = lk;
+                }
+                if (lk) c.add(y, z, __ldg(inten + m));
+            }
+            if (of) c.add_to(a1 + (of - 1u), x, exact);
+        }
+        if (lane == 0) F.count[b] = (uint8_t)(min(found, G.slots) | (g != 0u || found > G.slots ? kMore : 0u));
     }
     if (carried) carry.add_to(a1 + (carried - 1u), exact);
 }
@@ -426,32 +503,58 @@ brick_moments_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, B
                 w = wn;
             }
             __syncwarp();
-            const double S0 = warp_sum(sdc), S1 = warp_sum(sdm), S2 = warp_sum(ssq);
+            const double S = warp_sum4(sdc, sdm, ssq, 0.0);
             const uint32_t M0 = __reduce_max_sync(0xffffffffu, __float_as_uint(mdc));
             const uint32_t M1 = __reduce_max_sync(0xffffffffu, __float_as_uint(mdm));
             Acc2 *a = a2 + (g - 1u);
-            if (lane < 3) atomicAdd(a->s + lane, lane == 0 ? S0 : lane == 1 ? S1 : S2);
+            if (lane < 3) atomicAdd(a->s + lane, S);
             if (lane < 2) atomicMax(a->m + lane, lane == 0 ? M0 : M1);
         }
         if (found & kMore) {
-            // voxels of labels that were not kept, one by one
+            // voxels of labels that were not kept: what touches along a lane's column
+            // is added at once
             const uint32_t L = (uint32_t)live_labels(Lcap, d_L), x = bx * 32u + lane;
+            uint32_t of = 0;   // label at hand
+            float4 pc = make_float4(0.f, 0.f, 0.f, 0.f), pm = pc;
+            double sdc = 0.0, sdm = 0.0, ssq = 0.0;
+            float mdc = 0.0f, mdm = 0.0f;
+            auto flush = [&]() {
+                Acc2 *a = a2 + (of - 1u);
+                const uint2 m = *reinterpret_cast<const uint2 *>(a->m);   // only grow: an older value is as good
+                atomicAdd(a->s, sdc);
+                atomicAdd(a->s + 1, sdm);
+                atomicAdd(a->s + 2, ssq);
+                if (__float_as_uint(mdc) > m.x) atomicMax(a->m, __float_as_uint(mdc));
+                if (__float_as_uint(mdm) > m.y) atomicMax(a->m + 1, __float_as_uint(mdm));
+            };
 #pragma unroll 1
             for (int k = 0; k < 32; ++k) {
                 const uint32_t y = y0 + k % BY, z = z0 + k / BY, m = at + (uint32_t)(k / BY) * HW + (uint32_t)(k % BY) * G.W + lane;
-                if ((seen >> k & 1u) || x >= G.W || y >= G.H || z >= G.D) continue;
-                const uint32_t g = lab_of(__ldg(lab + m));
-                if (g == 0u || g > L) continue;
-                Acc2 *a = a2 + (g - 1u);
-                float dc, dm;
-                double dv;
-                voxel_moments(a->pc, a->pm, (float)x, (float)y, (float)z, to_f32(__ldg(inten + m)), dc, dm, dv);
-                atomicAdd(a->s, (double)dc);
-                atomicAdd(a->s + 1, (double)dm);
-                atomicAdd(a->s + 2, dv * dv);
-                atomicMax(a->m, __float_as_uint(fmaxf(0.0f, dc)));
-                atomicMax(a->m + 1, __float_as_uint(fmaxf(0.0f, dm)));
+                uint32_t g = 0;
+                if (!(seen >> k & 1u) && x < G.W && y < G.H && z < G.D) g = lab_of(__ldg(lab + m));
+                if (g > L) g = 0u;
+                if (g != of) {
+                    if (of) flush();
+                    sdc = sdm = ssq = 0.0;
+                    mdc = mdm = 0.0f;
+                    of = g;
+                    if (g) {
+                        pc = a2[g - 1u].pc;
+                        pm = a2[g - 1u].pm;
+                    }
+                }
+                if (g) {
+                    float dc, dm;
+                    double dv;
+                    voxel_moments(pc, pm, (float)x, (float)y, (float)z, to_f32(__ldg(inten + m)), dc, dm, dv);
+                    sdc += (double)dc;
+                    sdm += (double)dm;
+                    ssq += dv * dv;
+                    mdc = fmaxf(mdc, dc);
+                    mdm = fmaxf(mdm, dm);
+                }
             }
+            if (of) flush();
         }
     }
 }

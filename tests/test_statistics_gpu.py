@@ -45,3 +45,59 @@ def test_totals_beyond_2_to_53_are_exact(cle, axis):
     image = np.ascontiguousarray(row[None, :] if axis == "x" else row[:, None])
     table = cle.statistics_of_labelled_pixels(cle.push_native(image), _on_device(cle, np.ones(image.shape)))
     assert float(table["sum_intensity_times_" + axis][0]) == 2 ** 53 + 2 ** 30
+
+
+def _blocks(shape, block, seed=9):
+    """A label per block, in no order of place."""
+    at, n = np.zeros(shape, np.int64), 1
+    for g, s, k in zip(np.indices(shape), shape, block):
+        c = -(-s // k)
+        at = at * c + g // k
+        n *= c
+    return np.random.default_rng(seed).permutation(n)[at] + 1
+
+
+# many small labels: more in a brick (32 x 8 x 4 voxels, 32 x 32 pixels) than are kept for the
+# second pass, sizes on both sides of where voxels are added by themselves, partial
+# bricks, images thinner than a brick
+@pytest.mark.parametrize("shape,block", [((9, 21, 70), (1, 1, 1)), ((9, 21, 70), (1, 2, 3)), ((9, 21, 70), (2, 2, 2)),
+                                         ((9, 21, 70), (3, 3, 3)), ((13, 30, 65), (5, 5, 5)), ((70, 99), (2, 2)),
+                                         ((70, 99), (3, 4)), ((70, 99), (6, 7)), ((1, 300), (1, 2)), ((300, 1), (5, 1)),
+                                         ((40, 2, 3), (2, 1, 2)), ((600, 1, 1), (1, 1, 1))])
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_many_small_labels(cle, oracle, shape, block, dtype):
+    r = np.random.default_rng(10)
+    labels = _blocks(shape, block)
+    image = (r.integers(0, 250, size=shape) if dtype != np.float32 else r.uniform(-100, 5000, size=shape)).astype(dtype)
+    for lab in (labels, np.where(r.uniform(size=labels.max() + 1)[labels] < 0.4, 0, labels)):
+        want = oracle.statistics_of_labelled_pixels(image.astype(np.float32), lab.astype(np.uint32))
+        got = cle.statistics_of_labelled_pixels(cle.push_native(image), _on_device(cle, lab))
+        assert set(got) == set(want)
+        for key in want:
+            # sums of float64 or whole numbers, rounded to float32; distances in float32
+            np.testing.assert_allclose(got[key], want[key], rtol=2e-5, atol=2e-4, err_msg=key)
+
+
+def _table_time(cle, block, dtype):
+    from pyclesperanto_prototype_b200 import _ops
+    lab = _blocks((64, 256, 256), block)
+    image = cle.push_native(np.random.default_rng(1).integers(0, 4000, size=lab.shape).astype(dtype))
+    labels, n = _on_device(cle, lab), int(lab.max())
+    best = []
+    for _ in range(8):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        e0.record()
+        for _ in range(5):
+            _ops.statistics_table(image, labels, n)
+        e1.record()
+        torch.cuda.synchronize()
+        best.append(e0.elapsed_time(e1))
+    return min(best)
+
+
+# labels of 27 voxels, more than are kept of a brick, against labels of 64, which are all
+# kept (4.7 and 3.4 times the time while each voxel beyond was added by itself)
+@pytest.mark.parametrize("dtype,most", [(np.uint16, 3.8), (np.float32, 2.9)])
+def test_small_labels_do_not_fall_off(cle, dtype, most):
+    assert _table_time(cle, (3, 3, 3), dtype) < most * _table_time(cle, (4, 4, 4), dtype)
