@@ -431,7 +431,7 @@ voronoi_bricks_kernel(uint32_t *lab, const uint8_t *__restrict__ seg, BGeo G,
         const uint32_t bs = block_total(changed, s_red);
         if (threadIdx.x == 0 && bs) atomicAdd(&S->changes[t & 3], bs);
         if (!tail) ok = grid_sync(&S->bar, &S->err, barrier_ns);
-        else { __syncthreads(); ok = *(volatile int *)&S->err == 0; }
+        else ok = block_ok(&S->err);
         if (!ok) break;
         const uint32_t nchanged = __ldcg(&S->changes[t & 3]);
         if (trace && gtid == 0 && t < kTraceSteps) {
@@ -492,7 +492,7 @@ voronoi_bricks_kernel(uint32_t *lab, const uint8_t *__restrict__ seg, BGeo G,
         }
         if (!bitmap) ap.flush(Fn, nsize);
         if (!tail) ok = grid_sync(&S->bar, &S->err, barrier_ns);
-        else { __syncthreads(); ok = *(volatile int *)&S->err == 0; }
+        else ok = block_ok(&S->err);
         if (bitmap && ok) ok = compact_queue(Qb, Fn, nsize, S, barrier_ns, s_red, s_scan, s_off);
         if (trace && gtid == 0 && t < kTraceSteps) trace[4 * t + 3] = global_ns() - t_start;
         ++t;
@@ -552,7 +552,7 @@ struct KState {
     GridBarrier bar;
     int err;
     int gate;          // 1: the brick kernel grows the labels after this launch
-    int overflow;      // an s above kKeyMaxS was reached
+    int overflow[2];   // an s above kKeyMaxS was reached in an even, an odd round
     uint32_t sizes[4];
     uint32_t rounds;   // diagnostics of the last launch: rounds run,
     uint32_t stop_s;   // S,
@@ -670,7 +670,9 @@ voronoi_keys_kernel(uint32_t *lab, uint8_t *seg, BGeo G, const uint32_t *seeds,
         uint32_t *Fn = (r & 1) ? B0 : B1;
         const uint32_t nB = __ldcg(&S->sizes[r & 3]);
         if (nB == 0u) { done = true; break; }
-        if (*(volatile int *)&S->overflow) break;
+        // raised in the round before: that word no longer changes, while the
+        // round at hand may raise the other before a slower block is here
+        if (*(volatile int *)&S->overflow[(r + 1u) & 1u]) break;
         if (trace && gtid == 0 && r < kTraceSteps) {
             trace[4 * r] = global_ns() - t_start;
             trace[4 * r + 1] = nB;
@@ -888,7 +890,7 @@ voronoi_keys_kernel(uint32_t *lab, uint8_t *seg, BGeo G, const uint32_t *seeds,
                     chb[j] = __ballot_sync(0xffffffffu, c);
                     chall |= chb[j];
                 }
-                if (over) atomicExch(&S->overflow, 1);
+                if (over) atomicExch(&S->overflow[r & 1u], 1);
                 // this brick again if it is still changing, a neighbour when a
                 // changed voxel faces it and it holds a candidate next to them
                 bool want = false;
@@ -924,9 +926,9 @@ voronoi_keys_kernel(uint32_t *lab, uint8_t *seg, BGeo G, const uint32_t *seeds,
     for (int i = threadIdx.x; i < 256; i += KBT)
         if (s_hist[i]) atomicAdd(&S->hist[i], s_hist[i]);
     if (ok) ok = grid_sync(&S->bar, &S->err, barrier_ns);
-    const bool overflow = *(volatile int *)&S->overflow != 0;
+    const bool overflow = (*(volatile int *)&S->overflow[0] | *(volatile int *)&S->overflow[1]) != 0;
     if (ok && !done && !overflow) ok = false;   // round bound reached
-    if (!ok && !overflow) {
+    if (!ok) {
         if (gtid == 0) {
             const int e = *(volatile int *)&S->err;
             *d_status = e ? e : (int)CLE_ERR_ITER_LIMIT;
