@@ -110,12 +110,14 @@ size_t rank_workspace_bytes(uint64_t bits);
 // steps; otherwise the labels are left as given and the brick kernel behind it
 // grows them step by step.  seg: mask bytes as the seed passes write them
 // (kMaskByte); the growth keeps each labelled voxel's arrival step in them.
-// segments: the mask is the whole image, the list holds one labelled voxel per
-// 8-voxel row segment and the mask bytes of labelled voxels are 0x80 already.
+// label_bricks (optional): the mask is the whole image, the list holds one
+// labelled voxel per 8-voxel row segment, the mask bytes of labelled voxels are
+// 0x80 already, and the word counts the growth bricks that hold a label.
+constexpr int kBrickX = 8, kBrickY = 4, kBrickZ = 4;   // a growth brick (one plane in images)
 size_t voronoi_grow_workspace_bytes(const Img &im);
 int voronoi_grow(const Img &shape, uint32_t *labels, uint8_t *seg, const uint32_t *seeds,
                  const uint32_t *d_seed_count, const uint32_t *d_max_label, int *d_status, Arena &ws,
-                 cudaStream_t st, const Limits &lim, int segments = 0);
+                 cudaStream_t st, const Limits &lim, const uint32_t *label_bricks = nullptr);
 size_t voronoi_dense_workspace_bytes(const Img &im);
 int masked_voronoi_dense(const Img &binary, const Img &mask, const Img &dst, int *d_status,
                          Arena &ws, cudaStream_t st, const Limits &lim);

@@ -23,6 +23,8 @@ struct Scalars {
     uint32_t seed_count;
     uint32_t nlabels;        // labels of the last call (= its maximum label)
     uint32_t ccl_done;       // CTAs of the seed labelling that have finished
+    uint32_t label_bricks;   // growth bricks that hold a label (growth over the whole image)
+    uint32_t pad1;
     MinMaxState mm;          // of the outline blur
     float thr32;
     float pad;
@@ -192,37 +194,68 @@ __global__ void to_labels_kernel(const T *__restrict__ src, uint32_t *__restrict
 constexpr int kSeedWarps = 8;
 
 // One seed voxel per 8-voxel row segment (x aligned to 8) that holds a label;
-// the segment lies in one growth brick (8 x by 4 y), so the 3x3x3 brick
+// the segment lies in one growth brick (8 x by 4 y, BZ z), so the 3x3x3 brick
 // neighbourhood of the seed's brick covers every voxel next to a label of the
-// segment.  A warp reads 32 x of one row.  One global atomic per CTA.  Also
-// the mask bytes: arrival step 0 on labels, not yet known elsewhere.
+// segment.  A warp takes four bricks side by side, all of its rows loaded first.
+// Also the mask bytes (arrival step 0 on labels, not yet known elsewhere), the
+// largest label and the number of bricks that hold a label.  A few global
+// atomics per CTA.
+template <int BZ>
 __global__ void __launch_bounds__(kSeedWarps * 32)
-brick_seeds_kernel(const uint32_t *__restrict__ lab, uint8_t *__restrict__ seg, uint32_t W, uint32_t WB, FastDiv fWB,
-                   uint32_t nb, uint32_t *__restrict__ seeds, uint32_t *__restrict__ d_count) {
-    __shared__ uint32_t s_n, s_base;
+brick_seeds_kernel(const uint32_t *__restrict__ lab, uint8_t *__restrict__ seg, uint32_t D, uint32_t H, uint32_t W, uint32_t nx,
+                   FastDiv fnx, FastDiv fny, uint32_t n, uint32_t *__restrict__ seeds, Scalars *__restrict__ sc) {
+    constexpr int ROWS = kBrickY * BZ;
+    __shared__ uint32_t s_n, s_base, s_max, s_bricks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t base = blockIdx.x * kSeedWarps; base < nb; base += gridDim.x * kSeedWarps) {
+    if (threadIdx.x == 0) s_max = s_bricks = 0u;
+    for (uint32_t base = blockIdx.x * kSeedWarps; base < n; base += gridDim.x * kSeedWarps) {
         if (threadIdx.x == 0) s_n = 0;
         __syncthreads();
         const uint32_t b = base + warp;
-        uint32_t pos = 0, m = 0;
-        bool has = false;
-        if (b < nb) {
-            const uint32_t r = fWB.div(b), xb = b - r * WB, x = xb * 32u + (uint32_t)lane;
-            const bool on = x < W && lab[r * W + x] != 0u;
-            if (x < W) seg[r * W + x] = on ? (uint8_t)0x80 : kMaskByte;
-            const unsigned bal = __ballot_sync(0xffffffffu, on);
-            const unsigned seg8 = (bal >> (lane & 24)) & 0xFFu;   // this lane's 8-voxel segment
-            has = (lane & 7) == 0 && seg8 != 0u;
-            if (has) {
-                m = r * W + xb * 32u + (uint32_t)(lane & 24) + (uint32_t)(__ffs(seg8) - 1);
-                pos = atomicAdd(&s_n, 1u);
+        uint32_t held = 0, pos = 0;   // segments with a label (a row per bit; lanes 0, 8, 16, 24), their place in the CTA's
+        uint32_t v[ROWS], at = 0;
+        if (b < n) {
+            const uint32_t r = fnx.div(b), xb = b - r * nx, zb = fny.div(r), yb = r - zb * fny.d;
+            const uint32_t x = xb * 32u + (uint32_t)lane, y0 = yb * kBrickY, z0 = zb * BZ;
+            at = (z0 * H + y0) * W + x;
+            uint32_t most = 0;
+#pragma unroll
+            for (int k = 0; k < ROWS; ++k) {
+                const bool in = x < W && y0 + k % kBrickY < H && z0 + k / kBrickY < D;
+                v[k] = in ? lab[at + ((uint32_t)(k / kBrickY) * H + (uint32_t)(k % kBrickY)) * W] : 0u;
+                most = max(most, v[k]);
             }
+#pragma unroll
+            for (int k = 0; k < ROWS; ++k) {
+                if (x < W && y0 + k % kBrickY < H && z0 + k / kBrickY < D)
+                    seg[at + ((uint32_t)(k / kBrickY) * H + (uint32_t)(k % kBrickY)) * W] = v[k] ? (uint8_t)0x80 : kMaskByte;
+                const unsigned bal = __ballot_sync(0xffffffffu, v[k] != 0u);
+                if ((lane & 7) == 0 && (bal >> lane & 0xFFu)) held |= 1u << k;
+            }
+            most = __reduce_max_sync(0xffffffffu, most);
+            const unsigned bricks = __ballot_sync(0xffffffffu, held != 0u);
+            if (lane == 0 && most) {
+                atomicMax(&s_max, most);
+                atomicAdd(&s_bricks, (uint32_t)__popc(bricks));
+            }
+            if (held) pos = atomicAdd(&s_n, (uint32_t)__popc(held));
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_base = s_n ? atomicAdd(d_count, s_n) : 0u;
+        if (threadIdx.x == 0) s_base = s_n ? atomicAdd(&sc->seed_count, s_n) : 0u;
         __syncthreads();
-        if (has) seeds[s_base + pos] = m;
+        if (b < n) {
+            uint32_t *out = seeds + s_base + pos;
+#pragma unroll
+            for (int k = 0; k < ROWS; ++k) {
+                const unsigned bal = __ballot_sync(0xffffffffu, v[k] != 0u) >> (lane & 24);
+                if (held >> k & 1u) *out++ = at + ((uint32_t)(k / kBrickY) * H + (uint32_t)(k % kBrickY)) * W + (uint32_t)__ffs(bal & 0xFFu) - 1u;
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_max) {
+        atomicMax(&sc->nlabels, s_max);
+        atomicAdd(&sc->label_bricks, s_bricks);
     }
 }
 
@@ -245,16 +278,15 @@ ExtLayout take_ext_layout(Arena &a, const Img &im) {
 // Grows `lab` in place over the whole image; status in l.sc.
 int grow_everywhere(const Img &im, uint32_t *lab, ExtLayout &l, Arena &tail, cudaStream_t st,
                     const Limits &lim) {
-    const uint32_t WB = (uint32_t)((im.W + 31) / 32);
-    const uint32_t nb = (uint32_t)(im.D * im.H) * WB;
-    brick_seeds_kernel<<<launch_blocks((int64_t)nb * 32, kSeedWarps * 32), kSeedWarps * 32, 0, st>>>(
-        lab, l.seg, (uint32_t)im.W, WB, FastDiv(WB), nb, l.seeds, &l.sc->seed_count);
+    const int bz = im.ndim == 3 ? kBrickZ : 1;
+    const uint32_t nx = (uint32_t)((im.W + 31) / 32), ny = (uint32_t)((im.H + kBrickY - 1) / kBrickY);
+    const uint32_t n = nx * ny * (uint32_t)((im.D + bz - 1) / bz);
+    auto kern = im.ndim == 3 ? brick_seeds_kernel<kBrickZ> : brick_seeds_kernel<1>;
+    kern<<<launch_blocks((int64_t)n * 32, kSeedWarps * 32), kSeedWarps * 32, 0, st>>>(
+        lab, l.seg, (uint32_t)im.D, (uint32_t)im.H, (uint32_t)im.W, nx, FastDiv(nx), FastDiv(ny), n, l.seeds, l.sc);
     CLE_LAUNCH_CHECK("brick seeds");
-    Img L = im;
-    L.data = lab;
-    L.dtype = CLE_U32;
-    CLE_TRY(label_max(L, &l.sc->nlabels, tail, st));
-    return voronoi_grow(im, lab, l.seg, l.seeds, &l.sc->seed_count, &l.sc->nlabels, &l.sc->status, tail, st, lim, 1);
+    return voronoi_grow(im, lab, l.seg, l.seeds, &l.sc->seed_count, &l.sc->nlabels, &l.sc->status, tail, st, lim,
+                        &l.sc->label_bricks);
 }
 
 }  // namespace

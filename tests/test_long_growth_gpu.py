@@ -53,3 +53,21 @@ def test_few_seeds(cle, oracle, shape, seeds):
     lab.reshape(-1)[r.choice(lab.size, seeds, replace=False)] = np.arange(1, seeds + 1)
     dev = cle.B200Array(torch.from_numpy(lab.astype(np.int32)).cuda().view(torch.uint32))
     assert np.array_equal(cle.pull(cle.extend_labeling_via_voronoi(dev)).astype(np.uint32), oracle.extend_labeling_via_voronoi(lab))
+
+
+# labels in nearly every 8 x 4 (x 4) brick: the step-by-step growth takes over; one brick in 512
+# empty, two, none, images with partial bricks
+@pytest.mark.parametrize("shape", [(64, 128), (64, 256), (61, 250), (16, 64, 64), (15, 62, 61), (1, 8, 70), (40, 3, 5)])
+@pytest.mark.parametrize("empty", [0, 1, 2, 3])
+def test_labels_in_nearly_every_brick(cle, oracle, shape, empty):
+    r = np.random.default_rng(6)
+    lab = np.where(r.uniform(size=shape) < 0.5, r.integers(1, 1000, size=shape), 0).astype(np.uint32)
+    for k in range(empty):
+        x = 8 * (2 * k) % (8 * (-(-shape[-1] // 8)))
+        lab[..., :4, x:x + 8][..., :, :] = 0 if len(shape) == 2 else lab[..., :4, x:x + 8]
+        if len(shape) == 3:
+            lab[:4, :4, x:x + 8] = 0
+    if lab.max() == 0:
+        lab.reshape(-1)[-1] = 5
+    for src in (cle.B200Array(torch.from_numpy(lab.astype(np.int32)).cuda().view(torch.uint32)), lab.astype(np.float32)):
+        assert np.array_equal(cle.pull(cle.extend_labeling_via_voronoi(src)).astype(np.uint32), oracle.extend_labeling_via_voronoi(lab))
