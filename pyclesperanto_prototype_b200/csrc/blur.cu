@@ -195,11 +195,12 @@ blur_row_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t ro
 // Pass along an axis of length L with element stride `inner`, for a volume
 // viewed as [outer][L][inner]: a CTA takes NG x 8 outputs along the axis and
 // 2 x NC columns (NG x NC = 256 threads).  tile0: the launch's first tile of the
-// axis; ctas: the CTAs of all launches of the pass.
+// axis; ctas: the CTAs of all launches of the pass; clear (optional): a word to
+// set to 0 that neither src nor dst holds.
 template <typename Tin, int NG>
 __global__ void __launch_bounds__(kSepThreads)
 blur_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t inner, int L, int tile0, int vec,
-                const __grid_constant__ Taps taps, MinMaxState *__restrict__ mm, uint32_t ctas) {
+                const __grid_constant__ Taps taps, MinMaxState *__restrict__ mm, uint32_t ctas, int *clear) {
     constexpr int NC = kSepThreads / NG, COLS = 2 * NC, ROWS = NG * kK;
     extern __shared__ __align__(16) float2 sm[];
     const int n = taps.n, r = (n - 1) / 2;
@@ -208,6 +209,7 @@ blur_col_kernel(const Tin *__restrict__ src, float *__restrict__ dst, int64_t in
     const int64_t c0 = (int64_t)blockIdx.x * COLS;
     const int l0 = (tile0 + (int)blockIdx.y) * ROWS;
     const int64_t base = (int64_t)blockIdx.z * L * inner;
+    if (clear && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0u) *clear = 0;
     for (int i = threadIdx.x; i < n; i += kSepThreads) sw[i] = make_float2(taps.w[i], taps.w[i]);
     const int span = min(ROWS, L - l0) + 2 * r;
     if (vec) {
@@ -305,7 +307,7 @@ int col_groups(int64_t L, int n) { return L <= 32 && n <= 129 ? 4 : L <= 64 && n
 
 template <typename Tin, int NG>
 int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, const Taps &t, MinMaxState *mm,
-               cudaStream_t st) {
+               int *clear, cudaStream_t st) {
     constexpr int COLS = 2 * (kSepThreads / NG), ROWS = NG * kK;
     const int64_t cols = (inner + COLS - 1) / COLS, tiles = (L + ROWS - 1) / ROWS;
     const size_t smem = sizeof(float2) * tap_slots(t.n) + sizeof(float) * COLS * kK * line_blocks(ROWS, t.n);
@@ -319,7 +321,7 @@ int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, 
         for (int64_t tile0 = 0; tile0 < tiles; tile0 += kMost) {
             const dim3 grid((unsigned)cols, (unsigned)std::min(tiles - tile0, kMost), (unsigned)std::min(outer - o, kMost));
             blur_col_kernel<Tin, NG><<<grid, kSepThreads, smem, st>>>(src + o * L * inner, dst + o * L * inner, inner, L,
-                                                                      (int)tile0, vec, t, mm, (uint32_t)(cols * tiles * outer));
+                                                                      (int)tile0, vec, t, mm, (uint32_t)(cols * tiles * outer), clear);
             CLE_LAUNCH_CHECK("blur pass");
         }
     return CLE_OK;
@@ -327,14 +329,18 @@ int launch_col(const Tin *src, float *dst, int64_t inner, int L, int64_t outer, 
 
 template <typename Tin>
 int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps &t, MinMaxState *mm,
-                cudaStream_t st) {
+                int *clear, cudaStream_t st) {
     if (axis == 2) {
-        // the row split evenly into tiles of at most kRowMax outputs, row pairs
-        // to fill the CTA's threads
+        // the row split evenly into tiles of at most kRowMax outputs
         const int64_t rows = im.D * im.H;
         const int tiles = (int)((im.W + kRowMax - 1) / kRowMax);
         const int tile = (int)(((im.W + tiles - 1) / tiles + kK - 1) / kK * kK);
-        const int np = std::max(1, std::min(kSepThreads / (tile / kK), 16));
+        // row pairs to fill a CTA's threads, fewer where there would not be two
+        // CTAs per SM (256 x 256, 801 taps: a call of 83 us with 16 CTAs)
+        int dev = 0;
+        CLE_CUDA(cudaGetDevice(&dev));
+        const int64_t share = rows / 2 * tiles / (2 * num_sms(dev));
+        const int np = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(kSepThreads / (tile / kK), 16), share));
         const int64_t ctas = (rows + 2 * np - 1) / (2 * np);
         const dim3 grid((unsigned)((im.W + tile - 1) / tile), (unsigned)std::min<int64_t>(ctas, 65535),
                         (unsigned)((ctas + 65534) / 65535));
@@ -350,9 +356,9 @@ int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps 
         if (axis == 1) { inner = im.W; L = (int)im.H; outer = im.D; }
         else { inner = im.W * im.H; L = (int)im.D; outer = 1; }
         switch (col_groups(L, t.n)) {
-            case 4: CLE_TRY((launch_col<Tin, 4>(src, dst, inner, L, outer, t, mm, st))); break;
-            case 8: CLE_TRY((launch_col<Tin, 8>(src, dst, inner, L, outer, t, mm, st))); break;
-            default: CLE_TRY((launch_col<Tin, 16>(src, dst, inner, L, outer, t, mm, st))); break;
+            case 4: CLE_TRY((launch_col<Tin, 4>(src, dst, inner, L, outer, t, mm, clear, st))); break;
+            case 8: CLE_TRY((launch_col<Tin, 8>(src, dst, inner, L, outer, t, mm, clear, st))); break;
+            default: CLE_TRY((launch_col<Tin, 16>(src, dst, inner, L, outer, t, mm, clear, st))); break;
         }
     }
     return CLE_OK;
@@ -367,7 +373,7 @@ int launch_convert(const Tin *src, float *dst, int64_t n, cudaStream_t st) {
 
 template <typename Tin>
 int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, float *t2, MinMaxState *mm,
-                    cudaStream_t st) {
+                    int *clear, cudaStream_t st) {
     // pass order x (axis 2), y (axis 1), z (axis 0, 3D only)
     const int passes = (src.ndim == 3) ? 3 : 2;
     const int64_t n = src.n();
@@ -378,12 +384,14 @@ int separable_typed(const Img &src, float *dst, const Taps *taps[3], float *t1, 
     for (int p = 0; p < passes; ++p) {
         float *o = (p == passes - 1) ? dst : bufs[which];
         const Taps *t = taps[p];
+        const bool last = p == passes - 1;
         if (cur_is_src) {
-            if (t) CLE_TRY(launch_pass<Tin>((const Tin *)cur, o, src, 2 - p, *t, p == passes - 1 ? mm : nullptr, st));
+            if (t) CLE_TRY(launch_pass<Tin>((const Tin *)cur, o, src, 2 - p, *t, last ? mm : nullptr, last ? clear : nullptr, st));
             else CLE_TRY(launch_convert<Tin>((const Tin *)cur, o, n, st));
         } else {
-            if (t) CLE_TRY(launch_pass<float>((const float *)cur, o, src, 2 - p, *t, p == passes - 1 ? mm : nullptr, st));
+            if (t) CLE_TRY(launch_pass<float>((const float *)cur, o, src, 2 - p, *t, last ? mm : nullptr, last ? clear : nullptr, st));
             else if (o != cur) CLE_CUDA(cudaMemcpyAsync(o, cur, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+            if (last && clear && !t) CLE_CUDA(cudaMemsetAsync(clear, 0, sizeof(int), st));
         }
         cur = o;
         cur_is_src = false;
@@ -402,7 +410,7 @@ size_t separable_workspace_bytes(const Img &im) {
 }
 
 int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty, const Taps *tz,
-                     Arena &ws, cudaStream_t st, MinMaxState *mm) {
+                     Arena &ws, cudaStream_t st, MinMaxState *mm, int *clear) {
     float *t1 = ws.take<float>(src.n());
     float *t2 = ws.take<float>(src.n());
     if (!ws.ok()) {
@@ -411,9 +419,9 @@ int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty,
     }
     const Taps *taps[3] = {tx, ty, tz};
     switch (src.dtype) {
-        case CLE_F32: return separable_typed<float>(src, dst, taps, t1, t2, mm, st);
-        case CLE_U16: return separable_typed<uint16_t>(src, dst, taps, t1, t2, mm, st);
-        case CLE_U8: return separable_typed<uint8_t>(src, dst, taps, t1, t2, mm, st);
+        case CLE_F32: return separable_typed<float>(src, dst, taps, t1, t2, mm, clear, st);
+        case CLE_U16: return separable_typed<uint16_t>(src, dst, taps, t1, t2, mm, clear, st);
+        case CLE_U8: return separable_typed<uint8_t>(src, dst, taps, t1, t2, mm, clear, st);
         default:
             set_error("gaussian_blur: source dtype %d not supported (u8/u16/f32)", src.dtype);
             return CLE_ERR_DTYPE;
@@ -421,7 +429,7 @@ int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty,
 }
 
 int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, Arena &ws,
-                  cudaStream_t st, int *status) {
+                  cudaStream_t st, int *status, bool clear) {
     if (fused_blur_applies(src, sx, sy, sz))
         return fused_blur(src, dst, sx, st, nullptr, status);
     Taps tx, ty, tz;
@@ -429,7 +437,7 @@ int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, A
     if (sx > 0) { CLE_TRY(make_gauss_taps(sx, tx)); px = &tx; }
     if (sy > 0) { CLE_TRY(make_gauss_taps(sy, ty)); py = &ty; }
     if (src.ndim == 3 && sz > 0) { CLE_TRY(make_gauss_taps(sz, tz)); pz = &tz; }
-    return separable_filter(src, dst, px, py, pz, ws, st);
+    return separable_filter(src, dst, px, py, pz, ws, st, nullptr, clear && src.ndim == 3 ? status : nullptr);
 }
 
 int separable_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st) {

@@ -56,16 +56,13 @@ int cle_gaussian_blur(const cle_tensor *src, const cle_tensor *dst, double sx, d
     if (b.dtype != CLE_F32) { set_error("gaussian_blur: destination must be float32"); return CLE_ERR_DTYPE; }
     CLE_TRY(ws_check(ws, ws_bytes, separable_workspace_bytes(a), "gaussian_blur"));
     CLE_TRY(set_device_of(a, src));
-    // the workspace's first word is the call's status (cle_workspace_status): the
-    // fused path of a volume reports a staging wait that ran out there; the
-    // other paths, whose intermediates may lie there, leave it at 0
-    int *status = ws && ws_bytes >= sizeof(int) ? static_cast<int *>(ws) : nullptr;
-    const bool fused_volume = a.ndim == 3 && fused_blur_applies(a, sx, sy, sz);
-    if (fused_volume && status) CLE_CUDA(cudaMemsetAsync(status, 0, sizeof(int), S(stream)));
+    // the workspace's first word is a volume's status (cle_workspace_status): the
+    // fused path reports a staging wait that ran out there, the three-pass path,
+    // whose intermediates lie there, leaves it at 0.  Images have none.
+    int *status = a.ndim == 3 && ws && ws_bytes >= sizeof(int) ? static_cast<int *>(ws) : nullptr;
+    if (status && fused_blur_applies(a, sx, sy, sz)) CLE_CUDA(cudaMemsetAsync(status, 0, sizeof(int), S(stream)));
     Arena ar(ws, ws_bytes);
-    CLE_TRY(gaussian_blur(a, (float *)b.data, sx, sy, sz, ar, S(stream), fused_volume ? status : nullptr));
-    if (a.ndim == 3 && !fused_volume && status) CLE_CUDA(cudaMemsetAsync(status, 0, sizeof(int), S(stream)));
-    return CLE_OK;
+    return gaussian_blur(a, (float *)b.data, sx, sy, sz, ar, S(stream), status, true);
 }
 
 // ---- min / max -------------------------------------------------------------

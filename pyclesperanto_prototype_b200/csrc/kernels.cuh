@@ -8,15 +8,16 @@ namespace cle {
 // blur.cu
 size_t separable_workspace_bytes(const Img &im);
 int separable_filter(const Img &src, float *dst, const Taps *tx, const Taps *ty, const Taps *tz,
-                     Arena &ws, cudaStream_t st, MinMaxState *mm = nullptr);
+                     Arena &ws, cudaStream_t st, MinMaxState *mm = nullptr, int *clear = nullptr);
 // Three-pass isotropic blur (sigma > 0) whose {min, max} lands in mm->out (the
 // state zeroed before), reduced in the last pass.
 int separable_minmax(const Img &src, float *dst, double sigma, MinMaxState *mm, Arena &ws, cudaStream_t st);
 // status (optional): a device status word; given it, the fused path of a
 // volume may stage planes with TMA copies and reports a stage wait that ran
-// out there (CLE_ERR_ITER_LIMIT)
+// out there (CLE_ERR_ITER_LIMIT); with `clear` the other path of a volume sets it to
+// 0 (it may lie at the start of the workspace), without it leaves it alone
 int gaussian_blur(const Img &src, float *dst, double sx, double sy, double sz, Arena &ws,
-                  cudaStream_t st, int *status = nullptr);
+                  cudaStream_t st, int *status = nullptr, bool clear = false);
 
 // blur_fused.cu (isotropic sigma, one launch): radius up to kMaxFusedR in 2D,
 // kMaxFusedR3 in 3D

@@ -97,3 +97,30 @@ def test_aligned_sources_are_not_slower(cle, shape, dtype):
             times.append(e0.elapsed_time(e1))
         best.append(min(times))
     assert best[0] <= 1.25 * best[1]
+
+
+# the status word of a volume's blur, whichever form it takes and whatever the
+# workspace held; an axis without a blur ends the three-pass form with a copy
+@pytest.mark.parametrize("sigma", [(2, 2, 2), (3, 3, 3), (1, 2, 0.5), (4, 0, 0), (0, 0, 4), (0, 0, 0)])
+@pytest.mark.parametrize("shape", [(5, 40, 48), (9, 260, 272)])
+def test_status_word_of_a_blur(cle, oracle, shape, sigma):
+    import torch
+    from pyclesperanto_prototype_b200 import _lib
+    lib = _lib.load()
+    a = _image(shape, np.uint16)
+    src, dst = torch.from_numpy(a).cuda(), torch.empty(shape, device="cuda")
+    s, d = _lib.tensor_desc(src), _lib.tensor_desc(dst)
+    ws = torch.full((lib.cle_gaussian_blur_workspace_bytes(_lib.ref(s)),), 255, dtype=torch.uint8, device="cuda")
+    stream = _lib.stream_ptr()
+    _lib.check(lib.cle_gaussian_blur(_lib.ref(s), _lib.ref(d), *[float(v) for v in sigma], ws.data_ptr(), ws.numel(), stream))
+    assert lib.cle_workspace_status(ws.data_ptr(), ws.numel(), stream) == 0
+    assert np.array_equal(dst.cpu().numpy(), oracle.gaussian_blur(a.astype(np.float32), *sigma))
+
+
+# rows split over fewer or more row pairs per CTA: few rows, long windows
+@pytest.mark.parametrize("shape", [(1, 256), (2, 300), (9, 40), (700, 24), (5, 7, 33)])
+@pytest.mark.parametrize("sigma", [(100, 0.5, 0), (20, 0, 3), (6, 7, 8)])
+def test_gaussian_blur_of_few_rows(cle, oracle, shape, sigma):
+    a = _image(shape, np.uint16)
+    got = cle.pull(cle.gaussian_blur(a, None, *sigma))
+    assert np.array_equal(got, oracle.gaussian_blur(a.astype(np.float32), *sigma))
