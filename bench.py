@@ -102,20 +102,20 @@ def config_of(name, nvox):
 STAGES = ["blur_outline", "hist_otsu", "blur_spot", "maxima_seeds", "seed_ccl", "voronoi_growth", None,
           None, "stats_pass1", "stats_final1", "stats_pass2", "stats_final2"]
 ALGO_BYTES = {"blur_outline": 2 + 4, "hist_otsu": 4, "blur_spot": 2 + 4, "maxima_seeds": 4 + 4 + 1 + 4,
-              "voronoi_growth": 1 + 1 + 4, "stats_pass1": 4 + 2, "stats_pass2": 4 + 2}
+              "voronoi_growth": 1 + 1 + 4, "stats_pass1": 4 + 2, "stats_pass2": 2 + 0.125}
 
 
 def algo_bytes(w, labelled_fraction=None):
     """ALGO_BYTES for a workload: the seed pass finds the maxima (reads both
     blurs, writes the mask and the labels); with equal spot and outline sigmas
-    there is one blur.  The second statistics pass reads the label and
-    intensity of labelled voxels only."""
+    there is one blur.  The second statistics pass reads the intensity of
+    labelled voxels and a bit each from the masks the first pass kept."""
     b = dict(ALGO_BYTES)
     if w.get("spot") is not None and w.get("spot") == w.get("outline"):
         b["maxima_seeds"] = 4 + 1 + 4
         del b["blur_spot"]
     if labelled_fraction is not None:
-        b["stats_pass2"] = (4 + 2) * labelled_fraction
+        b["stats_pass2"] *= labelled_fraction
     return b
 # The pipeline's compulsory traffic per voxel (the minimal pass structure the
 # two global reductions force): read src + write blur 8, read blur for the

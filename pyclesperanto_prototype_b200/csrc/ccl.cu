@@ -341,49 +341,47 @@ template <int TY, int TZ, bool DIAMOND>
 __global__ void __launch_bounds__(kT)
 ccl_merge_kernel(const uint32_t *__restrict__ lab, const uint32_t *__restrict__ bits, uint32_t *parent, Geo g,
                  Tiles t, FastDiv fws, uint32_t nseg) {
-    {
-        const uint32_t sgm = blockIdx.x * kT + threadIdx.x;
-        const uint32_t m = sgm < nseg ? bits[sgm] : 0u;
-        if (!m) return;
-        const uint32_t r = fws.div(sgm), xs = sgm - r * t.ws;   // r = z * H + y
-        const uint32_t z = g.fH.div(r), y = r - z * g.H;
-        const bool first = xs == 0u, last = xs + 1u == t.ws;
-        const uint32_t mL = first ? 0u : bits[sgm - 1u], mR = last ? 0u : bits[sgm + 1u];
-        const uint32_t *row = lab + (size_t)r * g.W + xs * 32u;
-        // neighbouring contacts mostly join the same two components: the pair
-        // united last is not walked again
-        uint32_t la = 0u, lb = 0u;
-        auto join = [&](const uint32_t *p, const uint32_t *q) {
-            const uint32_t a = __ldg(p), b = __ldg(q);
-            if (a == la && b == lb) return;
-            la = a;
-            lb = b;
-            unite_plain<false>(parent, a - 1u, b - 1u);
-        };
-        if ((m & 1u) && (mL >> 31)) join(row, row - 1);
-        uint32_t q[4], qs[4];
-        bool in[4];
+    const uint32_t sgm = blockIdx.x * kT + threadIdx.x;
+    const uint32_t m = sgm < nseg ? bits[sgm] : 0u;
+    if (!m) return;
+    const uint32_t r = fws.div(sgm), xs = sgm - r * t.ws;   // r = z * H + y
+    const uint32_t z = g.fH.div(r), y = r - z * g.H;
+    const bool first = xs == 0u, last = xs + 1u == t.ws;
+    const uint32_t mL = first ? 0u : bits[sgm - 1u], mR = last ? 0u : bits[sgm + 1u];
+    const uint32_t *row = lab + (size_t)r * g.W + xs * 32u;
+    // neighbouring contacts mostly join the same two components: the pair
+    // united last is not walked again
+    uint32_t la = 0u, lb = 0u;
+    auto join = [&](const uint32_t *p, const uint32_t *q) {
+        const uint32_t a = __ldg(p), b = __ldg(q);
+        if (a == la && b == lb) return;
+        la = a;
+        lb = b;
+        unite_plain<false>(parent, a - 1u, b - 1u);
+    };
+    if ((m & 1u) && (mL >> 31)) join(row, row - 1);
+    uint32_t q[4], qs[4];
+    bool in[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int qy = (int)y + row_dy(k), qz = (int)z + row_dz(k);
-            in[k] = (TZ > 1 || k == 0) && qy >= 0 && qy < (int)g.H && qz >= 0;
-            qs[k] = in[k] ? ((uint32_t)qz * g.H + (uint32_t)qy) * t.ws + xs : 0u;
-            q[k] = in[k] ? bits[qs[k]] : 0u;
-        }
+    for (int k = 0; k < 4; ++k) {
+        const int qy = (int)y + row_dy(k), qz = (int)z + row_dz(k);
+        in[k] = (TZ > 1 || k == 0) && qy >= 0 && qy < (int)g.H && qz >= 0;
+        qs[k] = in[k] ? ((uint32_t)qz * g.H + (uint32_t)qy) * t.ws + xs : 0u;
+        q[k] = in[k] ? bits[qs[k]] : 0u;
+    }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (!in[k] || (DIAMOND && (k == 1 || k == 3))) continue;
-            const uint32_t qy = y + (uint32_t)row_dy(k), qz = z + (uint32_t)row_dz(k);
-            const bool cross = qy / TY != y / TY || qz / TZ != z / TZ;
-            const uint32_t *qrow = lab + ((size_t)qz * g.H + qy) * g.W + xs * 32u;
-            if (cross)
-                row_contacts<DIAMOND>(m, q[k], via_row<DIAMOND>(k, q), 0xFFFFFFFFu, [&](uint32_t i, uint32_t j) { join(row + i, qrow + j); });
-            if constexpr (!DIAMOND) {
-                // diagonal contacts over the segment's ends that no other
-                // contact implies
-                if ((m & 1u) && !first && !(q[k] & 1u) && !(mL >> 31) && (bits[qs[k] - 1u] >> 31)) join(row, qrow - 1);
-                if ((m >> 31) && !last && !(q[k] >> 31) && !(mR & 1u) && (bits[qs[k] + 1u] & 1u)) join(row + 31, qrow + 32);
-            }
+    for (int k = 0; k < 4; ++k) {
+        if (!in[k] || (DIAMOND && (k == 1 || k == 3))) continue;
+        const uint32_t qy = y + (uint32_t)row_dy(k), qz = z + (uint32_t)row_dz(k);
+        const bool cross = qy / TY != y / TY || qz / TZ != z / TZ;
+        const uint32_t *qrow = lab + ((size_t)qz * g.H + qy) * g.W + xs * 32u;
+        if (cross)
+            row_contacts<DIAMOND>(m, q[k], via_row<DIAMOND>(k, q), 0xFFFFFFFFu, [&](uint32_t i, uint32_t j) { join(row + i, qrow + j); });
+        if constexpr (!DIAMOND) {
+            // diagonal contacts over the segment's ends that no other
+            // contact implies
+            if ((m & 1u) && !first && !(q[k] & 1u) && !(mL >> 31) && (bits[qs[k] - 1u] >> 31)) join(row, qrow - 1);
+            if ((m >> 31) && !last && !(q[k] >> 31) && !(mR & 1u) && (bits[qs[k] + 1u] & 1u)) join(row + 31, qrow + 32);
         }
     }
 }

@@ -308,9 +308,9 @@ maxima_seeds2_kernel(const float *__restrict__ T, const float *__restrict__ d_th
 // per lane as above; otherwise one.
 template <int ROWS, bool PAIRS>
 __global__ void __launch_bounds__(32 * kGroups)
-maxima_seeds_outline_kernel(const float *__restrict__ T, const float *__restrict__ O, const float *__restrict__ d_thr32, Geo g,
-                    int zchunk, uint8_t *__restrict__ seg, uint32_t *__restrict__ lab, uint32_t *__restrict__ seeds,
-                    uint32_t *__restrict__ d_count) {
+maxima_seeds_outline_kernel(const float *__restrict__ T, const float *__restrict__ O, const float *__restrict__ d_thr32,
+                            Geo g, int zchunk, uint8_t *__restrict__ seg, uint32_t *__restrict__ lab,
+                            uint32_t *__restrict__ seeds, uint32_t *__restrict__ d_count) {
     constexpr int kRows = ROWS, kWin = ROWS + 2, C = PAIRS ? 2 : 1;
     struct Cols { float c[C]; };
     const int D = (int)g.D, H = (int)g.H, W = (int)g.W;
