@@ -26,9 +26,9 @@
 // pipe 73% busy; 0.49 at copy bandwidth), pass 2 0.74 ms (issue 71%: two exact
 // square roots and three float64 sums a voxel).  The sorted form before it
 // (voxel indices scattered into label order, then swept) took 2.31 and 0.67 ms.
-// 128 x 512 x 512 full of blocks of 3 x 3 x 3, uint16 / float32: 2.01 / 2.14 ms (sorted 2.40 / 2.42; with
-// an atomic set per voxel beyond the kept labels 3.22 / 3.30); 5 x 5 x 5 1.03 / 1.37 (1.18 / 1.29); 4 x 4 x 4
-// 0.68 / 0.93 (1.38 / 1.40); 2 x 2 x 2 3.37 / 3.46 (4.80 / 4.77); a random label per voxel 3.98 (3.30).
+// 128 x 512 x 512 full of blocks of 3 x 3 x 3, uint16 / float32: 2.05 / 2.10 ms (sorted 2.40 / 2.42; with
+// an atomic set per voxel beyond the kept labels 3.22 / 3.30); 5 x 5 x 5 1.05 / 1.35 (1.18 / 1.29); 4 x 4 x 4
+// 0.69 / 0.93 (1.38 / 1.40); 2 x 2 x 2 3.46 / 3.08 (4.80 / 4.77); a random label per voxel 3.46 (3.30).
 #include <cfloat>
 
 #include "common.cuh"
@@ -307,16 +307,33 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
                 else p += G.W;
             }
         }
-        uint32_t found = 0, covered = 0, mask_all = 0;   // labels, their voxels, this lane's
-        uint32_t g = 0;
+        uint32_t found = 0, covered = 0, more = 0;   // labels, their voxels
         for (;;) {
             // the largest label left in the brick
-            g = 0;
+            uint32_t g = 0;
 #pragma unroll
             for (int k = 0; k < 32; ++k) g = max(g, l[k]);
             g = __reduce_max_sync(0xffffffffu, g);
             if (g == 0u) break;
-            if (found >= kTryLabels && covered < (INT ? kWorthInt : kWorthFloat) * found) break;   // many tiny labels
+            if (found >= kTryLabels && covered < (INT ? kWorthInt : kWorthFloat) * found) {
+                // many tiny labels: the voxels left are added by themselves, those that
+                // follow one another in a lane's column together.  (From the registers:
+                // a rolled loop that reads the labels again makes the compiler's code of
+                // the whole kernel worse, 0.66 against 0.62 ms on sparse labels.)
+                more = kMore;
+                Column<INT> c;
+                c.clear();
+#pragma unroll
+                for (int k = 0; k < 32; ++k) {
+                    if (l[k] == 0u) continue;
+                    c.add(y0 + k % BY, z0 + k / BY, v[k]);
+                    if (k == 31 || l[k < 31 ? k + 1 : 31] != l[k]) {
+                        c.add_to(a1 + (l[k] - 1u), x, exact);
+                        c.clear();
+                    }
+                }
+                break;
+            }
             Sums<INT> t;
             uint32_t mine = 0;                     // this lane's voxels of label g
             uint32_t vmin = 0xFFFFFFFFu, vmax = 0u;
@@ -358,7 +375,6 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
             const uint32_t n = (uint32_t)__popc(mine);
             const uint32_t N = __reduce_add_sync(0xffffffffu, n);
             covered += N;
-            mask_all |= mine;
             const unsigned long long xb = bx * 32u;
             {
                 const uint32_t sx = __reduce_add_sync(0xffffffffu, n * lane);
@@ -411,28 +427,7 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
             }
             ++found;
         }
-        if (g != 0u) {
-            // the voxels left, one by one: each lane joins what touches along its
-            // column (the labels come from the L1 once more)
-            Column<INT> c;
-            uint32_t of = 0;   // label of c
-            c.clear();
-#pragma unroll 1
-            for (uint32_t k = 0; k < 32u; ++k) {
-                const uint32_t y = y0 + k % BY, z = z0 + k / BY, m = at + k / BY * HW + k % BY * G.W + lane;
-                uint32_t lk = 0;
-                if (!(mask_all >> k & 1u) && x < G.W && y < G.H && z < G.D) lk = lab_of(__ldg(lab + m));
-                if (lk > L) lk = 0u;
-                if (lk != of) {
-                    if (of) c.add_to(a1 + (of - 1u), x, exact);
-                    c.clear();
-                    of = lk;
-                }
-                if (lk) c.add(y, z, __ldg(inten + m));
-            }
-            if (of) c.add_to(a1 + (of - 1u), x, exact);
-        }
-        if (lane == 0) F.count[b] = (uint8_t)(min(found, G.slots) | (g != 0u || found > G.slots ? kMore : 0u));
+        if (lane == 0) F.count[b] = (uint8_t)(min(found, G.slots) | (found > G.slots ? kMore : more));
     }
     if (carried) carry.add_to(a1 + (carried - 1u), exact);
 }
@@ -441,7 +436,7 @@ brick_sums_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bric
 // into a list from the masks, so that every lane works, and their intensities
 // gathered; the label image itself is not read again.
 template <typename TL, typename TI, int BY>
-__global__ void __launch_bounds__(kST)
+__global__ void __launch_bounds__(kST, 6)
 brick_moments_kernel(const TL *__restrict__ lab, const TI *__restrict__ inten, Bricks G, int64_t Lcap,
                      const uint32_t *__restrict__ d_L, Acc2 *__restrict__ a2, Found F) {
     constexpr int BZ = 32 / BY;
