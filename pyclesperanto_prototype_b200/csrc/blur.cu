@@ -335,11 +335,12 @@ int launch_pass(const Tin *src, float *dst, const Img &im, int axis, const Taps 
         const int64_t rows = im.D * im.H;
         const int tiles = (int)((im.W + kRowMax - 1) / kRowMax);
         const int tile = (int)(((im.W + tiles - 1) / tiles + kK - 1) / kK * kK);
-        // row pairs to fill a CTA's threads, fewer where there would not be two
-        // CTAs per SM (256 x 256, 801 taps: a call of 83 us with 16 CTAs)
+        // row pairs to fill a CTA's threads, fewer where not even a quarter of the SMs
+        // would have a CTA (256 x 256, 801 taps: a call of 83 us with 16 CTAs; two CTAs
+        // for every SM cost a batch of tiles, which share the GPU, 2%)
         int dev = 0;
         CLE_CUDA(cudaGetDevice(&dev));
-        const int64_t share = rows / 2 * tiles / (2 * num_sms(dev));
+        const int64_t share = rows / 2 * tiles / std::max(1, num_sms(dev) / 4);
         const int np = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(kSepThreads / (tile / kK), 16), share));
         const int64_t ctas = (rows + 2 * np - 1) / (2 * np);
         const dim3 grid((unsigned)((im.W + tile - 1) / tile), (unsigned)std::min<int64_t>(ctas, 65535),
