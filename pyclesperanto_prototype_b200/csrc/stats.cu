@@ -26,9 +26,9 @@
 // pipe 73% busy; 0.49 at copy bandwidth), pass 2 0.74 ms (issue 71%: two exact
 // square roots and three float64 sums a voxel).  The sorted form before it
 // (voxel indices scattered into label order, then swept) took 2.31 and 0.67 ms.
-// 128 x 512 x 512 full of blocks of 3 x 3 x 3, uint16 / float32: 2.05 / 2.10 ms (sorted 2.40 / 2.42; with
-// an atomic set per voxel beyond the kept labels 3.22 / 3.30); 5 x 5 x 5 1.05 / 1.35 (1.18 / 1.29); 4 x 4 x 4
-// 0.69 / 0.93 (1.38 / 1.40); 2 x 2 x 2 3.46 / 3.08 (4.80 / 4.77); a random label per voxel 3.46 (3.30).
+// 128 x 512 x 512 full of blocks of 3 x 3 x 3, uint16 / float32: 2.07 / 2.24 ms (sorted 2.40 / 2.42; with
+// an atomic set per voxel beyond the kept labels 3.22 / 3.30); 5 x 5 x 5 1.05 / 1.36 (1.18 / 1.29); 4 x 4 x 4
+// 0.70 / 0.93 (1.38 / 1.40); 2 x 2 x 2 3.44 / 3.15 (4.80 / 4.77); a random label per voxel 3.67 (3.30).
 #include <cfloat>
 
 #include "common.cuh"
@@ -42,8 +42,11 @@ constexpr int kST = 256;
 constexpr int kMaxLabels = 24;   // labels of a brick kept for pass 2 (fewer in thin images)
 // Labels are reduced over the warp while they average kWorth voxels of the brick
 // (looked at from kTryLabels on): a reduction costs what adding that many voxels
-// by themselves does, more for float64 sums.
-constexpr uint32_t kTryLabels = 4, kWorthInt = 6, kWorthFloat = 12;
+// by themselves does, more for float64 sums.  The largest labels come first, so a
+// background that counts as label 1 comes last: with kTryLabels = 4 a few slivers of
+// cells sent it to its single voxels (2048 x 1024 float32, 3600 cells of 24 pixels and a
+// background: pass 2 20 -> 31 us).
+constexpr uint32_t kTryLabels = 16, kWorthInt = 6, kWorthFloat = 12;
 
 // Accumulators of a label: pass 1 ...
 struct alignas(32) Acc1 {

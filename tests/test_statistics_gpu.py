@@ -101,3 +101,18 @@ def _table_time(cle, block, dtype):
 @pytest.mark.parametrize("dtype,most", [(np.uint16, 3.8), (np.float32, 2.9)])
 def test_small_labels_do_not_fall_off(cle, dtype, most):
     assert _table_time(cle, (3, 3, 3), dtype) < most * _table_time(cle, (4, 4, 4), dtype)
+
+
+# a background that counts as a label (the smallest, taken last) between many tiny cells
+@pytest.mark.parametrize("dtype", [np.uint16, np.float32])
+def test_background_between_small_cells(cle, oracle, dtype):
+    r = np.random.default_rng(14)
+    shape = (96, 128)
+    lab = np.ones(shape, np.int64)
+    for k, (y, x) in enumerate(r.integers(0, 90, size=(200, 2))):
+        lab[y:y + 2, x:x + 3] = k + 2
+    image = r.integers(0, 4000, size=shape).astype(dtype)
+    want = oracle.statistics_of_labelled_pixels(image.astype(np.float32), lab.astype(np.uint32))
+    got = cle.statistics_of_labelled_pixels(cle.push_native(image), _on_device(cle, lab))
+    for key in want:
+        np.testing.assert_allclose(got[key], want[key], rtol=2e-5, atol=2e-4, err_msg=key)
